@@ -21,6 +21,7 @@
 #include <initializer_list>
 
 #include "krylov_device.cuh"
+#include "pairsums.cuh"
 #include "profile.cuh"
 
 namespace emusv {
@@ -266,91 +267,25 @@ k_contract(const KState *ks_g, int n, const void *g0_, const unsigned char *basi
     }
 }
 
-__global__ void k_sum_adj(const double *partials, int nblocks, int nv, double *out) {
-    for (int v = threadIdx.x; v < nv; v += blockDim.x) {
-        double s = 0.0;
-        for (int b = 0; b < nblocks; ++b) s += partials[(int64_t)b * (4 * ADJ_MAXQ + 8) + v];
-        out[v] = s;
-    }
+// out[v] = sum of the blocks' value v, one warp per value.
+__global__ void __launch_bounds__(32) k_sum_adj(const double *partials, int nblocks, double *out) {
+    const int v = blockIdx.x;
+    double s = 0.0;
+#pragma unroll 4
+    for (int b = threadIdx.x; b < nblocks; b += 32) s += partials[(int64_t)b * (4 * ADJ_MAXQ + 8) + v];
+    s = warp_sum(s);
+    if (threadIdx.x == 0) out[v] = s;
 }
 
-constexpr int PAIR_HB = 6;  // high bits enumerated per thread by k_pairs
-
-// Pair sums S_PQ = sum_x x_P x_Q rho(x) for bit positions P <= Q (complex).  Thread t owns
-// the amplitudes x = t + (k << s), s = n - h, k < 2^h (h = min(n, PAIR_HB)): its low s
-// bits are fixed, so only the h high bits need per-amplitude accumulators (the total, one
-// per high bit, one per high pair); the low bits enter when the pairs are reduced.
-__global__ void __launch_bounds__(BLOCK)
-k_pairs(const double *rho, int n, double *partials) {
-    __shared__ double acc[2 * ADJ_MAXQ * ADJ_MAXQ];
-    constexpr int NHH = PAIR_HB * (PAIR_HB + 1) / 2;
-    const int h = n < PAIR_HB ? n : PAIR_HB, s = n - h;
-    for (int k = threadIdx.x; k < 2 * n * n; k += blockDim.x) acc[k] = 0.0;
-    __syncthreads();
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    double Rr = 0.0, Ri = 0.0, Hr[PAIR_HB], Hi[PAIR_HB], HHr[NHH], HHi[NHH];
-#pragma unroll
-    for (int q = 0; q < PAIR_HB; ++q) Hr[q] = Hi[q] = 0.0;
-#pragma unroll
-    for (int q = 0; q < NHH; ++q) HHr[q] = HHi[q] = 0.0;
-    if (t < (int64_t(1) << s)) {
-        for (int k = 0; k < (1 << h); ++k) {
-            const int64_t x = t + ((int64_t)k << s);
-            const double rr = rho[2 * x], ri = rho[2 * x + 1];
-            Rr += rr;
-            Ri += ri;
-            int idx = 0;
-#pragma unroll
-            for (int q = 0; q < PAIR_HB; ++q) {
-                const double fq = double((k >> q) & 1);
-                Hr[q] += fq * rr;
-                Hi[q] += fq * ri;
-#pragma unroll
-                for (int p = 0; p <= q; ++p, ++idx) {
-                    const double f = fq * double((k >> p) & 1);
-                    HHr[idx] += f * rr;
-                    HHi[idx] += f * ri;
-                }
-            }
-        }
+// rho(x) as the (complex) weight of the pair sums S_PQ = sum_x x_P x_Q rho(x).
+struct RhoWeight {
+    const double2 *rho;
+    __device__ __forceinline__ void operator()(int64_t x, double (&w)[2]) const {
+        const double2 r = rho[x];
+        w[0] = r.x;
+        w[1] = r.y;
     }
-    const int lane = threadIdx.x & 31;
-    auto add = [&](int P, int Q, double vr, double vi) {
-        vr = warp_sum(vr);
-        vi = warp_sum(vi);
-        if (lane == 0) {
-            atomicAdd(&acc[2 * (P * n + Q)], vr);
-            atomicAdd(&acc[2 * (P * n + Q) + 1], vi);
-        }
-    };
-    for (int P = 0; P < s; ++P) {
-        const double fP = double((t >> P) & 1);
-        for (int Q = P; Q < s; ++Q) {  // both bits low: fixed for this thread
-            const double f = fP * double((t >> Q) & 1);
-            add(P, Q, f * Rr, f * Ri);
-        }
-#pragma unroll
-        for (int q = 0; q < PAIR_HB; ++q)  // P low, Q = s + q high
-            if (q < h) add(P, s + q, fP * Hr[q], fP * Hi[q]);
-    }
-    int idx = 0;
-#pragma unroll
-    for (int q = 0; q < PAIR_HB; ++q)
-#pragma unroll
-        for (int p = 0; p <= q; ++p, ++idx)
-            if (q < h) add(s + p, s + q, HHr[idx], HHi[idx]);
-    __syncthreads();
-    for (int k = threadIdx.x; k < 2 * n * n; k += blockDim.x)
-        partials[(int64_t)blockIdx.x * 2 * ADJ_MAXQ * ADJ_MAXQ + k] = acc[k];
-}
-
-__global__ void k_sum_pairs(const double *partials, int nblocks, int n, double *out) {
-    for (int k = threadIdx.x; k < 2 * n * n; k += blockDim.x) {
-        double s = 0.0;
-        for (int b = 0; b < nblocks; ++b) s += partials[(int64_t)b * 2 * ADJ_MAXQ * ADJ_MAXQ + k];
-        out[k] = s;
-    }
-}
+};
 
 }  // namespace emusv
 
@@ -459,22 +394,17 @@ int emusv_adjoint_step(int nqubits, int dtype, double dt, const double *omegas,
     EMUSV_CHECK_LAUNCH();
     {
         ProfScope ps_(PROF_ADJOINT, s);
-        k_sum_adj<<<1, BLOCK, 0, s>>>(W.part_c, gx, 4 * n + 2, W.scal->sums);
+        k_sum_adj<<<4 * n + 2, 32, 0, s>>>(W.part_c, gx, W.scal->sums);
     }
     EMUSV_CHECK_LAUNCH();
     const bool want_pairs = g_deltas || g_interaction;
     if (want_pairs) {
         // the pair partials reuse part_h/part_o (both Lanczos runs are finished)
-        const int hb = n < PAIR_HB ? n : PAIR_HB;
-        const int gp = (int)(((int64_t(1) << (n - hb)) + BLOCK - 1) / BLOCK);
-        const size_t per = 2 * ADJ_MAXQ * ADJ_MAXQ;
-        if ((size_t)gp * per > 2 * part_bytes() / sizeof(double)) return EMUSV_BAD_ARGUMENT;
-        {
-            ProfScope ps_(PROF_ADJOINT, s);
-            k_pairs<<<gp, BLOCK, 0, s>>>(rho, n, W.part_h);
-            k_sum_pairs<<<1, BLOCK, 0, s>>>(W.part_h, gp, n, W.scal->pairs);
-        }
-        EMUSV_CHECK_LAUNCH();
+        if (ps_partials(n, 2) > 2 * part_bytes() / sizeof(double)) return EMUSV_BAD_ARGUMENT;
+        ProfScope ps_(PROF_ADJOINT, s);
+        const int st2 = launch_pair_sums<2, true>(RhoWeight{reinterpret_cast<const double2 *>(rho)}, n, W.part_h,
+                                                  W.scal->pairs, false, s);
+        if (st2) return st2;
     }
     AdjScal H;
     EMUSV_CHECK(cudaMemcpyAsync(&H, W.scal, sizeof(AdjScal), cudaMemcpyDeviceToHost, s));

@@ -4,6 +4,7 @@
 #include <string.h>
 
 #include "hpsi_kernel.cuh"
+#include "pairsums.cuh"
 #include "profile.cuh"
 
 namespace emusv {
@@ -183,120 +184,22 @@ __global__ void k_sum_partials(const double *partials, int nblocks, double *out)
         for (int k = 0; k < NRED; ++k) out[k] = v[k];
 }
 
-// Occupation / correlation in one pass.  For a grid-stride loop with a power-of-two
-// stride S, the low log2(S) bits of a thread's indices are fixed: those bits get the
-// thread's total weight once; the bits above vary with the loop and are accumulated
-// per amplitude.  CORR additionally accumulates the n*n pair sums (n <= 32).
-template <typename R, bool CORR>
-__global__ void __launch_bounds__(BLOCK) k_occupation(const void *psi_, int n, double *partials) {
-    typedef typename cvec<R>::T C;
-    const C *psi = reinterpret_cast<const C *>(psi_);
-    __shared__ double red[(BLOCK / 32) * MAXQ];
-    const i64 D = i64(1) << n;
-    const i64 S = (i64)gridDim.x * blockDim.x;  // power of two by construction
-    int sbits = 0;
-    while ((i64(1) << sbits) < S) ++sbits;
-    const i64 start = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    double total = 0.0;
-    double hi[MAXQ];
-#pragma unroll
-    for (int p = 0; p < MAXQ; ++p) hi[p] = 0.0;
-    for (i64 x = start; x < D; x += S) {
-        const C a = psi[x];
-        const double w = double(a.x) * double(a.x) + double(a.y) * double(a.y);
-        total += w;
-#pragma unroll
-        for (int p = 0; p < MAXQ; ++p)
-            if (p >= sbits && p < n && ((x >> p) & 1)) hi[p] += w;
+// |psi_x|^2 as the weight of the pair sums (occupations and correlations).
+template <typename R> struct PsiWeight {
+    const typename cvec<R>::T *psi;
+    __device__ __forceinline__ void operator()(i64 x, double (&w)[1]) const {
+        const typename cvec<R>::T a = psi[x];
+        w[0] = double(a.x) * double(a.x) + double(a.y) * double(a.y);
     }
-    // occupation by qubit i (bit p = n-1-i)
-    double occ[MAXQ];
-#pragma unroll
-    for (int p = 0; p < MAXQ; ++p) occ[p] = (p < sbits) ? (((start >> p) & 1) ? total : 0.0) : hi[p];
-    // block reduction of MAXQ values
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int p = 0; p < MAXQ; ++p) occ[p] = warp_sum(occ[p]);
-    if (lane == 0)
-        for (int p = 0; p < MAXQ; ++p) red[warp * MAXQ + p] = occ[p];
-    __syncthreads();
-    if (threadIdx.x < MAXQ) {
-        double s = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w * MAXQ + threadIdx.x];
-        partials[(i64)blockIdx.x * MAXQ + threadIdx.x] = s;
-    }
-}
+};
 
-// Pair sums sum_x |psi_x|^2 x_p x_q for p <= q: one block per (tile of amplitudes),
-// each thread accumulates the n(n+1)/2 pairs of its amplitudes in shared memory rows.
-template <typename R>
-__global__ void __launch_bounds__(BLOCK) k_correlation(const void *psi_, int n, double *partials) {
-    typedef typename cvec<R>::T C;
-    const C *psi = reinterpret_cast<const C *>(psi_);
-    __shared__ double acc[MAXQ * MAXQ];
-    for (int k = threadIdx.x; k < MAXQ * MAXQ; k += blockDim.x) acc[k] = 0.0;
-    __syncthreads();
-    const i64 D = i64(1) << n;
-    const i64 S = (i64)gridDim.x * blockDim.x;
-    // each thread handles the pair rows p = lane-strided, after a warp shares weights
-    const int lane = threadIdx.x & 31;
-    double rowacc[MAXQ];
-#pragma unroll
-    for (int q = 0; q < MAXQ; ++q) rowacc[q] = 0.0;
-    for (i64 x0 = (i64)blockIdx.x * blockDim.x + (threadIdx.x & ~31); x0 < D; x0 += S) {
-        // the warp loads 32 consecutive amplitudes; lane p then accumulates row p
-        const i64 xl = x0 + lane;
-        double w = 0.0;
-        if (xl < D) {
-            const C a = psi[xl];
-            w = double(a.x) * double(a.x) + double(a.y) * double(a.y);
-        }
-        for (int j = 0; j < 32; ++j) {
-            const double wj = __shfl_sync(0xffffffffu, w, j);
-            const i64 xj = x0 + j;
-            if (lane < n && ((xj >> lane) & 1)) {
-#pragma unroll
-                for (int q = 0; q < MAXQ; ++q)
-                    if (q < n && ((xj >> q) & 1)) rowacc[q] += wj;
-            }
-        }
-    }
-    if (lane < n) {
-        for (int q = 0; q < n; ++q) atomicAdd(&acc[lane * MAXQ + q], rowacc[q]);
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
-        const int p = k / n, q = k % n;
-        partials[(i64)blockIdx.x * n * n + k] = acc[p * MAXQ + q];
-    }
-}
-
-// Sum occupation partials into qubit order: out[i] = sum_b partials[b][n-1-i].
-__global__ void k_finish_occ(const double *partials, int nblocks, int n, int stride, double *out) {
-    const int i = threadIdx.x;
-    if (i >= n) return;
-    const int p = n - 1 - i;
-    double s = 0.0;
-    for (int b = 0; b < nblocks; ++b) s += partials[(i64)b * stride + p];
-    out[i] = s;
-}
-
-__global__ void k_finish_corr(const double *partials, int nblocks, int n, double *out) {
-    for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
-        const int i = k / n, j = k % n;
-        const int p = n - 1 - i, q = n - 1 - j;
-        double s = 0.0;
-        for (int b = 0; b < nblocks; ++b) s += partials[(i64)b * n * n + p * n + q];
-        out[k] = s;
-    }
-}
-
-static int occ_grid(int n) {
-    // power-of-two grid with at most one block per 256 amplitudes
-    i64 D = i64(1) << n;
-    i64 g = 1;
-    while (g * 2 * BLOCK <= D && g * 2 <= (i64)sm_count() * 4) g *= 2;
-    return (int)g;
+template <bool PAIRS>
+static int launch_psi_sums(int dtype, const void *psi, int n, double *part, double *out, cudaStream_t s) {
+    ProfScope ps_(PROF_OBS, s);
+    if (dtype == EMUSV_C128)
+        return launch_pair_sums<1, PAIRS>(PsiWeight<double>{reinterpret_cast<const double2 *>(psi)}, n, part, out,
+                                          true, s);
+    return launch_pair_sums<1, PAIRS>(PsiWeight<float>{reinterpret_cast<const float2 *>(psi)}, n, part, out, true, s);
 }
 
 }  // namespace emusv
@@ -334,9 +237,11 @@ const char *emusv_status_string(int status) {
 // Scratch of the observables: FP64 partial sums, and for the moments of H on registers
 // wider than one pass-L tile (emusv_expect through the streaming passes) one vector of
 // the register's size for the flips of the high bits.
-static size_t scratch_head_bytes() {
+static size_t scratch_head_bytes(int n) {
     const size_t per = (size_t)MAXQ * MAXQ > NRED ? (size_t)MAXQ * MAXQ : NRED;
-    return ((sizeof(double) * ((size_t)max_grid_blocks() * per + 64)) + 255) / 256 * 256;
+    size_t d = (size_t)max_grid_blocks() * per + 64;
+    if (d < ps_partials(n, 1)) d = ps_partials(n, 1);
+    return (sizeof(double) * d + 255) / 256 * 256;
 }
 static bool expect_by_passes(int dtype, int n) {
     return (dtype == EMUSV_C64 || dtype == EMUSV_C128) && lanczos_h_first(dtype, n);
@@ -344,7 +249,7 @@ static bool expect_by_passes(int dtype, int n) {
 
 size_t emusv_scratch_bytes(int nqubits, int dtype) {
     if (nqubits < 1 || nqubits > EMUSV_MAX_QUBITS) return 0;
-    size_t b = scratch_head_bytes();
+    size_t b = scratch_head_bytes(nqubits);
     if (expect_by_passes(dtype, nqubits)) b += (size_t(1) << nqubits) * (dtype == EMUSV_C128 ? 16 : 8);
     return b;
 }
@@ -411,7 +316,7 @@ int emusv_expect(int nqubits, int dtype, const double *omegas, const double *del
     if (expect_by_passes(dtype, nqubits) && !P.noisy) {
         // streaming passes: X_high psi into the scratch vector, then H psi per tile
         if (reinterpret_cast<uintptr_t>(psi) & 15) return EMUSV_BAD_ARGUMENT;
-        unsigned char *vec = reinterpret_cast<unsigned char *>(scratch) + scratch_head_bytes();
+        unsigned char *vec = reinterpret_cast<unsigned char *>(scratch) + scratch_head_bytes(nqubits);
         double *part_h = sums + 64;  // the pass H kernels' partials (not used here)
         unsigned *cnt = reinterpret_cast<unsigned *>(part_h + (size_t)max_grid_blocks() * NRED);
         st = lz_moments(dtype, P, psi, vec, partials, part_h, cnt, device_error_word(), s, &grid);
@@ -442,26 +347,7 @@ int emusv_occupation(int nqubits, int dtype, const void *psi, double *occ_dev, v
         scratch_bytes < emusv_scratch_bytes(nqubits, dtype) || (dtype != EMUSV_C128 && dtype != EMUSV_C64))
         return EMUSV_BAD_ARGUMENT;
     cudaStream_t s = as_stream(stream);
-    double *partials = reinterpret_cast<double *>(scratch);
-    const int grid = occ_grid(nqubits);
-    const int block = (i64(1) << nqubits) < BLOCK ? 32 : BLOCK;
-    if (dtype == EMUSV_C128)
-        {
-            ProfScope ps_(PROF_OBS, s);
-            k_occupation<double, false><<<grid, block, 0, s>>>(psi, nqubits, partials);
-        }
-    else
-        {
-            ProfScope ps_(PROF_OBS, s);
-            k_occupation<float, false><<<grid, block, 0, s>>>(psi, nqubits, partials);
-        }
-    EMUSV_CHECK_LAUNCH();
-    {
-        ProfScope ps_(PROF_OBS, s);
-        k_finish_occ<<<1, 32, 0, s>>>(partials, grid, nqubits, MAXQ, occ_dev);
-    }
-    EMUSV_CHECK_LAUNCH();
-    return EMUSV_OK;
+    return launch_psi_sums<false>(dtype, psi, nqubits, reinterpret_cast<double *>(scratch), occ_dev, s);
 }
 
 int emusv_correlation(int nqubits, int dtype, const void *psi, double *corr_dev, void *scratch,
@@ -470,26 +356,7 @@ int emusv_correlation(int nqubits, int dtype, const void *psi, double *corr_dev,
         scratch_bytes < emusv_scratch_bytes(nqubits, dtype) || (dtype != EMUSV_C128 && dtype != EMUSV_C64))
         return EMUSV_BAD_ARGUMENT;
     cudaStream_t s = as_stream(stream);
-    double *partials = reinterpret_cast<double *>(scratch);
-    int grid = occ_grid(nqubits);
-    if (grid > max_grid_blocks()) grid = max_grid_blocks();
-    if (dtype == EMUSV_C128)
-        {
-            ProfScope ps_(PROF_OBS, s);
-            k_correlation<double><<<grid, BLOCK, 0, s>>>(psi, nqubits, partials);
-        }
-    else
-        {
-            ProfScope ps_(PROF_OBS, s);
-            k_correlation<float><<<grid, BLOCK, 0, s>>>(psi, nqubits, partials);
-        }
-    EMUSV_CHECK_LAUNCH();
-    {
-        ProfScope ps_(PROF_OBS, s);
-        k_finish_corr<<<1, BLOCK, 0, s>>>(partials, grid, nqubits, corr_dev);
-    }
-    EMUSV_CHECK_LAUNCH();
-    return EMUSV_OK;
+    return launch_psi_sums<true>(dtype, psi, nqubits, reinterpret_cast<double *>(scratch), corr_dev, s);
 }
 
 }  // extern "C"

@@ -9,64 +9,78 @@ namespace emusv {
 
 constexpr int RHO_THREADS = 256;
 
-// partials[block][p][4]: sum over pairs (x0, x1 = x0 | 2^p) of |psi_x0|^2, |psi_x1|^2 and
-// psi_x1 conj(psi_x0) (re, im), for every bit p.
+// part[4 p + c][block]: sums over the pairs (x0, x1 = x0 | 2^p) of |psi_x0|^2, |psi_x1|^2 and
+// psi_x1 conj(psi_x0) (re, im).  Blocks with blockIdx.y = g take the bits 3g..3g+2: a thread
+// reads the 8 amplitudes that differ in them, so the state is read once for three bits (from
+// the L2 after the first) and all groups run together.  Bound by those reads and the launch:
+// n = 19 complex128 31 us before (one bit after the other, each reading the whole state).
+constexpr int RHO_G = 3;
 template <typename R>
-__global__ void __launch_bounds__(RHO_THREADS) k_qubit_rho(const void *psi_, int n, double *partials) {
+__global__ void __launch_bounds__(RHO_THREADS) k_qubit_rho(const void *psi_, int n, double *part) {
     typedef typename cvec<R>::T C;
     const C *psi = reinterpret_cast<const C *>(psi_);
-    __shared__ double red[(RHO_THREADS / 32) * 4];
-    const i64 half = i64(1) << (n - 1);
+    constexpr int NA = 1 << RHO_G, NV = 4 * RHO_G;
+    __shared__ double red[(RHO_THREADS / 32) * NV];
+    const int b0 = RHO_G * blockIdx.y, m = n - b0 < RHO_G ? n - b0 : RHO_G, na = 1 << m;
+    const i64 count = i64(1) << (n - m), lowmask = (i64(1) << b0) - 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int p = 0; p < n; ++p) {
-        const i64 lowmask = (i64(1) << p) - 1;
-        double a00 = 0.0, a11 = 0.0, cr = 0.0, ci = 0.0;
-        for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < half; i += (i64)gridDim.x * blockDim.x) {
-            const i64 x0 = ((i >> p) << (p + 1)) | (i & lowmask);
-            const C a = psi[x0], b = psi[x0 | (i64(1) << p)];
-            const double ar = double(a.x), ai = double(a.y), br = double(b.x), bi = double(b.y);
-            a00 += ar * ar + ai * ai;
-            a11 += br * br + bi * bi;
-            cr += br * ar + bi * ai;  // b conj(a)
-            ci += bi * ar - br * ai;
-        }
-        a00 = warp_sum(a00);
-        a11 = warp_sum(a11);
-        cr = warp_sum(cr);
-        ci = warp_sum(ci);
-        if (lane == 0) {
-            red[warp * 4 + 0] = a00;
-            red[warp * 4 + 1] = a11;
-            red[warp * 4 + 2] = cr;
-            red[warp * 4 + 3] = ci;
-        }
-        __syncthreads();
-        if (threadIdx.x < 4) {
-            double t = 0.0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w * 4 + threadIdx.x];
-            partials[((i64)blockIdx.x * MAXQ + p) * 4 + threadIdx.x] = t;
-        }
-        __syncthreads();
+    double acc[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) acc[k] = 0.0;
+    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (i64)gridDim.x * blockDim.x) {
+        const i64 x0 = ((i >> b0) << (b0 + m)) | (i & lowmask);
+        C v[NA];
+#pragma unroll
+        for (int a = 0; a < NA; ++a) v[a] = a < na ? psi[x0 | ((i64)a << b0)] : cmake<C>(0.0, 0.0);
+#pragma unroll
+        for (int q = 0; q < RHO_G; ++q)
+#pragma unroll
+            for (int a = 0; a < NA; ++a) {
+                if ((a >> q) & 1) continue;
+                const double ar = double(v[a].x), ai = double(v[a].y);
+                const double br = double(v[a | (1 << q)].x), bi = double(v[a | (1 << q)].y);
+                acc[4 * q] += ar * ar + ai * ai;
+                acc[4 * q + 1] += br * br + bi * bi;
+                acc[4 * q + 2] += br * ar + bi * ai;  // b conj(a)
+                acc[4 * q + 3] += bi * ar - br * ai;
+            }
+    }
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        acc[k] = warp_sum(acc[k]);
+        if (lane == 0) red[warp * NV + k] = acc[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 4 * m) {
+        double t = 0.0;
+        for (int w = 0; w < RHO_THREADS / 32; ++w) t += red[w * NV + threadIdx.x];
+        part[((i64)4 * b0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
     }
 }
 
-// rho[i] (qubit i = bit n-1-i): 2x2 complex row-major, 8 doubles: [00, 01, 10, 11].
-__global__ void k_finish_rho(const double *partials, int nb, int n, double *rho) {
-    const int i = threadIdx.x;
-    if (i >= n) return;
-    const int p = n - 1 - i;
-    double v[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int b = 0; b < nb; ++b)
-        for (int k = 0; k < 4; ++k) v[k] += partials[((i64)b * MAXQ + p) * 4 + k];
+// rho[i] (qubit i = bit n-1-i): 2x2 complex row-major, 8 doubles: [00, 01, 10, 11].  One
+// block per qubit, one warp per sum.
+__global__ void __launch_bounds__(128) k_finish_rho(const double *part, int nb, int n, double *rho) {
+    const int i = blockIdx.x, p = n - 1 - i, k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double v = 0.0;
+#pragma unroll 4
+    for (int b = lane; b < nb; b += 32) v += part[((i64)4 * p + k) * nb + b];
+    v = warp_sum(v);
+    if (lane) return;
     double *o = rho + 8 * i;
-    o[0] = v[0];  // rho_00
-    o[1] = 0.0;
-    o[2] = v[2];  // rho_01 = sum psi_0 conj(psi_1) = conj(rho_10)
-    o[3] = -v[3];
-    o[4] = v[2];  // rho_10 = sum psi_1 conj(psi_0)
-    o[5] = v[3];
-    o[6] = v[1];  // rho_11
-    o[7] = 0.0;
+    if (k == 0) {
+        o[0] = v;  // rho_00
+        o[1] = 0.0;
+    } else if (k == 1) {
+        o[6] = v;  // rho_11
+        o[7] = 0.0;
+    } else if (k == 2) {
+        o[2] = v;  // rho_01 = sum psi_0 conj(psi_1) = conj(rho_10)
+        o[4] = v;  // rho_10 = sum psi_1 conj(psi_0)
+    } else {
+        o[3] = -v;
+        o[5] = v;
+    }
 }
 
 template <typename R>
@@ -88,10 +102,12 @@ k_apply_1q(void *psi_, int n, int p, double o00r, double o00i, double o01r, doub
     }
 }
 
+// Blocks per group of bits: eight amplitudes a thread, at most four blocks per SM over all
+// groups.
 static int rho_grid(int n) {
-    const i64 half = i64(1) << (n - 1);
-    i64 g = (half + RHO_THREADS - 1) / RHO_THREADS;
-    const i64 cap = (i64)sm_count() * 4;
+    const i64 count = n > RHO_G ? i64(1) << (n - RHO_G) : 1;
+    const int groups = (n + RHO_G - 1) / RHO_G;
+    const i64 g = (count + RHO_THREADS - 1) / RHO_THREADS, cap = ((i64)sm_count() * 4 + groups - 1) / groups;
     return (int)(g < cap ? g : cap);
 }
 
@@ -117,9 +133,10 @@ int emusv_qubit_densities(int nqubits, int dtype, const void *psi, double *rho_d
     const int g = rho_grid(nqubits);
     {
         ProfScope ps_(PROF_OBS, s);
-        if (dtype == EMUSV_C128) k_qubit_rho<double><<<g, RHO_THREADS, 0, s>>>(psi, nqubits, partials);
-        else k_qubit_rho<float><<<g, RHO_THREADS, 0, s>>>(psi, nqubits, partials);
-        k_finish_rho<<<1, 32, 0, s>>>(partials, g, nqubits, rho_dev);
+        const dim3 grid(g, (nqubits + RHO_G - 1) / RHO_G);
+        if (dtype == EMUSV_C128) k_qubit_rho<double><<<grid, RHO_THREADS, 0, s>>>(psi, nqubits, partials);
+        else k_qubit_rho<float><<<grid, RHO_THREADS, 0, s>>>(psi, nqubits, partials);
+        k_finish_rho<<<nqubits, 128, 0, s>>>(partials, g, nqubits, rho_dev);
     }
     EMUSV_CHECK_LAUNCH();
     return EMUSV_OK;
