@@ -37,12 +37,16 @@ int arnoldi_run(const HamParams &P, const LindbladJumps *J, int dtype, double dt
 constexpr int ARN_KMAX = 100;                  // largest Arnoldi max_krylov_dim
 constexpr int ARN_M = ARN_KMAX + 2;            // largest extended matrix
 constexpr int ARN_KA = ARN_KMAX + 1;           // finalised basis vectors at most
-// partial row of a pass: z_k = <v_k, w> (re, im), s_k = <v_k, vt>, a = <vt, w>, ||w||^2,
-// ||vt||^2 (pass A); pass B writes its norm at ARN_NORM
-constexpr int ARN_S0 = 2 * ARN_KA, ARN_A0 = 4 * ARN_KA, ARN_NORM = ARN_A0 + 2;
-constexpr int ARN_PS = ARN_A0 + 4;
+// Partial sums of a pass, value-major ([value][block]): per group of ARN_KB basis vectors 32
+// values, (k - group start) * 4 + c with c = 0, 1: z_k = <v_k, w> (re, im), 2, 3: s_k =
+// <v_k, vt>; then a = <vt, w> (re, im), ||w||^2, ||vt||^2 (pass A) and pass B's norm.
+constexpr int ARN_KB = 8;
+constexpr int ARN_GROUPS = (ARN_KA + ARN_KB - 1) / ARN_KB;
+constexpr int ARN_A0 = 32 * ARN_GROUPS, ARN_NORM = ARN_A0 + 4;
+constexpr int ARN_PS = ARN_A0 + 5;
 constexpr int ORTHO_THREADS = 256;
-constexpr int DECIDE_THREADS = 256;
+constexpr int DECIDE_THREADS = 512;
+constexpr int STAGE_THREADS = 1024;
 
 struct ArnState {
     double2 T[ARN_M * ARN_M];  // Hessenberg matrix of H - sigma (row-major [r][c]), basis v_k
@@ -64,31 +68,50 @@ struct ArnState {
 //     combinations of w, vt and V), ||w'||^2.
 // Two streaming passes per iteration; every basis vector but the newest is orthogonalised
 // twice, as in classical Gram-Schmidt with reorthogonalisation.
-template <typename R, int E = 4, int KB = 4>
-__global__ void __launch_bounds__(ORTHO_THREADS)
+//
+// Pass A is the basis read once (nk + 2 vectors).  A block takes chunks of E amplitudes a
+// thread; per group of ARN_KB vectors a thread adds its 32 products and the warp reduces all
+// 32 values at once by a transposing butterfly (31 FP64 shuffles instead of 5 for each value:
+// one value at a time, the shuffles took as long as the loads -- 140 us a pass against 70 us
+// for pass B at 2^20 complex128 amplitudes and 24 vectors), lane l ending with value l, which
+// it adds to the warp's row in shared memory.  Blocks with blockIdx.y = g take every
+// gridDim.y-th group: on registers with fewer chunks than the GPU has blocks, the groups are
+// what fills it.
+__device__ __forceinline__ double warp_transpose_sum(double (&v)[32]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) {
+        const bool up = (lane & m) != 0;
+#pragma unroll
+        for (int i = 0; i < m; ++i) {
+            const double send = up ? v[i] : v[i + m], keep = up ? v[i + m] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+        }
+    }
+    return v[0];  // value `lane`, summed over the warp
+}
+
+constexpr int LAG_E = 4;  // amplitudes per thread and chunk
+template <typename R>
+__global__ void __launch_bounds__(ORTHO_THREADS, 1)
 k_arn_lagdots(const KState *ks, int j, const void *v0_, const unsigned char *basis, i64 D,
               const void *w_, double *part) {
     typedef typename cvec<R>::T C;
     if (ks->status != KS_RUNNING) return;
-    constexpr int NW = ORTHO_THREADS / 32;
-    __shared__ double sc[ARN_M];
-    __shared__ double2 accz[NW][ARN_KA], accs[NW][ARN_KA];
+    constexpr int NW = ORTHO_THREADS / 32, E = LAG_E, KB = ARN_KB;
+    constexpr int EL = sizeof(R) == 8 ? 2 : 4;  // amplitudes whose loads are in flight: 256 bytes a thread
+    __shared__ double acc[NW][ARN_GROUPS][32];
     __shared__ double sa[NW][4];
     const bool has_vt = j >= 1;
-    const int nk = has_vt ? j : 1;
+    const int nk = has_vt ? j : 1, ngroups = (nk + KB - 1) / KB;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int k = tid; k < nk; k += ORTHO_THREADS) sc[k] = ks->scale[k];
-    for (int k = tid; k < NW * ARN_KA; k += ORTHO_THREADS) {
-        (&accz[0][0])[k] = make_double2(0.0, 0.0);
-        (&accs[0][0])[k] = make_double2(0.0, 0.0);
-    }
+    const int g0 = blockIdx.y, gs = gridDim.y;
+    for (int g = g0; g < ngroups; g += gs) acc[warp][g][lane] = 0.0;
     const double st = has_vt ? ks->scale[j] : 0.0;
-    __syncthreads();
     const C *v0 = reinterpret_cast<const C *>(v0_);
     const C *bs = reinterpret_cast<const C *>(basis);
     const C *w = reinterpret_cast<const C *>(w_);
     const C *vt = has_vt ? bs + (i64)j * D : nullptr;
-    auto vk = [&](int k) -> const C * { return k == 0 ? v0 : bs + (i64)k * D; };
     double nw = 0.0, nv = 0.0, ar = 0.0, ai = 0.0;
     const i64 CH = (i64)ORTHO_THREADS * E;
     for (i64 c0 = (i64)blockIdx.x * CH; c0 < D; c0 += (i64)gridDim.x * CH) {
@@ -107,89 +130,76 @@ k_arn_lagdots(const KState *ks, int j, const void *v0_, const unsigned char *bas
                     ti[e] = st * double(b.y);
                 }
             }
-            nw += wr[e] * wr[e] + wi[e] * wi[e];
-            nv += tr[e] * tr[e] + ti[e] * ti[e];
-            ar += tr[e] * wr[e] + ti[e] * wi[e];
-            ai += tr[e] * wi[e] - ti[e] * wr[e];
+            if (g0 == 0) {
+                nw += wr[e] * wr[e] + wi[e] * wi[e];
+                nv += tr[e] * tr[e] + ti[e] * ti[e];
+                ar += tr[e] * wr[e] + ti[e] * wi[e];
+                ai += tr[e] * wi[e] - ti[e] * wr[e];
+            }
         }
-        int k = 0;
-        for (; k < nk; k += KB) {
-            C a[KB][E];
+        for (int g = g0; g < ngroups; g += gs) {
+            double v[4 * KB];
 #pragma unroll
-            for (int kb = 0; kb < KB; ++kb)
+            for (int i = 0; i < 4 * KB; ++i) v[i] = 0.0;
 #pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    const i64 x = c0 + tid + (i64)e * ORTHO_THREADS;
-                    a[kb][e] = (k + kb < nk && x < D) ? vk(k + kb)[x] : cmake<C>(0.0, 0.0);
-                }
-            double zr[KB], zi[KB], sr[KB], si[KB];
-#pragma unroll
-            for (int kb = 0; kb < KB; ++kb) {
-                zr[kb] = zi[kb] = sr[kb] = si[kb] = 0.0;
-#pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    const double px = double(a[kb][e].x), py = double(a[kb][e].y);
-                    zr[kb] += px * wr[e] + py * wi[e];
-                    zi[kb] += px * wi[e] - py * wr[e];
-                    sr[kb] += px * tr[e] + py * ti[e];
-                    si[kb] += px * ti[e] - py * tr[e];
-                }
-            }
-#pragma unroll
-            for (int kb = 0; kb < KB; ++kb) {
-                zr[kb] = warp_sum(zr[kb]);
-                zi[kb] = warp_sum(zi[kb]);
-                if (has_vt) {
-                    sr[kb] = warp_sum(sr[kb]);
-                    si[kb] = warp_sum(si[kb]);
-                }
-            }
-            if (lane == 0) {
+            for (int h = 0; h < E; h += EL) {
+                C a[KB][EL];
 #pragma unroll
                 for (int kb = 0; kb < KB; ++kb) {
-                    if (k + kb >= nk) break;
-                    accz[warp][k + kb].x += zr[kb];
-                    accz[warp][k + kb].y += zi[kb];
-                    accs[warp][k + kb].x += sr[kb];
-                    accs[warp][k + kb].y += si[kb];
+                    const int k = g * KB + kb;
+                    const C *vk = k == 0 ? v0 : bs + (i64)k * D;
+#pragma unroll
+                    for (int e = 0; e < EL; ++e) {
+                        const i64 x = c0 + tid + (i64)(h + e) * ORTHO_THREADS;
+                        a[kb][e] = (k < nk && x < D) ? vk[x] : cmake<C>(0.0, 0.0);
+                    }
                 }
+#pragma unroll
+                for (int kb = 0; kb < KB; ++kb)
+#pragma unroll
+                    for (int e = 0; e < EL; ++e) {
+                        const double px = double(a[kb][e].x), py = double(a[kb][e].y);
+                        v[4 * kb] += px * wr[h + e] + py * wi[h + e];
+                        v[4 * kb + 1] += px * wi[h + e] - py * wr[h + e];
+                        v[4 * kb + 2] += px * tr[h + e] + py * ti[h + e];
+                        v[4 * kb + 3] += px * ti[h + e] - py * tr[h + e];
+                    }
             }
+            acc[warp][g][lane] += warp_transpose_sum(v);
         }
     }
-    nw = warp_sum(nw);
-    nv = warp_sum(nv);
-    ar = warp_sum(ar);
-    ai = warp_sum(ai);
-    if (lane == 0) {
-        sa[warp][0] = ar;
-        sa[warp][1] = ai;
-        sa[warp][2] = nw;
-        sa[warp][3] = nv;
+    if (g0 == 0) {
+        nw = warp_sum(nw);
+        nv = warp_sum(nv);
+        ar = warp_sum(ar);
+        ai = warp_sum(ai);
+        if (lane == 0) {
+            sa[warp][0] = ar;
+            sa[warp][1] = ai;
+            sa[warp][2] = nw;
+            sa[warp][3] = nv;
+        }
     }
     __syncthreads();
-    double *row = part + (i64)blockIdx.x * ARN_PS;
-    for (int k = tid; k < nk; k += ORTHO_THREADS) {
-        double2 z = make_double2(0.0, 0.0), q = make_double2(0.0, 0.0);
-        for (int u = 0; u < NW; ++u) {
-            z.x += accz[u][k].x;
-            z.y += accz[u][k].y;
-            q.x += accs[u][k].x;
-            q.y += accs[u][k].y;
-        }
-        row[2 * k] = sc[k] * z.x;
-        row[2 * k + 1] = sc[k] * z.y;
-        row[ARN_S0 + 2 * k] = sc[k] * q.x;
-        row[ARN_S0 + 2 * k + 1] = sc[k] * q.y;
+    const size_t nb = gridDim.x;
+    for (int g = g0 + gs * warp; g < ngroups; g += gs * NW) {  // one warp per group, lane = value
+        const int k = g * KB + (lane >> 2);
+        double t = 0.0;
+#pragma unroll
+        for (int u = 0; u < NW; ++u) t += acc[u][g][lane];
+        if (k < nk) part[(size_t)(32 * g + lane) * nb + blockIdx.x] = ks->scale[k] * t;
     }
-    if (tid < 4) {
+    if (g0 == 0 && tid < 4) {
         double t = 0.0;
         for (int u = 0; u < NW; ++u) t += sa[u][tid];
-        row[ARN_A0 + tid] = t;
+        part[(size_t)(ARN_A0 + tid) * nb + blockIdx.x] = t;
     }
 }
 
 // Pass B: w' = cw w - ct vt - sum cw1_l v_l (in place over w) and, for j >= 1, the
 // corrected v_j = cv vt - sum cvj_l v_l (in place over vt, stored with scale 1); ||w'||^2.
+// The chunks run from the last to the first, pass A's from the first to the last: each pass
+// begins on the part of the basis that the other left in the L2.
 template <typename R, int E = 4, int KB = 4>
 __global__ void __launch_bounds__(ORTHO_THREADS)
 k_arn_lagupdate(const KState *ks, const ArnState *as, int j, const void *v0_, unsigned char *basis,
@@ -217,8 +227,9 @@ k_arn_lagupdate(const KState *ks, const ArnState *as, int j, const void *v0_, un
     C *vt = has_vt ? bs + (i64)j * D : nullptr;
     auto vk = [&](int k) -> const C * { return k == 0 ? v0 : bs + (i64)k * D; };
     double nacc = 0.0;
-    const i64 CH = (i64)ORTHO_THREADS * E;
-    for (i64 c0 = (i64)blockIdx.x * CH; c0 < D; c0 += (i64)gridDim.x * CH) {
+    const i64 CH = (i64)ORTHO_THREADS * E, nch = (D + CH - 1) / CH;
+    for (i64 ch = nch - 1 - blockIdx.x; ch >= 0; ch -= gridDim.x) {
+        const i64 c0 = ch * CH;
         double ur[E], ui[E], qr[E], qi[E];
 #pragma unroll
         for (int e = 0; e < E; ++e) {
@@ -279,15 +290,16 @@ k_arn_lagupdate(const KState *ks, const ArnState *as, int j, const void *v0_, un
     if (tid == 0) {
         double t = 0.0;
         for (int u = 0; u < NW; ++u) t += snorm[u];
-        part[(i64)blockIdx.x * ARN_PS + ARN_NORM] = t;
+        part[(size_t)ARN_NORM * gridDim.x + blockIdx.x] = t;
     }
 }
 
-// Sum of value i of the pass partial rows over nb blocks by one warp (lanes stride over
-// the blocks, then a fixed shuffle tree: deterministic).  Result in every lane.
+// Sum of value i of a pass over its nb blocks by one warp (lanes stride over the blocks,
+// then a fixed shuffle tree: deterministic).  Result in every lane.
 __device__ __forceinline__ double arn_sum_warp(const double *part, int nb, int i) {
     double t = 0.0;
-    for (int b = threadIdx.x & 31; b < nb; b += 32) t += part[(i64)b * ARN_PS + i];
+#pragma unroll 4
+    for (int b = threadIdx.x & 31; b < nb; b += 32) t += part[(size_t)i * nb + b];
     return warp_sum(t);
 }
 
@@ -296,8 +308,11 @@ __device__ __forceinline__ double2 cmulc(double2 a, double2 b) {  // conj(a) b
 }
 
 // After pass A of iteration j: the lagged correction of v_j and of column j-1, column j of
-// T, ||H v_j|| (krylov_exp.py:52), and pass B's coefficients (see the pass comments).
-__global__ void __launch_bounds__(DECIDE_THREADS)
+// T, ||H v_j|| (krylov_exp.py:52), and pass B's coefficients (see the pass comments).  One
+// block, latency-bound: one warp per partial sum and per row of T s, every sum over k by the
+// lanes of a warp (2^20 amplitudes, 47 iterations: 50 us a stage before, with one thread
+// walking T and the sums).
+__global__ void __launch_bounds__(STAGE_THREADS)
 k_arn_lagstage(KState *ks, ArnState *as, int j, const double *part, int nb) {
     if (ks->status != KS_RUNNING) return;
     __shared__ double2 zs[ARN_M], ss[ARN_M], hs[ARN_M], cc[ARN_M];
@@ -305,105 +320,109 @@ k_arn_lagstage(KState *ks, ArnState *as, int j, const double *part, int nb) {
     __shared__ double salpha;
     __shared__ int bad;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int NWD = DECIDE_THREADS / 32;
+    constexpr int NWD = STAGE_THREADS / 32;
     const bool has_vt = j >= 1;
     const int nk = has_vt ? j : 1;
     if (tid == 0) bad = 0;
-    for (int k = warp; k < nk; k += NWD) {  // one warp per value
-        const double2 z = make_double2(arn_sum_warp(part, nb, 2 * k), arn_sum_warp(part, nb, 2 * k + 1));
-        const double2 q = make_double2(arn_sum_warp(part, nb, ARN_S0 + 2 * k),
-                                       arn_sum_warp(part, nb, ARN_S0 + 2 * k + 1));
-        if (lane == 0) {
-            zs[k] = z;
-            ss[k] = has_vt ? q : make_double2(0.0, 0.0);
-        }
-    }
-    if (warp == NWD - 1) {
-        for (int i = 0; i < 4; ++i) {
-            const double v = arn_sum_warp(part, nb, ARN_A0 + i);
-            if (lane == 0) sa[i] = v;
+    for (int i = warp; i < 4 * nk + 4; i += NWD) {  // value 4 k + c, then the four of vt and w
+        const double v = arn_sum_warp(part, nb, i < 4 * nk ? i : ARN_A0 + i - 4 * nk);
+        if (lane) continue;
+        if (i >= 4 * nk) {
+            sa[i - 4 * nk] = v;
+        } else if (i & 2) {
+            (&ss[i >> 2].x)[i & 1] = has_vt ? v : 0.0;
+        } else {
+            (&zs[i >> 2].x)[i & 1] = v;
         }
     }
     __syncthreads();
-    if (tid == 0) {
+    const double beta = has_vt ? ks->r[j - 1] : 0.0;
+    if (warp == 0) {
         double alpha = 1.0;
         if (has_vt) {
             double s2 = 0.0;
-            for (int k = 0; k < nk; ++k) s2 += ss[k].x * ss[k].x + ss[k].y * ss[k].y;
+            for (int k = lane; k < nk; k += 32) s2 += ss[k].x * ss[k].x + ss[k].y * ss[k].y;
+            s2 = warp_sum(s2);
             const double a2 = sa[3] - s2;  // ||vt||^2 - |V^H vt|^2
             alpha = a2 > 0.0 ? sqrt(a2) : 0.0;
-            if (!(alpha > 0.0) || !isfinite(alpha)) bad = 1;
-            const double beta = ks->r[j - 1];
-            for (int l = 0; l < j; ++l) {  // column j-1: w'_{j-1} = beta (alpha v_j + V s)
-                double2 &t = as->T[l * ARN_M + (j - 1)];
-                t.x += beta * ss[l].x;
-                t.y += beta * ss[l].y;
-            }
-            as->T[j * ARN_M + (j - 1)] = make_double2(beta * alpha, 0.0);
-            ks->r[j - 1] = beta * alpha;
         }
-        salpha = alpha;
+        if (lane == 0) {
+            if (!(alpha > 0.0) || !isfinite(alpha)) bad = 1;
+            salpha = alpha;
+        }
+    } else if (has_vt) {  // column j-1: w'_{j-1} = beta (alpha v_j + V s)
+        for (int l = tid - 32; l < j; l += STAGE_THREADS - 32) {
+            double2 &t = as->T[l * ARN_M + (j - 1)];
+            t.x += beta * ss[l].x;
+            t.y += beta * ss[l].y;
+        }
     }
     __syncthreads();
     const double alpha = salpha;
-    // (T s)_l for l <= j over the columns k < j (Hessenberg rows: k >= l - 1)
-    for (int l = tid; l <= j; l += DECIDE_THREADS) {
+    if (has_vt && tid == 0) {
+        as->T[j * ARN_M + (j - 1)] = make_double2(beta * alpha, 0.0);
+        ks->r[j - 1] = beta * alpha;
+    }
+    if (has_vt && warp == 0) {  // <v_j, w> = (<vt, w> - s^H z) / alpha
+        double2 p = make_double2(0.0, 0.0);
+        for (int k = lane; k < nk; k += 32) {
+            const double2 q = cmulc(ss[k], zs[k]);
+            p.x += q.x;
+            p.y += q.y;
+        }
+        p.x = warp_sum(p.x);
+        p.y = warp_sum(p.y);
+        if (lane == 0) zs[j] = make_double2((sa[0] - p.x) / alpha, (sa[1] - p.y) / alpha);
+    }
+    __syncthreads();
+    // (T s)_l for l <= j over the columns k < j (Hessenberg rows: k >= l - 1), a warp per row
+    for (int l = warp; l <= j; l += NWD) {
         double2 acc = make_double2(0.0, 0.0);
         if (has_vt)
-            for (int k = l > 0 ? l - 1 : 0; k < j; ++k) {
+            for (int k = (l > 0 ? l - 1 : 0) + lane; k < j; k += 32) {
                 const double2 t = as->T[l * ARN_M + k], q = ss[k];
                 acc.x += t.x * q.x - t.y * q.y;
                 acc.y += t.x * q.y + t.y * q.x;
             }
-        hs[l] = acc;
-    }
-    __syncthreads();
-    if (tid == 0) {  // <v_j, w> = (<vt, w> - s^H z) / alpha
-        if (has_vt) {
-            double2 t = make_double2(sa[0], sa[1]);
-            for (int k = 0; k < nk; ++k) {
-                const double2 p = cmulc(ss[k], zs[k]);
-                t.x -= p.x;
-                t.y -= p.y;
-            }
-            zs[j] = make_double2(t.x / alpha, t.y / alpha);
+        acc.x = warp_sum(acc.x);
+        acc.y = warp_sum(acc.y);
+        if (lane == 0) {
+            hs[l] = acc;
+            // h_l = (z_l - (T s)_l) / alpha
+            const double2 h = make_double2((zs[l].x - acc.x) / alpha, (zs[l].y - acc.y) / alpha);
+            if (!isfinite(h.x) || !isfinite(h.y)) bad = 1;
+            cc[l] = make_double2(acc.x + alpha * h.x, acc.y + alpha * h.y);
+            if (l == j) ks->a_re[j] = h.x;  // Re <v_j, (H - sigma) v_j>
+            as->T[l * ARN_M + j] = h;
         }
     }
     __syncthreads();
-    for (int l = tid; l <= j; l += DECIDE_THREADS) {  // h_l = (z_l - (T s)_l) / alpha
-        const double2 h = make_double2((zs[l].x - hs[l].x) / alpha, (zs[l].y - hs[l].y) / alpha);
-        if (!isfinite(h.x) || !isfinite(h.y)) bad = 1;
-        as->T[l * ARN_M + j] = h;
-        cc[l] = make_double2(hs[l].x + alpha * h.x, hs[l].y + alpha * h.y);
-        if (l == j) ks->a_re[j] = h.x;  // Re <v_j, (H - sigma) v_j>
-    }
-    __syncthreads();
     // pass B: w' = (w - V_j c) / alpha with v_j = (vt - V s) / alpha substituted
-    for (int l = tid; l < nk; l += DECIDE_THREADS) {
+    for (int l = tid; l < nk; l += STAGE_THREADS) {
         const double2 sl = ss[l], cj = has_vt ? cc[j] : make_double2(0.0, 0.0);
         const double2 p = make_double2((cj.x * sl.x - cj.y * sl.y) / alpha, (cj.x * sl.y + cj.y * sl.x) / alpha);
         as->cw1[l] = has_vt ? make_double2((cc[l].x - p.x) / alpha, (cc[l].y - p.y) / alpha) : cc[l];
         as->cvj[l] = make_double2(sl.x / alpha, sl.y / alpha);
     }
-    if (tid == 0) {
-        as->cw = 1.0 / alpha;
-        as->cv = 1.0 / alpha;
-        as->ct = has_vt ? make_double2(cc[j].x / (alpha * alpha), cc[j].y / (alpha * alpha))
-                        : make_double2(0.0, 0.0);
+    if (warp == NWD - 1) {
         // ||(H - sigma) v_j||^2 = ||w - V_j (T s)||^2 / alpha^2, then ||H v_j||
-        double n2 = sa[2];
-        for (int l = 0; l <= j; ++l) {
-            if (!has_vt && l > 0) break;
+        double n2 = 0.0;
+        for (int l = lane; l <= (has_vt ? j : 0); l += 32) {
             const double2 p = cmulc(hs[l], zs[l]);
             n2 += -2.0 * p.x + hs[l].x * hs[l].x + hs[l].y * hs[l].y;
         }
-        n2 /= alpha * alpha;
-        const double sg = ks->shift;
-        ks->hn[j] = sqrt(fmax(0.0, n2 + 2.0 * sg * ks->a_re[j] + sg * sg));
-        if (!isfinite(n2)) bad = 1;
-        if (bad) {
-            ks->status = KS_NONFINITE;
-            ks->iters = j + 1;
+        n2 = (sa[2] + warp_sum(n2)) / (alpha * alpha);
+        if (lane == 0) {
+            as->cw = 1.0 / alpha;
+            as->cv = 1.0 / alpha;
+            as->ct = has_vt ? make_double2(cc[j].x / (alpha * alpha), cc[j].y / (alpha * alpha))
+                            : make_double2(0.0, 0.0);
+            const double sg = ks->shift;
+            ks->hn[j] = sqrt(fmax(0.0, n2 + 2.0 * sg * ks->a_re[j] + sg * sg));
+            if (bad || !isfinite(n2)) {
+                ks->status = KS_NONFINITE;
+                ks->iters = j + 1;
+            }
         }
     }
 }
@@ -413,6 +432,53 @@ k_arn_lagstage(KState *ks, ArnState *as, int j, const double *part, int nb) {
 // 4^35/35! ~ 1e-19 relative per substep, terms at most 4^4/4! ~ 11 times the result (about
 // one digit of cancellation).  Returns false when the norm is not finite or would need
 // more than 2^20 substeps.  All threads of the block.
+// A serial chain of 34 s matrix-vector products: TPR threads share a row, each with its NC
+// entries in registers, and the terms alternate between two vectors in shared memory, one
+// barrier a product.
+template <int TPR, int NC>
+__device__ __forceinline__ void arn_taylor(const double2 *A, int M, int s, double2 *y, double2 *t, double2 *tn) {
+    const int tid = threadIdx.x, r = tid / TPR, q = tid % TPR;
+    double2 a[NC];
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+        const int c = q + i * TPR;
+        a[i] = (r < M && c < M) ? A[c * M + r] : make_double2(0.0, 0.0);
+    }
+    double2 yr = make_double2(r == 0 ? 1.0 : 0.0, 0.0);  // y[r] in every thread of the row
+    const double is = 1.0 / (double)s;
+    for (int step = 0; step < s; ++step) {
+        if (q == 0 && r < M) t[r] = yr;
+        __syncthreads();
+        for (int k = 1; k <= 34; ++k) {
+            double2 acc = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int i = 0; i < NC; ++i) {
+                const int c = q + i * TPR;
+                const double2 v = c < M ? t[c] : make_double2(0.0, 0.0);
+                acc.x += a[i].x * v.x - a[i].y * v.y;
+                acc.y += a[i].x * v.y + a[i].y * v.x;
+            }
+#pragma unroll
+            for (int o = TPR >> 1; o > 0; o >>= 1) {  // TPR lanes of one warp
+                acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+                acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+            }
+            const double f = is / (double)k;
+            acc.x *= f;
+            acc.y *= f;
+            yr.x += acc.x;
+            yr.y += acc.y;
+            if (q == 0 && r < M) tn[r] = acc;
+            __syncthreads();
+            double2 *tmp = t;
+            t = tn;
+            tn = tmp;
+        }
+    }
+    if (q == 0 && r < M) y[r] = yr;
+    __syncthreads();
+}
+
 __device__ bool arn_expm_col0(const double2 *A, int M, double2 *y, double2 *t, double2 *tn,
                               double *red) {
     const int tid = threadIdx.x;
@@ -430,37 +496,10 @@ __device__ bool arn_expm_col0(const double2 *A, int M, double2 *y, double2 *t, d
     __syncthreads();
     if (!isfinite(nrm) || nrm > 4.0 * 1048576.0) return false;
     const int s = nrm > 4.0 ? (int)ceil(nrm / 4.0) : 1;
-    const int TPR = M <= 32 ? 8 : (M <= 64 ? 4 : 2);
-    const int r = tid / TPR, q = tid % TPR;
-    if (tid < M) y[tid] = make_double2(tid == 0 ? 1.0 : 0.0, 0.0);
-    __syncthreads();
-    for (int step = 0; step < s; ++step) {
-        if (tid < M) t[tid] = y[tid];
-        __syncthreads();
-        for (int k = 1; k <= 34; ++k) {
-            double2 acc = make_double2(0.0, 0.0);
-            if (r < M) {
-                for (int c = q; c < M; c += TPR) {
-                    const double2 a = A[c * M + r], v = t[c];
-                    acc.x += a.x * v.x - a.y * v.y;
-                    acc.y += a.x * v.y + a.y * v.x;
-                }
-            }
-            for (int o = TPR >> 1; o > 0; o >>= 1) {  // TPR lanes of one warp
-                acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
-                acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
-            }
-            const double f = 1.0 / ((double)s * (double)k);
-            if (q == 0 && r < M) tn[r] = make_double2(acc.x * f, acc.y * f);
-            __syncthreads();
-            if (tid < M) {
-                t[tid] = tn[tid];
-                y[tid].x += tn[tid].x;
-                y[tid].y += tn[tid].y;
-            }
-            __syncthreads();
-        }
-    }
+    static_assert(DECIDE_THREADS == 512 && ARN_M <= 128, "threads per row below");
+    if (M <= 32) arn_taylor<16, 2>(A, M, s, y, t, tn);
+    else if (M <= 64) arn_taylor<8, 8>(A, M, s, y, t, tn);
+    else arn_taylor<4, (ARN_M + 3) / 4>(A, M, s, y, t, tn);
     return true;
 }
 
@@ -626,23 +665,28 @@ static size_t decide_smem(int maxdim) {
     return sizeof(double2) * (M * M + 3 * M) + sizeof(double) * DECIDE_THREADS;
 }
 
-// Grid of the Gram-Schmidt passes: the streaming grid of the vector kernels (up to four
-// blocks per SM), never more blocks than chunks; *grid_out receives it (the number of
-// partial rows).
+// Grid of the Gram-Schmidt passes: never more blocks than chunks; *grid_out receives the
+// number of blocks in x (the partial sums per value).  Pass A holds one block per SM (its 32
+// sums and 16 loads a thread fill the registers), a persistent grid; where that leaves SMs
+// idle, the groups of basis vectors are spread over blocks in y.
 template <typename R>
 static int launch_lagged(int pass, const KState *ks, const ArnState *as, int j, const void *v0,
                          unsigned char *basis, i64 D, void *w, double *part, cudaStream_t s,
                          int *grid_out) {
-    constexpr int E = 4;
-    i64 grid = krylov_stream_grid(D);
+    constexpr int E = LAG_E;
     const i64 chunks = (D + (i64)ORTHO_THREADS * E - 1) / ((i64)ORTHO_THREADS * E);
+    i64 grid = pass == 0 ? (i64)sm_count() : (i64)krylov_stream_grid(D);
     if (grid > chunks) grid = chunks;
     *grid_out = (int)grid;
     ProfScope ps_(PROF_ORTH, s);
-    if (pass == 0)
-        k_arn_lagdots<R, E><<<(int)grid, ORTHO_THREADS, 0, s>>>(ks, j, v0, basis, D, w, part);
-    else
+    if (pass == 0) {
+        const int groups = ((j >= 1 ? j : 1) + ARN_KB - 1) / ARN_KB;
+        int gy = (int)(sm_count() / grid);
+        if (gy > groups) gy = groups;
+        k_arn_lagdots<R><<<dim3((unsigned)grid, gy), ORTHO_THREADS, 0, s>>>(ks, j, v0, basis, D, w, part);
+    } else {
         k_arn_lagupdate<R, E><<<(int)grid, ORTHO_THREADS, 0, s>>>(ks, as, j, v0, basis, D, w, part);
+    }
     EMUSV_CHECK_LAUNCH();
     return EMUSV_OK;
 }
@@ -775,7 +819,7 @@ int arnoldi_run(const HamParams &P, const LindbladJumps *J, int dtype, double dt
             if (st) return st;
             if (pass == 0) {
                 ProfScope ps_(PROF_SMALL, s);
-                k_arn_lagstage<<<1, DECIDE_THREADS, 0, s>>>(ks, as, j, part, og);
+                k_arn_lagstage<<<1, STAGE_THREADS, 0, s>>>(ks, as, j, part, og);
                 EMUSV_CHECK_LAUNCH();
             }
         }

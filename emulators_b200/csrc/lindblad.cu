@@ -123,7 +123,9 @@ static bool make_jumps(int n, int nops, const double *ops, LindbladJumps *J) {
 }
 
 // out[x] += i su sum_q sum_{i',j'} K[(i,j),(i',j')] u[x with the row/column bits of q set to
-// (i', j')], (i, j) = the row and column bits of q in x.
+// (i', j')], (i, j) = the row and column bits of q in x.  K's diagonal multiplies u[x] by a
+// sum over the qubits that depends on the counts of (i, j) only; the other nonzero entries
+// (one for relaxation) load their partner.
 template <typename R>
 __global__ void __launch_bounds__(BLOCK)
 k_lindblad_jumps(const LindbladJumps J, const void *u_, const double *su_p, void *out_, i64 D,
@@ -134,21 +136,34 @@ k_lindblad_jumps(const LindbladJumps J, const void *u_, const double *su_p, void
     C *out = reinterpret_cast<C *>(out_);
     const double su = su_p ? *su_p : 1.0;
     const int n = J.nq;
+    const unsigned off = J.mask & ~0x8421u;  // nonzero entries off K's diagonal
+    const unsigned low = (1u << n) - 1u;
     for (i64 x = (i64)blockIdx.x * blockDim.x + threadIdx.x; x < D; x += (i64)gridDim.x * blockDim.x) {
-        double ar = 0.0, ai = 0.0;
-        for (int pc = 0; pc < n; ++pc) {
-            const int pr = pc + n;
-            const int i = (int)((x >> pr) & 1), j = (int)((x >> pc) & 1);
-            const i64 xb = x & ~((i64(1) << pr) | (i64(1) << pc));
+        const unsigned row = (unsigned)(x >> n), col = (unsigned)x & low;
+        const C ux = u[x];
+        // the diagonal entries of K act on u[x] itself: counts of the qubits by (i, j)
+        const int n11 = __popc(row & col), n10 = __popc(row) - n11, n01 = __popc(col) - n11;
+        const double cnt[4] = {double(n - n11 - n10 - n01), double(n01), double(n10), double(n11)};
+        double dr = 0.0, di = 0.0;
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                const int e = (i * 2 + j) * 4 + t;
-                if (!((J.mask >> e) & 1)) continue;
-                const i64 y = xb | ((i64)(t >> 1) << pr) | ((i64)(t & 1) << pc);
-                const C v = u[y];
-                const double kr = J.K[2 * e], ki = J.K[2 * e + 1];
-                ar += kr * double(v.x) - ki * double(v.y);
-                ai += kr * double(v.y) + ki * double(v.x);
+        for (int e = 0; e < 4; ++e) {
+            dr += cnt[e] * J.K[2 * 5 * e];
+            di += cnt[e] * J.K[2 * 5 * e + 1];
+        }
+        double ar = dr * double(ux.x) - di * double(ux.y), ai = dr * double(ux.y) + di * double(ux.x);
+        if (off) {
+            for (int pc = 0; pc < n; ++pc) {
+                const int ij = (int)((row >> pc) & 1u) * 2 + (int)((col >> pc) & 1u);
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    const int e = ij * 4 + t;
+                    if (!((off >> e) & 1)) continue;
+                    const i64 bits = (i64)(((ij ^ t) >> 1) & 1) << (pc + n) | (i64)((ij ^ t) & 1) << pc;
+                    const C v = u[x ^ bits];
+                    const double kr = J.K[2 * e], ki = J.K[2 * e + 1];
+                    ar += kr * double(v.x) - ki * double(v.y);
+                    ai += kr * double(v.y) + ki * double(v.x);
+                }
             }
         }
         const C o = out[x];
