@@ -20,8 +20,8 @@
 
 #include <initializer_list>
 
-#include "krylov_device.cuh"
 #include "pairsums.cuh"
+#include "persist.cuh"
 #include "profile.cuh"
 
 namespace emusv {
@@ -38,6 +38,7 @@ static size_t al(size_t v) { return (v + 255) / 256 * 256; }
 
 struct AdjWorkspace {
     KState *ks_s, *ks_g;
+    PExchange *x_s, *x_g;
     double *part_h, *part_o, *part_c;
     double2 *dS;  // [KMAX][KMAX] (row i of the state basis, column k of the grad basis)
     AdjScal *scal;
@@ -48,7 +49,7 @@ struct AdjWorkspace {
 int max_grid_blocks();
 static size_t part_bytes() { return al(sizeof(double) * max_grid_blocks() * (4 * ADJ_MAXQ + 8)); }
 static size_t adj_header() {
-    return 2 * al(sizeof(KState)) + 3 * part_bytes() + al(sizeof(double2) * KMAX * KMAX) +
+    return 2 * al(sizeof(KState)) + 2 * persist_exchange_bytes() + 3 * part_bytes() + al(sizeof(double2) * KMAX * KMAX) +
            al(sizeof(AdjScal));
 }
 
@@ -62,6 +63,8 @@ static bool carve_adj(void *ws, size_t bytes, int64_t D, size_t es, AdjWorkspace
     };
     W->ks_s = reinterpret_cast<KState *>(take(sizeof(KState)));
     W->ks_g = reinterpret_cast<KState *>(take(sizeof(KState)));
+    W->x_s = reinterpret_cast<PExchange *>(take(persist_exchange_bytes()));
+    W->x_g = reinterpret_cast<PExchange *>(take(persist_exchange_bytes()));
     W->part_h = reinterpret_cast<double *>(take(part_bytes()));
     W->part_o = reinterpret_cast<double *>(take(part_bytes()));
     W->part_c = reinterpret_cast<double *>(take(part_bytes()));
@@ -324,21 +327,26 @@ int emusv_adjoint_step(int nqubits, int dtype, double dt, const double *omegas,
     const int n = nqubits;
 
     // 1. the two Lanczos bases (double_krylov.py:51-52), both tolerances = tolerance
-    int st_s = 0, st_g = 0;
-    int st = lanczos_run(P, dtype, dt, state, W.ks_s, W.part_h, W.part_o, W.basis_s, W.capacity,
-                         tolerance, tolerance, max_krylov_dim, 0, false, s, &st_s);
-    if (st) return st;
-    if (st_s == 0) return EMUSV_WORKSPACE_TOO_SMALL;
-    st = lanczos_run(P, dtype, dt, grad_out, W.ks_g, W.part_h, W.part_o, W.basis_g, W.capacity,
-                     tolerance, tolerance, max_krylov_dim, 0, false, s, &st_g);
-    if (st) return st;
-    if (st_g == 0) return EMUSV_WORKSPACE_TOO_SMALL;
-    int hg[2];
-    double s0[2];
-    EMUSV_CHECK(cudaMemcpyAsync(hg, &W.ks_g->status, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-    EMUSV_CHECK(cudaMemcpyAsync(&s0[0], &W.ks_s->s0, sizeof(double), cudaMemcpyDeviceToHost, s));
-    EMUSV_CHECK(cudaMemcpyAsync(&s0[1], &W.ks_g->s0, sizeof(double), cudaMemcpyDeviceToHost, s));
-    EMUSV_CHECK(cudaStreamSynchronize(s));
+    int st;
+    KHead h[2];
+    KState *const ks2[2] = {W.ks_s, W.ks_g};
+    if (persist_applies(dtype, n)) {  // both in one launch, side by side where they fit
+        const PJob jobs[2] = {{state, nullptr, W.ks_s, W.x_s, W.basis_s, 0},
+                              {grad_out, nullptr, W.ks_g, W.x_g, W.basis_g, 0}};
+        st = persist_launch(P, dtype, dt, jobs, 2, W.capacity, tolerance, tolerance, max_krylov_dim, s);
+        if (st || (st = read_heads(ks2, 2, s, h))) return st;
+        for (KHead &k : h)
+            if (k.kerr) k.status = KS_TIMEOUT;
+    } else {
+        int run = 0;
+        st = lanczos_run(P, dtype, dt, state, W.ks_s, W.part_h, W.part_o, W.basis_s, W.capacity, tolerance,
+                         tolerance, max_krylov_dim, 0, false, s, &run);
+        if (st) return st;
+        st = lanczos_run(P, dtype, dt, grad_out, W.ks_g, W.part_h, W.part_o, W.basis_g, W.capacity, tolerance,
+                         tolerance, max_krylov_dim, 0, false, s, &run);
+        if (st || (st = read_heads(ks2, 2, s, h))) return st;
+    }
+    const double s0[2] = {h[0].s0, h[1].s0};
     if (s0[0] == 0.0 || s0[1] == 0.0) {  // a zero state or gradient: dU|s><g| = 0
         for (int i = 0; i < n; ++i) {
             if (g_omegas) g_omegas[i] = 0.0;
@@ -348,13 +356,14 @@ int emusv_adjoint_step(int nqubits, int dtype, double dt, const double *omegas,
         if (g_interaction) memset(g_interaction, 0, sizeof(double) * n * n);
         return EMUSV_OK;
     }
-    for (int r : {st_s, st_g}) {
-        if (r == KS_MAXDIM) return EMUSV_NOT_CONVERGED;  // double_krylov.py:107-110
-        if (r == EMUSV_TIMEOUT) return EMUSV_TIMEOUT;
-        if (r != KS_CONVERGED && r != KS_HAPPY) return EMUSV_NONFINITE;
+    for (const KHead &k : h) {
+        if (k.status == KS_RUNNING) return EMUSV_WORKSPACE_TOO_SMALL;
+        if (k.status == KS_MAXDIM) return EMUSV_NOT_CONVERGED;  // double_krylov.py:107-110
+        if (k.status == KS_TIMEOUT) return EMUSV_TIMEOUT;
+        if (k.status != KS_CONVERGED && k.status != KS_HAPPY) return EMUSV_NONFINITE;
     }
     // size of the gradient basis (the dS columns)
-    const int mg = hg[0] == KS_HAPPY ? hg[1] : hg[1] + 1;
+    const int mg = h[1].status == KS_HAPPY ? h[1].iters : h[1].iters + 1;
 
     // 2. dS (c = 1; scaled by c = |state||grad| below)
     {

@@ -849,17 +849,9 @@ int arnoldi_run(const HamParams &P, const LindbladJumps *J, int dtype, double dt
     }
     if ((st = krylov_combine(dtype, ks, psi_in, basis, D, psi_out, part_n, s))) return st;
     if (info) {
-        KState h;
-        EMUSV_CHECK(cudaMemcpyAsync(&h, ks, offsetof(KState, a_re), cudaMemcpyDeviceToHost, s));
-        EMUSV_CHECK(cudaStreamSynchronize(s));
-        info->iterations = h.iters;
-        info->happy_breakdown = h.status == KS_HAPPY;
-        info->converged = h.status == KS_HAPPY || h.status == KS_CONVERGED;
-        info->basis_vectors = h.nvec;
-        info->error_estimate = h.err;
-        info->input_norm = h.s0;
-        info->output_norm = sqrt(h.outnorm2);
-        info->second_rounds = h.iters > 0 ? h.iters - 1 : 0;  // every vector but the first
+        KHead h;
+        if ((st = read_heads(&ks, 1, s, &h))) return st;
+        fill_info(h, h.iters > 0 ? h.iters - 1 : 0, info);  // every vector but the first
     }
     return status == KS_MAXDIM ? EMUSV_NOT_CONVERGED : EMUSV_OK;
 }

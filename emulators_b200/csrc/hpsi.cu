@@ -121,8 +121,7 @@ static int launch_one(const HamParams &P, HpsiArgs A, int max_grid, cudaStream_t
 }
 
 int pass_min_qubits(int dtype);
-int launch_hpsi_passes(int dtype, int mode, const HamParams &H, const HpsiArgs &A,
-                       cudaStream_t s, int *grid_out);
+int launch_hpsi_passes(int dtype, const HamParams &H, const HpsiArgs &A, cudaStream_t s);
 
 // EMUSV_HPSI_SINGLE_PASS=1 selects the single-pass tile kernel for every size (A/B checks).
 static bool single_pass_forced() {
@@ -137,18 +136,14 @@ static bool single_pass_forced() {
 bool lz_applies(int dtype, int n);
 int lz_moments(int dtype, const HamParams &H, const void *psi, void *part, double *partials,
                double *part_h, unsigned *cnt, int *err, cudaStream_t s, int *grid_out);
-// The Lanczos iteration of this register runs in the H-first order (hpsi_pass.cu): wider
-// than one pass-L tile and the passes not switched off.
-bool lanczos_h_first(int dtype, int n) { return !single_pass_forced() && lz_applies(dtype, n); }
-
 // Dispatch on dtype / real coefficients / mode.  Registers of at least one pass-L tile
-// use the two-pass kernels for H*psi (store and Lanczos modes); the single-pass kernel
-// serves small registers, the energy reductions and the diagonal.
+// use the two-pass kernels for H*psi; the single-pass kernel serves small registers, the
+// energy reductions and the diagonal.
 int launch_hpsi(int dtype, int mode, const HamParams &P, HpsiArgs A, int max_grid,
                 cudaStream_t s, int *grid_out) {
-    if ((mode == HP_STORE || mode == HP_LANCZOS) && (dtype == EMUSV_C64 || dtype == EMUSV_C128) &&
+    if (mode == HP_STORE && (dtype == EMUSV_C64 || dtype == EMUSV_C128) &&
         P.n >= pass_min_qubits(dtype) && !single_pass_forced())
-        return launch_hpsi_passes(dtype, mode, P, A, s, grid_out);
+        return launch_hpsi_passes(dtype, P, A, s);
 #define EMUSV_DISPATCH(R, M)                                                           \
     return P.real_coef ? launch_one<R, true, M>(P, A, max_grid, s, grid_out)           \
                        : launch_one<R, false, M>(P, A, max_grid, s, grid_out)
@@ -156,14 +151,12 @@ int launch_hpsi(int dtype, int mode, const HamParams &P, HpsiArgs A, int max_gri
         switch (mode) {
         case HP_STORE: EMUSV_DISPATCH(double, HP_STORE);
         case HP_ENERGY: EMUSV_DISPATCH(double, HP_ENERGY);
-        case HP_LANCZOS: EMUSV_DISPATCH(double, HP_LANCZOS);
         case HP_DIAG: return launch_one<double, true, HP_DIAG>(P, A, max_grid, s, grid_out);
         }
     } else if (dtype == EMUSV_C64) {
         switch (mode) {
         case HP_STORE: EMUSV_DISPATCH(float, HP_STORE);
         case HP_ENERGY: EMUSV_DISPATCH(float, HP_ENERGY);
-        case HP_LANCZOS: EMUSV_DISPATCH(float, HP_LANCZOS);
         case HP_DIAG: return launch_one<float, true, HP_DIAG>(P, A, max_grid, s, grid_out);
         }
     }
@@ -244,7 +237,7 @@ static size_t scratch_head_bytes(int n) {
     return (sizeof(double) * d + 255) / 256 * 256;
 }
 static bool expect_by_passes(int dtype, int n) {
-    return (dtype == EMUSV_C64 || dtype == EMUSV_C128) && lanczos_h_first(dtype, n);
+    return !single_pass_forced() && lz_applies(dtype, n);
 }
 
 size_t emusv_scratch_bytes(int nqubits, int dtype) {

@@ -21,24 +21,20 @@ namespace emusv {
 enum HpsiMode {
     HP_STORE = 0,    // out = H v
     HP_ENERGY = 1,   // no store; <v,Hv>, ||Hv||^2
-    HP_LANCZOS = 2,  // out = H v; ||Hv||^2, <v,Hv>, <vp,Hv>, <v,vp>
-    HP_DIAG = 3      // out (float64) = diag
+    HP_DIAG = 2      // out (float64) = diag
 };
 
 struct HpsiArgs {
     const void *u;     // input (stored) vector; v = su * u
     double su;
     const double *su_dev;     // if non-null, su is read from here (device scalar)
-    const void *up;    // previous Lanczos vector (HP_LANCZOS, may be null); vp = sp * up
-    double sp;
-    const double *sp_dev;
     void *out;
     double *partials;  // [gridDim.x * NRED]
     int tile_bits;
     const int *gate;   // if non-null and *gate != 0 the kernel returns at once
     void *part_buf;    // two-pass H*psi: buffer for the partial sums of pass L
     int *err;          // device word receiving EMUSV_TIMEOUT if a bounded wait gives up
-    const double *eshift;  // HP_LANCZOS, HP_STORE: if non-null, the diagonal is taken minus *eshift
+    const double *eshift;  // HP_STORE: if non-null, the diagonal is taken minus *eshift
 };
 
 // Arguments of the Lanczos iteration's pass L (k_pass_lz in hpsi_pass.cuh).
@@ -122,9 +118,7 @@ k_hpsi(const HamParams P, HpsiArgs A) {
     }
 
     const double su = A.su_dev ? *A.su_dev : A.su;
-    const double sp = (MODE == HP_LANCZOS && A.up) ? (A.sp_dev ? *A.sp_dev : A.sp) : 0.0;
     const C *__restrict__ u = reinterpret_cast<const C *>(A.u);
-    const C *__restrict__ upv = reinterpret_cast<const C *>(A.up);
 
     double acc_r[NRED];
 #pragma unroll
@@ -173,7 +167,7 @@ k_hpsi(const HamParams P, HpsiArgs A) {
             }
         }
         __syncthreads();
-        const double ehigh = gv[MAXQ] - ((MODE == HP_LANCZOS || MODE == HP_STORE) && A.eshift ? *A.eshift : 0.0) +
+        const double ehigh = gv[MAXQ] - (MODE == HP_STORE && A.eshift ? *A.eshift : 0.0) +
                              (MODE == HP_DIAG ? 0.0 : P.dc_re);
 
         for (int k = tid; k < TILE; k += BLOCK) {
@@ -226,24 +220,16 @@ k_hpsi(const HamParams P, HpsiArgs A) {
                 hi = su * (double(ai) + d * double(v.y));
             }
             const double vr = su * double(v.x), vi = su * double(v.y);
-            if (MODE == HP_STORE || MODE == HP_LANCZOS)
+            if (MODE == HP_STORE)
                 reinterpret_cast<C *>(A.out)[x] = cmake<C>(hr, hi);
-            if (MODE == HP_ENERGY || MODE == HP_LANCZOS) {
+            if (MODE == HP_ENERGY) {
                 acc_r[0] += hr * hr + hi * hi;
                 acc_r[1] += vr * hr + vi * hi;  // <v, Hv>
                 acc_r[2] += vr * hi - vi * hr;
             }
-            if (MODE == HP_LANCZOS && upv) {
-                const C q = upv[x];
-                const double pr = sp * double(q.x), pi = sp * double(q.y);
-                acc_r[3] += pr * hr + pi * hi;  // <vp, Hv>
-                acc_r[4] += pr * hi - pi * hr;
-                acc_r[5] += vr * pr + vi * pi;  // <v, vp>
-                acc_r[6] += vr * pi - vi * pr;
-            }
         }
     }
-    if (MODE == HP_ENERGY || MODE == HP_LANCZOS) {
+    if (MODE == HP_ENERGY) {
         block_sum<NRED>(acc_r, red);
         if (tid == 0) {
 #pragma unroll

@@ -114,7 +114,7 @@ static void fill_params(const HamParams &H, int TB, int RB, PassParams *P) {
 }
 
 template <typename R, bool REALC, int EPI, bool NOISY>
-static int launch_low(const PassParams &P, const PassArgs &A, cudaStream_t s, int *grid_out) {
+static int launch_low(const PassParams &P, const PassArgs &A, cudaStream_t s) {
     typedef typename cvec<R>::T C;
     constexpr int TB = PassShape<R>::TB, RB = PassShape<R>::RB, NT = 1 << (TB - RB);
     auto kern = k_pass_low<R, REALC, TB, RB, EPI, 0, NOISY>;
@@ -131,7 +131,6 @@ static int launch_low(const PassParams &P, const PassArgs &A, cudaStream_t s, in
         kern<<<(unsigned)grid, NT, smem, s>>>(P, A);
     }
     EMUSV_CHECK_LAUNCH();
-    if (grid_out) *grid_out = (int)grid;
     return EMUSV_OK;
 }
 
@@ -180,8 +179,8 @@ static int launch_high(PassParams P, int hpos, const PassArgs &A, const void *pa
 // pass L) are skipped, so every H pass keeps the compile-time chunk of CMIN bits.  The
 // partial sums live in HA.part_buf (which may be HA.out: every pass reads a tile before
 // writing it).
-template <typename R, bool REALC, int EPI_F, int CMIN, bool NOISY>
-static int run_passes(const HamParams &H, const HpsiArgs &HA, cudaStream_t s, int *grid_out) {
+template <typename R, bool REALC, int CMIN, bool NOISY>
+static int run_passes_c(const HamParams &H, const HpsiArgs &HA, cudaStream_t s) {
     constexpr int TB = PassShape<R>::TB, RB = PassShape<R>::RB;
     const int n = H.n;
     PassParams P;
@@ -202,50 +201,33 @@ static int run_passes(const HamParams &H, const HpsiArgs &HA, cudaStream_t s, in
     int st;
     if (rem == 0) {
         A.out = HA.out;
-        return launch_low<R, REALC, EPI_F, NOISY>(P, A, s, grid_out);
+        return launch_low<R, REALC, EPI_STORE, NOISY>(P, A, s);
     }
     A.out = HA.part_buf;
-    if ((st = launch_low<R, REALC, EPI_PARTIAL, NOISY>(P, A, s, nullptr))) return st;
+    if ((st = launch_low<R, REALC, EPI_PARTIAL, NOISY>(P, A, s))) return st;
     if (rem > G) {
         if ((st = launch_high<R, REALC, EPI_PARTIAL, CMIN>(P, n - 2 * G, A, HA.part_buf, s, nullptr)))
             return st;
     }
     A.out = HA.out;
-    return launch_high<R, REALC, EPI_F, CMIN>(P, n - G, A, HA.part_buf, s, grid_out);
+    return launch_high<R, REALC, EPI_STORE, CMIN>(P, n - G, A, HA.part_buf, s, nullptr);
 }
 
 // 64-byte rows (PassShape CMIN) where two H passes cover the bits above pass L, else
 // 32-byte rows
-template <typename R, bool REALC, int EPI_F, bool NOISY = false>
-static int run_passes(const HamParams &H, const HpsiArgs &HA, cudaStream_t s, int *grid_out) {
+template <typename R, bool REALC, bool NOISY = false>
+static int run_passes(const HamParams &H, const HpsiArgs &HA, cudaStream_t s) {
     constexpr int TB = PassShape<R>::TB, CMIN = PassShape<R>::CMIN;
-    if (H.n - TB <= 2 * (TB - CMIN)) return run_passes<R, REALC, EPI_F, CMIN, NOISY>(H, HA, s, grid_out);
-    return run_passes<R, REALC, EPI_F, CMIN - 1, NOISY>(H, HA, s, grid_out);
+    if (H.n - TB <= 2 * (TB - CMIN)) return run_passes_c<R, REALC, CMIN, NOISY>(H, HA, s);
+    return run_passes_c<R, REALC, CMIN - 1, NOISY>(H, HA, s);
 }
 
-// mode: HP_STORE or HP_LANCZOS (values of HpsiMode)
-int launch_hpsi_passes(int dtype, int mode, const HamParams &H, const HpsiArgs &A,
-                       cudaStream_t s, int *grid_out) {
-    const bool lz = mode == HP_LANCZOS;
-    if (H.noisy) {  // the non-Hermitian noise term: store mode only (Arnoldi, H*psi)
-        if (lz) return EMUSV_BAD_ARGUMENT;
-        return dtype == EMUSV_C64 ? run_passes<float, false, EPI_STORE, true>(H, A, s, grid_out)
-                                  : run_passes<double, false, EPI_STORE, true>(H, A, s, grid_out);
-    }
-    if (dtype == EMUSV_C64) {
-        if (H.real_coef)
-            return lz ? run_passes<float, true, EPI_LANCZOS>(H, A, s, grid_out)
-                      : run_passes<float, true, EPI_STORE>(H, A, s, grid_out);
-        return lz ? run_passes<float, false, EPI_LANCZOS>(H, A, s, grid_out)
-                  : run_passes<float, false, EPI_STORE>(H, A, s, grid_out);
-    }
-    if (dtype == EMUSV_C128) {
-        if (H.real_coef)
-            return lz ? run_passes<double, true, EPI_LANCZOS>(H, A, s, grid_out)
-                      : run_passes<double, true, EPI_STORE>(H, A, s, grid_out);
-        return lz ? run_passes<double, false, EPI_LANCZOS>(H, A, s, grid_out)
-                  : run_passes<double, false, EPI_STORE>(H, A, s, grid_out);
-    }
+int launch_hpsi_passes(int dtype, const HamParams &H, const HpsiArgs &A, cudaStream_t s) {
+    if (H.noisy)  // the non-Hermitian noise term
+        return dtype == EMUSV_C64 ? run_passes<float, false, true>(H, A, s) : run_passes<double, false, true>(H, A, s);
+    if (dtype == EMUSV_C64) return H.real_coef ? run_passes<float, true>(H, A, s) : run_passes<float, false>(H, A, s);
+    if (dtype == EMUSV_C128)
+        return H.real_coef ? run_passes<double, true>(H, A, s) : run_passes<double, false>(H, A, s);
     return EMUSV_BAD_ARGUMENT;
 }
 

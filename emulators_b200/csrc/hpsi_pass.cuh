@@ -39,16 +39,15 @@ namespace emusv {
 enum PassEpi {
     EPI_PARTIAL = 0,  // store the partial sum (another pass follows)
     EPI_STORE = 1,    // store H v
-    EPI_LANCZOS = 2,  // store H v; FP64 partials ||Hv||^2, <v,Hv>
     // flips of the pass's group bits only, unscaled (the Lanczos iteration's pass H, which
     // runs before its pass L): out = X u (first pass, no partial-sum input) or
     // out = part + X u; FP64 partials of <u, X u> (0 re, 1 im)
-    EPI_X_FIRST = 3,
-    EPI_X_ADD = 4,
+    EPI_X_FIRST = 2,
+    EPI_X_ADD = 3,
 };
 template <int EPI> __host__ __device__ constexpr bool epi_has_part() { return EPI != EPI_X_FIRST; }
 template <int EPI> __host__ __device__ constexpr bool epi_reduces() {
-    return EPI == EPI_LANCZOS || EPI == EPI_X_FIRST || EPI == EPI_X_ADD;
+    return EPI == EPI_X_FIRST || EPI == EPI_X_ADD;
 }
 
 constexpr int PBMAX_ALL = 3;  // largest cluster (2^3 CTAs) either pass uses
@@ -279,7 +278,6 @@ k_pass_low(const PassParams P, PassArgs A) {
     double *Ush = reinterpret_cast<double *>(smem_pass + SL * TILE_BYTES + 8 * SL);
     double *fld = Ush + MAXQ * UPAD;
     double *scal = fld + MAXQ;       // [SL][64]: crossT[SB] crossR[RB] eh
-    double *red_scr = scal + SL * 64;
 
     const int n = P.n;
     const int tid = threadIdx.x;
@@ -342,10 +340,6 @@ k_pass_low(const PassParams P, PassArgs A) {
     }
     const double su = A.su_dev ? *A.su_dev : A.su;
     const float suf = float(su);
-    double red[NRED];
-#pragma unroll
-    for (int k = 0; k < NRED; ++k) red[k] = 0.0;
-
     int it = 0, buf = 0;
     uint32_t phase = 0;
     for (int64_t s = cid; s < nsuper; s += nclusters, ++it) {
@@ -398,7 +392,6 @@ k_pass_low(const PassParams P, PassArgs A) {
             float hRf[RB];
 #pragma unroll
             for (int k = 0; k < RB; ++k) hRf[k] = float(hR[k]);
-            float rf[3] = {0.f, 0.f, 0.f};
             const uint32_t boff = (uint32_t)buf * TILE_BYTES;
             C v[NA];
 #pragma unroll
@@ -441,11 +434,6 @@ k_pass_low(const PassParams P, PassArgs A) {
                     } else {
                         const float2 h = make_float2(suf * t.x, suf * t.y);
                         out_t[a * NT] = h;
-                        if (EPI == EPI_LANCZOS) {
-                            rf[0] = fmaf(h.x, h.x, fmaf(h.y, h.y, rf[0]));
-                            rf[1] = fmaf(v[a].x, h.x, fmaf(v[a].y, h.y, rf[1]));
-                            rf[2] = fmaf(v[a].x, h.y, fmaf(-v[a].y, h.x, rf[2]));
-                        }
                     }
                 } else {
                     double d = St + P.ER[a];
@@ -464,20 +452,7 @@ k_pass_low(const PassParams P, PassArgs A) {
                     } else {
                         const double hr = su * tr, hi = su * ti;
                         out_t[a * NT] = cmake<C>(hr, hi);
-                        if (EPI == EPI_LANCZOS) {
-                            const double vr = su * ur, vi = su * ui;
-                            red[0] += hr * hr + hi * hi;
-                            red[1] += vr * hr + vi * hi;
-                            red[2] += vr * hi - vi * hr;
-                        }
                     }
-                }
-            }
-            if constexpr (std::is_same<R, float>::value) {
-                if (EPI == EPI_LANCZOS) {  // per-tile FP32 partial sums -> FP64 accumulators
-                    red[0] += double(rf[0]);
-                    red[1] += su * double(rf[1]);
-                    red[2] += su * double(rf[2]);
                 }
             }
         }
@@ -488,7 +463,6 @@ k_pass_low(const PassParams P, PassArgs A) {
     }
     // no CTA may leave while a sibling can still read its shared memory
     if (PB) cluster_sync_all();
-    write_partials<EPI>(A, red, red_scr);
 }
 
 // ------------------------------------------------------------------------- pass H
@@ -634,7 +608,7 @@ k_pass_high(const PassParams P, PassArgs A, const __grid_constant__ PassHighMaps
         }
         if (ok) {
             const uint32_t boff = (uint32_t)buf * TILE_BYTES;
-            float rf[3] = {0.f, 0.f, 0.f};
+            float rf[2] = {0.f, 0.f};
             C v[NA];
 #pragma unroll
             for (int a = 0; a < NA; ++a) v[a] = tile[tid + a * NT];
@@ -686,29 +660,13 @@ k_pass_high(const PassParams P, PassArgs A, const __grid_constant__ PassHighMaps
                     const float2 t = upk2(acc.a);
                     const float2 h = make_float2(suf * (pt.x + t.x), suf * (pt.y + t.y));
                     outp[x] = h;
-                    if (EPI == EPI_LANCZOS) {
-                        rf[0] = fmaf(h.x, h.x, fmaf(h.y, h.y, rf[0]));
-                        rf[1] = fmaf(v[a].x, h.x, fmaf(v[a].y, h.y, rf[1]));
-                        rf[2] = fmaf(v[a].x, h.y, fmaf(-v[a].y, h.x, rf[2]));
-                    }
                 } else {
                     const double hr = su * (double(pt.x) + acc.re());
                     const double hi = su * (double(pt.y) + acc.im());
                     outp[x] = cmake<C>(hr, hi);
-                    if (EPI == EPI_LANCZOS) {
-                        const double vr = su * double(v[a].x), vi = su * double(v[a].y);
-                        red[0] += hr * hr + hi * hi;
-                        red[1] += vr * hr + vi * hi;
-                        red[2] += vr * hi - vi * hr;
-                    }
                 }
             }
             if constexpr (std::is_same<R, float>::value) {
-                if (EPI == EPI_LANCZOS) {  // per-tile FP32 partial sums -> FP64 accumulators
-                    red[0] += double(rf[0]);
-                    red[1] += su * double(rf[1]);
-                    red[2] += su * double(rf[2]);
-                }
                 if (EPI == EPI_X_FIRST || EPI == EPI_X_ADD) {
                     red[0] += double(rf[0]);
                     red[1] += double(rf[1]);

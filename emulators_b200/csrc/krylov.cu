@@ -1,8 +1,9 @@
 // Lanczos time step exp(-i dt H) psi on the GPU (C ABI emusv_krylov_step) and the
 // building blocks of the generic krylov_exp.
 //
-// Per Lanczos iteration j (reference emu_base/math/krylov_exp.py:49-96), registers wider
-// than one pass-L tile (the H-first order, lanczos_run):
+// Registers whose vectors fit the GPU's shared memory take the whole step in one launch
+// (persist.cu).  Wider ones, per Lanczos iteration j (reference emu_base/math/krylov_exp.py:
+// 49-96, the H-first order, lanczos_run):
 //   1. pass H kernels (k_pass_high, EPI_X_FIRST / EPI_X_ADD): part = the flips of the bits
 //      above the pass-L tile applied to v_j, and their share of <v_j, H v_j>;
 //   2. k_lz_coef: a_j = <v_j, H v_j> - b_j <v_j, v_{j-1}> with b_j = ||w_{j-1}|| (the
@@ -15,8 +16,6 @@
 //   5. k_lz_decide (one warp, on a second stream, overlapping iteration j+1): the
 //      exponential of the extended Krylov matrix and the Expokit error estimate
 //      (krylov_exp.py:77-86), all FP64 on the device.
-// Smaller registers: k_hpsi<HP_LANCZOS> (H v with its reductions), k_orth (the recurrence),
-// k_small.
 // Basis vectors are stored unnormalised with a device scale factor (v_k = scale_k u_k),
 // so no separate normalisation pass exists; the input vector is basis vector 0 in place.
 // Every kernel after the first reads a device status word and exits at once when the
@@ -26,15 +25,11 @@
 
 #include <mutex>
 
-#include "krylov_device.cuh"
+#include "persist.cuh"
 #include "profile.cuh"
 
 namespace emusv {
 
-int hpsi_tile_bits(int n);
-int launch_hpsi(int dtype, int mode, const HamParams &P, HpsiArgs A, int max_grid,
-                cudaStream_t s, int *grid_out);
-bool lanczos_h_first(int dtype, int n);
 int lz_energy0(int dtype, const HamParams &H, const LzArgs &A, cudaStream_t s, int *grid_out);
 int lz_low(int dtype, const HamParams &H, const LzArgs &A, cudaStream_t s, int *grid_out);
 int lz_high(int dtype, const HamParams &H, const void *u, void *part, double *partials, const int *gate,
@@ -43,6 +38,7 @@ int max_grid_blocks();
 
 struct Workspace {
     KState *ks;
+    PExchange *x;
     double *part_h, *part_o, *part_c;
     unsigned char *basis;
     size_t basis_bytes;
@@ -51,7 +47,8 @@ struct Workspace {
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 static size_t header_bytes() {
-    return align_up(sizeof(KState), 256) + 3 * align_up(sizeof(double) * max_grid_blocks() * NRED, 256);
+    return align_up(sizeof(KState), 256) + persist_exchange_bytes() +
+           3 * align_up(sizeof(double) * max_grid_blocks() * NRED, 256);
 }
 
 static Workspace carve(void *ws, size_t bytes) {
@@ -60,6 +57,8 @@ static Workspace carve(void *ws, size_t bytes) {
     size_t off = 0;
     W.ks = reinterpret_cast<KState *>(p);
     off += align_up(sizeof(KState), 256);
+    W.x = reinterpret_cast<PExchange *>(p + off);
+    off += persist_exchange_bytes();
     const size_t pb = align_up(sizeof(double) * max_grid_blocks() * NRED, 256);
     W.part_h = reinterpret_cast<double *>(p + off);
     off += pb;
@@ -125,67 +124,6 @@ __global__ void k_init(KState *ks, const double *partials, int nblocks, int ener
     }
 }
 
-// Three-term recurrence w <- H v_j - b v_{j-1} - a v_j with b = ||w_{j-1}|| (which equals
-// <v_{j-1}, H v_j> in exact arithmetic) and a = <v_j, H v_j> - b <v_j, v_{j-1}>, the
-// modified Gram-Schmidt value of krylov_exp.py:55-58 with the measured non-orthogonality
-// <v_j, v_{j-1}> carried over from the previous iteration.  FP64 partials: ||w||^2 and
-// <v_j, w> (the next iteration's <v_{j+1}, v_j>).
-template <typename R>
-__global__ void __launch_bounds__(BLOCK)
-k_orth(KState *ks, int j, const double *part_h, int nb_h, const void *vj_, const void *vp_,
-       void *w_, i64 D, double *part_o) {
-    typedef typename cvec<R>::T C;
-    if (ks->status != KS_RUNNING) return;
-    __shared__ double red[(BLOCK / 32) * NRED];
-    double s[NRED];
-    sum_partials<NRED>(part_h, nb_h, NRED, s, red);
-    // s: 0 ||Hv||^2, 1-2 <v,Hv>
-    const double b = j > 0 ? ks->r[j - 1] : 0.0;
-    const double cr = j > 0 ? ks->vv_re[j] : 0.0, ci = j > 0 ? ks->vv_im[j] : 0.0;
-    const double ar = s[1] - b * cr;
-    const double ai = s[2] - b * ci;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        ks->a_re[j] = ar;
-        ks->a_im[j] = ai;
-        ks->b_re[j] = b;
-        ks->b_im[j] = 0.0;
-        // ||H v||^2 = ||(H - sigma) v||^2 + 2 sigma Re<v,(H - sigma) v> + sigma^2
-        const double sg = ks->shift;
-        ks->hn[j] = sqrt(fmax(0.0, s[0] + 2.0 * sg * s[1] + sg * sg));
-    }
-    const double sj = ks->scale[j];
-    const double sp = j > 0 ? ks->scale[j - 1] : 0.0;
-    // coefficients on the stored (unscaled) vectors
-    const double car = ar * sj, cai = ai * sj, cb = b * sp;
-    const C *vj = reinterpret_cast<const C *>(vj_);
-    const C *vp = reinterpret_cast<const C *>(vp_);
-    C *w = reinterpret_cast<C *>(w_);
-    double acc[NRED];
-#pragma unroll
-    for (int k = 0; k < NRED; ++k) acc[k] = 0.0;
-    for (i64 x = (i64)blockIdx.x * blockDim.x + threadIdx.x; x < D; x += (i64)gridDim.x * blockDim.x) {
-        const C h = w[x];
-        const C a = vj[x];
-        double wr = double(h.x) - (car * double(a.x) - cai * double(a.y));
-        double wi = double(h.y) - (car * double(a.y) + cai * double(a.x));
-        if (j > 0) {
-            const C p = vp[x];
-            wr -= cb * double(p.x);
-            wi -= cb * double(p.y);
-        }
-        const C o = cmake<C>(wr, wi);
-        w[x] = o;
-        const double orr = double(o.x), oi = double(o.y);
-        const double vr = sj * double(a.x), vi = sj * double(a.y);
-        acc[0] += orr * orr + oi * oi;
-        acc[1] += vr * orr + vi * oi;  // <v_j, w>
-        acc[2] += vr * oi - vi * orr;
-    }
-    block_sum<NRED>(acc, red);
-    if (threadIdx.x == 0)
-        for (int k = 0; k < NRED; ++k) part_o[(i64)blockIdx.x * NRED + k] = acc[k];
-}
-
 // H-first iteration j: <v_j, (H - sigma) v_j> is the pass-L part el (computed by the pass
 // that produced v_j -- the previous iteration's pass L, or for j = 0 the start-of-run
 // energy pass, partials 4-5 of part_e0) plus the pass-H part (partials 0-1 of part_h, on
@@ -224,33 +162,6 @@ __global__ void k_lz_coef(KState *ks, int j, const double *part_h, int nb_h, con
         ks->ocoef[1] = ai * sj;
         ks->ocoef[2] = b * sp;
     }
-}
-
-// Decide iteration j (krylov_decide) from the orthogonalisation's partial sums.  Later
-// kernels of the step return at once once the status leaves KS_RUNNING.
-__global__ void __launch_bounds__(32)
-k_small(KState *ks, int j, const double *part_o, int nb_o, double dt, double exp_tol,
-        double norm_tol, int poll, int first_poll, int maxdim) {
-    if (ks->status != KS_RUNNING) return;
-    if (ks->kerr) {  // a streaming kernel gave up on a bounded wait
-        if (threadIdx.x == 0) {
-            ks->status = KS_TIMEOUT;
-            ks->iters = j + 1;
-        }
-        return;
-    }
-    const int lane = threadIdx.x;
-    // deterministic sums of the ||w||^2 and <v_j, w> partials by one warp
-    double v = 0.0, vr = 0.0, vi = 0.0;
-    for (int b = lane; b < nb_o; b += 32) {
-        v += part_o[(i64)b * NRED];
-        vr += part_o[(i64)b * NRED + 1];
-        vi += part_o[(i64)b * NRED + 2];
-    }
-    v = warp_sum(v);
-    vr = warp_sum(vr);
-    vi = warp_sum(vi);
-    krylov_decide(ks, j, v, vr, vi, dt, exp_tol, norm_tol, poll != 0, first_poll != 0, maxdim);
 }
 
 // H-first iteration j, first part (on the step's stream): from the pass-L partials
@@ -492,7 +403,7 @@ using namespace emusv;
 
 namespace emusv {
 namespace {
-thread_local int *pinned_status = nullptr;
+thread_local KHead *pinned_heads = nullptr;
 }  // namespace
 
 // Input norm and KState reset, as the start of lanczos_run (k_init).
@@ -531,20 +442,38 @@ int krylov_combine(int dtype, KState *ks, const void *psi_in, const unsigned cha
     return EMUSV_OK;
 }
 
+void fill_info(const KHead &h, int second_rounds, emusv_krylov_info *info) {
+    info->iterations = h.iters;
+    info->happy_breakdown = h.status == KS_HAPPY;
+    info->converged = h.status == KS_HAPPY || h.status == KS_CONVERGED;
+    info->basis_vectors = h.nvec;
+    info->error_estimate = h.err;
+    info->input_norm = h.s0;
+    info->output_norm = sqrt(h.outnorm2);
+    info->second_rounds = second_rounds;
+}
+
 int krylov_stream_grid(i64 D) { return stream_grid(D); }
 size_t krylov_header_bytes() { return header_bytes(); }
 
-int read_status(KState *ks, cudaStream_t s, int *out) {
-    if (!pinned_status) {
-        if (cudaHostAlloc((void **)&pinned_status, 4 * sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
-            pinned_status = nullptr;
-            return EMUSV_CUDA_ERROR;
-        }
+// Waits for the stream and reads the heads of njobs run states (one copy each).
+int read_heads(KState *const *ks, int njobs, cudaStream_t s, KHead *out) {
+    if (!pinned_heads &&
+        cudaHostAlloc((void **)&pinned_heads, 2 * sizeof(KHead), cudaHostAllocDefault) != cudaSuccess) {
+        pinned_heads = nullptr;
+        return EMUSV_CUDA_ERROR;
     }
-    EMUSV_CHECK(cudaMemcpyAsync(pinned_status, &ks->status, sizeof(int), cudaMemcpyDeviceToHost, s));
+    for (int k = 0; k < njobs; ++k)
+        EMUSV_CHECK(cudaMemcpyAsync(&pinned_heads[k], ks[k], sizeof(KHead), cudaMemcpyDeviceToHost, s));
     EMUSV_CHECK(cudaStreamSynchronize(s));
-    *out = pinned_status[0];
+    for (int k = 0; k < njobs; ++k) out[k] = pinned_heads[k];
     return EMUSV_OK;
+}
+int read_status(KState *ks, cudaStream_t s, int *out) {
+    KHead h;
+    const int st = read_heads(&ks, 1, s, &h);
+    if (!st) *out = h.status;
+    return st;
 }
 }  // namespace emusv
 
@@ -585,14 +514,12 @@ int lanczos_run(const HamParams &P, int dtype, double dt, const void *v0, KState
     EMUSV_CHECK_LAUNCH();
 
     int status = KS_RUNNING;
-    // Registers wider than one pass-L tile run the H-first iteration: the pass H kernels
-    // write part = X_high v_j (the flips of the bits above the pass-L tile) and their share
+    // The H-first iteration: the pass H kernels write part = X_high v_j (the flips of the bits above the pass-L tile) and their share
     // of <v_j, H v_j>; k_lz_coef forms a_j; the pass L kernel forms H v_j tile by tile and
     // writes w = H v_j - a_j v_j - b_j v_{j-1} and the pass-L share of <w, H w> for the
     // next a; k_lz_norms and k_lz_decide conclude the iteration.  Streamed vector units per iteration: pass L 4 (read v_j,
     // part, v_{j-1}; write w), one H pass 2 (read v_j, write part) or two H passes 2 + 3.
-    const bool hfirst = lanczos_h_first(dtype, nqubits);
-    if (hfirst) {
+    {
         // with `overlap`, the decision of iteration j (k_lz_decide) runs on a second stream
         // while the main stream goes on with iteration j+1, which needs only k_lz_norms'
         // outputs (k_lz_decide reads a, r, b up to index j and hn[j]; iteration j+1 writes
@@ -689,58 +616,6 @@ int lanczos_run(const HamParams &P, int dtype, double dt, const void *v0, KState
             EMUSV_CHECK(cudaStreamWaitEvent(s, ev_d, 0));
         }
     }
-    for (int j = 0; !hfirst && j < max_krylov_dim; ++j) {
-        if (j + 1 > capacity) {
-            int st = read_status(W.ks, s, &status);
-            if (st) return st;
-            if (status == KS_RUNNING) return EMUSV_WORKSPACE_TOO_SMALL;
-            break;
-        }
-        HpsiArgs A = {};
-        A.u = stored(j);
-        A.su_dev = &W.ks->scale[j];
-        A.up = nullptr;  // b comes from the previous norm (see k_orth)
-        A.out = const_cast<void *>(stored(j + 1));
-        A.partials = W.part_h;
-        A.tile_bits = hpsi_tile_bits(nqubits);
-        A.gate = &W.ks->status;
-        A.err = &W.ks->kerr;
-        A.part_buf = part_vec;
-        A.eshift = &W.ks->shift;
-        int gh = 0;
-        int st = launch_hpsi(dtype, HP_LANCZOS, P, A, max_grid_blocks(), s, &gh);
-        if (st) return st;
-        if (dtype == EMUSV_C128)
-            {
-                ProfScope ps_(PROF_ORTH, s);
-                k_orth<double><<<sg, BLOCK, 0, s>>>(W.ks, j, W.part_h, gh, stored(j),
-                                                    j > 0 ? stored(j - 1) : nullptr,
-                                                    const_cast<void *>(stored(j + 1)), D, W.part_o);
-            }
-        else
-            {
-                ProfScope ps_(PROF_ORTH, s);
-                k_orth<float><<<sg, BLOCK, 0, s>>>(W.ks, j, W.part_h, gh, stored(j),
-                                                   j > 0 ? stored(j - 1) : nullptr,
-                                                   const_cast<void *>(stored(j + 1)), D, W.part_o);
-            }
-        EMUSV_CHECK_LAUNCH();
-        // the device tests convergence at every iteration, as the reference does; the host
-        // reads the status (one synchronisation) from the hint on, and kernels launched
-        // after the device converged return at once
-        const int poll = (j + 1 >= krylov_dim_hint) || (j + 1 >= max_krylov_dim);
-        {
-            ProfScope ps_(PROF_SMALL, s);
-            k_small<<<1, 32, 0, s>>>(W.ks, j, W.part_o, sg, dt, exp_tolerance, norm_tolerance, 1,
-                                     j == 0, max_krylov_dim);
-        }
-        EMUSV_CHECK_LAUNCH();
-        if (poll) {
-            st = read_status(W.ks, s, &status);
-            if (st) return st;
-            if (status != KS_RUNNING) break;
-        }
-    }
     if (status == KS_RUNNING) {
         int st = read_status(W.ks, s, &status);
         if (st) return st;
@@ -781,53 +656,31 @@ int emusv_krylov_step(int nqubits, int dtype, double dt, const double *omegas,
     // basis region: [partial-sum vector of the two-pass H*psi][stored_1][stored_2]...
     const int capacity = (int)(W.basis_bytes / (D * es)) - 1;
     if (capacity < 1) return EMUSV_WORKSPACE_TOO_SMALL;
-    const int sg = stream_grid(D);
 
-    int status = KS_RUNNING;
-    {
-        const int st = lanczos_run(P, dtype, dt, psi_in, W.ks, W.part_h, W.part_o, W.basis, capacity,
-                                   exp_tolerance, norm_tolerance, max_krylov_dim, krylov_dim_hint,
-                                   true, s, &status);
+    KHead h;
+    if (persist_applies(dtype, nqubits)) {  // the whole step in one launch
+        const PJob job = {psi_in, psi_out, W.ks, W.x, W.basis, 1};
+        int st = persist_launch(P, dtype, dt, &job, 1, capacity, exp_tolerance, norm_tolerance, max_krylov_dim, s);
+        if (st || (st = read_heads(&W.ks, 1, s, &h))) return st;
+        if (h.kerr) h.status = KS_TIMEOUT;
+        else if (h.status == KS_RUNNING) return EMUSV_WORKSPACE_TOO_SMALL;
+    } else {
+        int status = KS_RUNNING;
+        int st = lanczos_run(P, dtype, dt, psi_in, W.ks, W.part_h, W.part_o, W.basis, capacity,
+                             exp_tolerance, norm_tolerance, max_krylov_dim, krylov_dim_hint, true, s, &status);
         if (st) return st;
-    }
-    if (status == KS_TIMEOUT) {
-        if (info) memset(info, 0, sizeof(*info));
-        return EMUSV_TIMEOUT;
-    }
-    if (status == KS_NONFINITE || status == KS_RUNNING) {
-        if (info) memset(info, 0, sizeof(*info));
-        return EMUSV_NONFINITE;
-    }
-    if (dtype == EMUSV_C128)
-        {
-            ProfScope ps_(PROF_COMBINE, s);
-            k_combine<double><<<sg, BLOCK, 0, s>>>(W.ks, psi_in, W.basis, D, psi_out, W.part_c);
+        h.status = status;
+        if (status == KS_CONVERGED || status == KS_HAPPY || status == KS_MAXDIM) {
+            if ((st = krylov_combine(dtype, W.ks, psi_in, W.basis, D, psi_out, W.part_c, s))) return st;
+            if (info && (st = read_heads(&W.ks, 1, s, &h))) return st;
         }
-    else
-        {
-            ProfScope ps_(PROF_COMBINE, s);
-            k_combine<float><<<sg, BLOCK, 0, s>>>(W.ks, psi_in, W.basis, D, psi_out, W.part_c);
-        }
-    EMUSV_CHECK_LAUNCH();
-    {
-        ProfScope ps_(PROF_SMALL, s);
-        k_finish_combine<<<1, BLOCK, 0, s>>>(W.ks, W.part_c, sg);
     }
-    EMUSV_CHECK_LAUNCH();
-    if (info) {
-        KState h;
-        EMUSV_CHECK(cudaMemcpyAsync(&h, W.ks, offsetof(KState, a_re), cudaMemcpyDeviceToHost, s));
-        EMUSV_CHECK(cudaStreamSynchronize(s));
-        info->iterations = h.iters;
-        info->happy_breakdown = h.status == KS_HAPPY;
-        info->converged = h.status == KS_HAPPY || h.status == KS_CONVERGED;
-        info->basis_vectors = h.nvec;
-        info->error_estimate = h.err;
-        info->input_norm = h.s0;
-        info->output_norm = sqrt(h.outnorm2);
-        info->second_rounds = 0;
+    if (h.status != KS_CONVERGED && h.status != KS_HAPPY && h.status != KS_MAXDIM) {
+        if (info) memset(info, 0, sizeof(*info));
+        return h.status == KS_TIMEOUT ? EMUSV_TIMEOUT : EMUSV_NONFINITE;
     }
-    return status == KS_MAXDIM ? EMUSV_NOT_CONVERGED : EMUSV_OK;
+    if (info) fill_info(h, 0, info);
+    return h.status == KS_MAXDIM ? EMUSV_NOT_CONVERGED : EMUSV_OK;
 }
 
 int emusv_vec_dot(int64_t len, int dtype, const void *a, const void *b, double *res_dev,

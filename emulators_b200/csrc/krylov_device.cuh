@@ -235,11 +235,13 @@ static __device__ void reg_expm(int M, const double2 (&d)[NE], const double2 (&l
 // Bessel values J_k(|z|) in the same order (normalised at the end by
 // J_0 + 2 sum J_2k = 1).  About |z| + 40 tridiagonal products instead of the Taylor
 // form's ~12 |z|.  `Tdiag[e]` is T's (real) diagonal centre of row e and `Trad[e]` its
-// Gershgorin radius (|row| off-diagonal sum of T).
+// Gershgorin radius (|row| off-diagonal sum of T).  `abandon`: when given and set, the
+// result is no longer wanted and y is left undefined (looked at every eighth term).
 template <int NE>
 static __device__ void cheb_expm(const double2 (&d)[NE], const double2 (&l)[NE], const double2 (&u)[NE],
                                  int cpl, double2 cplv, int col, double dt, const double (&Tdiag)[NE],
-                                 const double (&Trad)[NE], int M, double2 (&y)[NE]) {
+                                 const double (&Trad)[NE], int M, double2 (&y)[NE],
+                                 const volatile int *abandon = nullptr) {
     const int lane = threadIdx.x & 31;
     double lo = 1e300, hi = -1e300;
 #pragma unroll
@@ -314,6 +316,7 @@ static __device__ void cheb_expm(const double2 (&d)[NE], const double2 (&l)[NE],
     }
     const double2 up_step = make_double2(0.0, sgn);
     for (int k = K; k >= 1; --k) {
+        if (abandon && (k & 7) == 0 && *abandon) return;
         if ((k & 1) == 0) S += 2.0 * jk;
         if (k <= N) {  // b_k = coef_k e_col + 2 X b_{k+1} - b_{k+2}
             double2 xb[NE];

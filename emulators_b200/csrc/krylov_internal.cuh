@@ -11,13 +11,17 @@ constexpr int KMAX = 128;  // largest max_krylov_dim supported
 enum KStatus { KS_RUNNING = 0, KS_CONVERGED = 1, KS_HAPPY = 2, KS_MAXDIM = 3, KS_NONFINITE = 4,
                KS_TIMEOUT = EMUSV_TIMEOUT };
 
-struct KState {
+// The head of a run's state, what the host reads back.
+struct KHead {
     int status;
     int iters;
     int nvec;
-    int kerr;  // error word of the streaming kernels (EMUSV_TIMEOUT), read by k_small
+    int kerr;  // error word of the run's kernels (EMUSV_TIMEOUT)
     double s0, err, outnorm2;
     double shift;  // sigma: the run works on H - sigma (the previous step's energy), see k_init
+};
+
+struct KState : KHead {
     double a_re[KMAX], a_im[KMAX];   // T_H[k][k]   = <v_k, H v_k> - b_k <v_k, v_{k-1}>
     double b_re[KMAX], b_im[KMAX];   // T_H[k-1][k] = ||w_{k-1}|| (= <v_{k-1}, H v_k> exactly)
     double vv_re[KMAX + 2], vv_im[KMAX + 2];  // <v_k, v_{k-1}>: residual non-orthogonality
@@ -45,6 +49,8 @@ int lanczos_run(const HamParams &P, int dtype, double dt, const void *v0, KState
                 double exp_tol, double norm_tol, int maxdim, int hint, bool energy_shift,
                 cudaStream_t s, int *status_out);
 int read_status(KState *ks, cudaStream_t s, int *out);
+int read_heads(KState *const *ks, int njobs, cudaStream_t s, KHead *out);
+void fill_info(const KHead &h, int second_rounds, emusv_krylov_info *info);
 // Input norm and KState reset (k_norm2 + k_init); with energy_shift, sigma = the previous
 // finished run's sigma + a_re[0] (the workspace must be zeroed before its first run).
 int krylov_begin(int dtype, const void *psi_in, i64 D, KState *ks, double *partials, bool energy_shift,

@@ -1,0 +1,928 @@
+// Single-launch Lanczos runs (see persist.cuh).
+#include <atomic>
+#include <chrono>
+
+#include "persist.cuh"
+#include "profile.cuh"
+
+namespace emusv {
+
+// ------------------------------------------------------------------ records in global memory
+__device__ __forceinline__ void rec_put(PRec *r, double v, unsigned long long e) {
+    asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}"
+                 ::"l"(r), "l"(__double_as_longlong(v)), "l"(e) : "memory");
+}
+template <bool ACQUIRE = false>
+__device__ __forceinline__ PRec rec_get(const PRec *r) {
+    long long v;
+    unsigned long long e;
+    if (ACQUIRE)
+        asm volatile("{\n .reg .b128 t;\n ld.acquire.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+                     : "=l"(v), "=l"(e) : "l"(r) : "memory");
+    else
+    asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+                 : "=l"(v), "=l"(e) : "l"(r) : "memory");
+    PRec o;
+    o.v = __longlong_as_double(v);
+    o.e = e;
+    return o;
+}
+constexpr unsigned long long PSTOP = 1ull << 63;  // epoch flag: the run was decided
+
+// Waits until the record carries the epoch; false on a timeout.
+template <bool ACQUIRE = false>
+__device__ __forceinline__ bool rec_wait(const PRec *r, unsigned long long e, PRec *o) {
+    *o = rec_get<ACQUIRE>(r);
+    if ((o->e & ~PSTOP) == e) return true;
+    const long long t0 = clock64();
+    for (unsigned i = 1;; ++i) {
+        *o = rec_get<ACQUIRE>(r);
+        if ((o->e & ~PSTOP) == e) return true;
+        if ((i & 255u) == 0 && clock64() - t0 > PWAIT_LIMIT) return false;
+    }
+}
+
+// ------------------------------------------------------------------ cluster helpers
+__device__ __forceinline__ uint32_t sm_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t cl_addr(const void *p, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(sm_addr(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ float2 cl_ld(uint32_t a, float2) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ double2 cl_ld(uint32_t a, double2) {
+    double2 v;
+    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cl_st(uint32_t a, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cl_st_rel(uint32_t a, int v) {
+    asm volatile("st.release.cluster.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ int cl_ld_acq(uint32_t a) {
+    int v;
+    asm volatile("ld.acquire.cluster.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void mbar_init_count(uint64_t *bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\nfence.mbarrier_init.release.cluster;"
+                 ::"r"(sm_addr(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void cl_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool cl_wait(uint64_t *bar, uint32_t parity) {
+    const long long t0 = clock64();
+    for (unsigned i = 1;; ++i) {
+        uint32_t ok;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                     " selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(ok) : "r"(sm_addr(bar)), "r"(parity) : "memory");
+        if (ok) return true;
+        if ((i & 255u) == 0 && clock64() - t0 > PWAIT_LIMIT) return false;
+    }
+}
+__device__ __forceinline__ void cl_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// ------------------------------------------------------------------ shared state of a CTA
+template <int CT> struct PShared {
+    double red[2][CT / 32][3];      // the warps' sums, alternating between exchanges
+    double xs[2][3][1 << PCL_BITS]; // the cluster's CTAs' sums of phases A and B
+    double part[3];                 // grid jobs: the sums
+    double up_re[MAXQ], up_im[MAXQ], field[MAXQ];
+    double U[MAXQ * MAXQ];
+    // the run's scalars, every CTA's own copy
+    double ar[KMAX], ai[KMAX], r[KMAX], hn2[KMAX], scale[KMAX + 2];
+    double2 coef[KMAX + 2];
+    int flag[KMAX];
+    int result[KMAX];               // iteration j: 1 goes on, 2 ends the run (in CTA 0 of a
+                                    // cluster job, in the deciding CTA of a grid job)
+    uint64_t bar;
+    volatile int ready;             // iterations whose scalars are here
+    volatile int done;              // the run's status + 1 once it is decided
+    volatile int dead;              // a wait of this CTA ran out
+    int fin[2];
+    double sigma;
+};
+
+template <int CT> __device__ __forceinline__ void compute_sync() {  // the compute warps only
+    asm volatile("bar.sync 1, %0;" ::"n"(CT) : "memory");
+}
+
+// The sums of v[0..2] over the job's compute threads, in every thread, in a fixed order; a
+// barrier of the job (ordering global stores before it for grid jobs when PUBLISH).  PH 0:
+// phase A, 1: phase B.  *stop: CTA 0's flag.  False on a timeout.
+template <int CT, bool CL, int PH, bool PUBLISH>
+__device__ __forceinline__ bool p_exchange(PShared<CT> &sh, double (&v)[3], PExchange *X, unsigned long long e, int r,
+                                           int gbits, uint32_t &parity, bool stop_in, bool *stop) {
+    constexpr int NW = CT / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, G = 1 << gbits;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) sh.red[PH][warp][k] = v[k];
+    }
+    if (gbits == 0 && threadIdx.x == 0) sh.fin[PH] = stop_in;
+    compute_sync<CT>();
+    auto block_total = [&](int k) {
+        double t[NW];
+#pragma unroll
+        for (int w = 0; w < NW; ++w) t[w] = sh.red[PH][w][k];
+#pragma unroll
+        for (int o = NW / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int w = 0; w < o; ++w) t[w] += t[w + o];
+        return t[0];
+    };
+    if (gbits == 0) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) v[k] = block_total(k);
+        *stop = sh.fin[PH] != 0;
+        return true;
+    }
+    if constexpr (CL) {
+        // every CTA receives every CTA's sums (and CTA 0's flag), then the phase completes
+        const int fin = __shfl_sync(0xffffffffu, (int)stop_in, 0);
+        if (warp < 3 && lane < G) {
+            cl_st(cl_addr(&sh.xs[PH][warp][r], lane), block_total(warp));
+            if (warp == 0 && r == 0)
+                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cl_addr(&sh.fin[PH], lane)), "r"(fin)
+                             : "memory");
+            cl_arrive(cl_addr(&sh.bar, lane));
+        }
+        const bool ok = cl_wait(&sh.bar, parity);
+        parity ^= 1u;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            double t = 0.0;
+            for (int g = 0; g < G; g += 2) t += sh.xs[PH][k][g] + sh.xs[PH][k][g + 1];
+            v[k] = t;
+        }
+        *stop = sh.fin[PH] != 0;
+        return ok;
+    } else {
+        // clusters of PGC CTAs first: their sums meet in the cluster's first CTA, which writes
+        // the cluster's records; every CTA reads all clusters' records, one a lane
+        constexpr int PGC = 1 << PGC_BITS;
+        static_assert((PMAXG >> PGC_BITS) <= 32, "a warp reads the records of one sum");
+        PRec(*recs)[PMAXG >> PGC_BITS] = PH == 0 ? X->a : X->b;
+        if (warp < 3) {
+            if (lane == 0) {
+                cl_st(cl_addr(&sh.xs[PH][warp][r & (PGC - 1)], 0), block_total(warp));
+                cl_arrive(cl_addr(&sh.bar, 0));
+            }
+            bool ok = true;
+            if ((r & (PGC - 1)) == 0 && lane == 0) {
+                ok = cl_wait(&sh.bar, parity);
+                double t = 0.0;
+#pragma unroll
+                for (int g = 0; g < PGC; ++g) t += sh.xs[PH][warp][g];
+                if (PUBLISH) __threadfence();  // the cluster's stores before its record
+                rec_put(&recs[warp][r >> PGC_BITS], t, e | (stop_in ? PSTOP : 0ull));
+            }
+            __syncwarp();
+            double t = 0.0;
+            if (lane < (G >> PGC_BITS)) {
+                PRec o;
+                ok = rec_wait<PUBLISH>(&recs[warp][lane], e, &o) && ok;
+                t = o.v;
+                if (warp == 0 && lane == 0) sh.fin[PH] = (o.e & PSTOP) != 0;
+            }
+            t = warp_sum(t);
+            if (lane == 0) sh.part[warp] = t;
+            if (!ok) sh.dead = 1;
+        }
+        parity ^= 1u;
+        compute_sync<CT>();
+#pragma unroll
+        for (int k = 0; k < 3; ++k) v[k] = sh.part[k];
+        *stop = sh.fin[PH] != 0;
+        return sh.dead == 0;
+    }
+}
+
+// ------------------------------------------------------------------ decisions
+// Is the run decided?  (cluster jobs: every CTA's `done`; grid jobs: the verdict record)
+template <int CT, bool CL>
+__device__ __forceinline__ bool p_decided(PShared<CT> &sh, const PExchange *X, unsigned long long epoch) {
+    if (sh.done || sh.dead) return true;
+    if constexpr (!CL) {
+        const PRec v = rec_get(&X->verdict);
+        if (v.e == epoch) {
+            sh.done = (int)v.v + 1;
+            return true;
+        }
+    }
+    return false;
+}
+
+// Announces the run's status to the job's CTAs (one lane; the state's arrays are written).
+template <int CT, bool CL>
+__device__ __forceinline__ void p_announce(PShared<CT> &sh, PExchange *X, unsigned long long epoch, int G, int status) {
+    __threadfence();
+    if constexpr (CL) {
+        for (int g = 0; g < G; ++g) cl_st_rel(cl_addr((const void *)&sh.done, g), status + 1);
+    } else {
+        rec_put(&X->verdict, (double)status, epoch);
+        sh.done = status + 1;
+    }
+}
+
+// Conclusion of iteration j (krylov_exp.py:63-96) by one warp; NE: the smallest register
+// layout that holds the extended matrix's rows.
+template <int NE, int CT, bool CL>
+__device__ __noinline__ void p_conclude(const PArgs &A, const PJob &J, PShared<CT> &sh, int j) {
+    const int lane = threadIdx.x & 31, G = 1 << A.gbits;
+    KState *ks = J.ks;
+    const int m = j + 1, flag = sh.flag[j];
+    const bool ext = flag == KD_OK;
+    double2 y[NE];
+    double err = 0.0;
+    if (flag != KD_NONFINITE) {
+        // rows of A = -i dt T, T real symmetric off its diagonal (b_{k+1} = r_k), and the two
+        // extension rows (krylov_exp.py:77-78)
+        double2 d[NE], l[NE], u[NE];
+        double td[NE], tr[NE];
+#pragma unroll
+        for (int e = 0; e < NE; ++e) {
+            const int k = lane * NE + e;
+            d[e] = l[e] = u[e] = make_double2(0.0, 0.0);
+            td[e] = tr[e] = 0.0;
+            if (k < m) {
+                const double a = sh.ar[k] + sh.sigma, ai = sh.ai[k];  // a_k of H (the run uses H - sigma)
+                d[e] = make_double2(A.dt * ai, -A.dt * a);
+                td[e] = a;
+                tr[e] = fabs(ai);
+                if (k + 1 < m) {
+                    u[e] = make_double2(0.0, -A.dt * sh.r[k]);
+                    tr[e] += fabs(sh.r[k]);
+                }
+            }
+            if (k > 0 && (k < m || (ext && k == m))) {
+                l[e] = make_double2(0.0, -A.dt * sh.r[k - 1]);
+                tr[e] += fabs(sh.r[k - 1]);
+            }
+            if (ext && k == m + 1) {
+                l[e] = make_double2(1.0, 0.0);
+                tr[e] = 1.0 / fabs(A.dt);
+            }
+        }
+        cheb_expm<NE>(d, l, u, -1, make_double2(0.0, 0.0), 0, A.dt, td, tr, ext ? m + 2 : m, y, &sh.done);
+        if (sh.done) return;
+        if (ext) {
+            const double2 x1 = reg_pick(y, m), x2 = reg_pick(y, m + 1);
+            const double hn = sqrt(fmax(0.0, sh.hn2[j]));
+            const double err1 = hypot(x1.x, x1.y);                        // krylov_exp.py:81
+            const double err2 = hypot(x2.x, x2.y) * (fabs(A.dt) * hn);    // krylov_exp.py:82
+            err = err1 < err2 ? err1 : (err1 * err2 / (err1 - err2));     // krylov_exp.py:84
+        }
+    }
+    int st = KS_RUNNING, nvec = j + 2;
+    if (flag == KD_NONFINITE) {
+        st = KS_NONFINITE;
+    } else if (flag == KD_HAPPY) {
+        st = KS_HAPPY;
+        nvec = m;
+    } else if (err < A.exp_tol) {
+        st = KS_CONVERGED;
+    } else if (j + 1 >= A.maxdim) {
+        st = KS_MAXDIM;
+    }
+    const bool ends = st != KS_RUNNING || j + 1 >= A.limit;
+    if (lane == 0) {
+        if constexpr (CL) cl_st_rel(cl_addr(&sh.result[j], 0), ends ? 2 : 1);
+        else *(volatile int *)&sh.result[j] = ends ? 2 : 1;
+    }
+    if (!ends) return;
+    // every earlier iteration must be known to go on
+    const long long t0 = clock64();
+    for (int k = lane; k < j; k += 32) {
+        for (;;) {
+            int res;
+            if constexpr (CL) res = cl_ld_acq(cl_addr(&sh.result[k], 0));
+            else res = *(volatile int *)&sh.result[k];
+            if (res == 2) st = -1;  // an earlier iteration ended the run
+            if (res) break;
+            if (p_decided<CT, CL>(sh, J.x, A.epoch) || clock64() - t0 > PWAIT_LIMIT) {
+                st = -1;
+                break;
+            }
+        }
+        if (st < 0) break;
+    }
+    if (!__all_sync(0xffffffffu, st >= 0)) return;
+    // the run ends here (KS_RUNNING: the basis has no room for another vector)
+    if (st != KS_NONFINITE) {
+#pragma unroll
+        for (int e = 0; e < NE; ++e) {
+            const int k = lane * NE + e;
+            if (k < nvec) {  // c[m] = x1 multiplies v_{j+1} (krylov_exp.py:88-90)
+                ks->c_re[k] = y[e].x;
+                ks->c_im[k] = y[e].y;
+            }
+        }
+    }
+    for (int k = lane; k <= j; k += 32) {  // the run's scalars, as the adjoint reads them
+        const double b = k > 0 ? sh.r[k - 1] : 0.0;
+        ks->a_re[k] = sh.ar[k];
+        ks->a_im[k] = sh.ai[k];
+        ks->b_re[k] = b;
+        ks->b_im[k] = 0.0;
+        ks->r[k] = sh.r[k];
+        ks->hn[k] = sqrt(fmax(0.0, sh.hn2[k]));
+    }
+    for (int k = lane; k <= j + 1; k += 32) ks->scale[k] = sh.scale[k];
+    __syncwarp();
+    if (lane == 0) {
+        ks->status = st;
+        ks->iters = j + 1;
+        ks->nvec = nvec;
+        ks->err = err;
+        p_announce<CT, CL>(sh, J.x, A.epoch, G, st);
+    }
+    __syncwarp();
+}
+
+// The deciding CTA of a grid job: its first warp brings the iterations' scalars from CTA 0's
+// records into shared memory.
+template <int CT>
+__device__ void p_collect(const PArgs &A, const PJob &J, PShared<CT> &sh) {
+    const int lane = threadIdx.x & 31;
+    const unsigned long long e0 = A.epoch + 1;
+    for (int j = -1; j < A.limit; ++j) {
+        PRec q;
+        q.v = 0.0;
+        bool got = true;
+        if (lane < (j < 0 ? 2 : 5)) {
+            const PRec *rec = j < 0 ? &J.x->start[lane] : &J.x->iter[j][lane];
+            const unsigned long long e = j < 0 ? A.epoch : e0 + j;
+            const long long t0 = clock64();
+            for (;;) {
+                q = rec_get(rec);
+                if (q.e == e) break;
+                if (sh.done || sh.dead || clock64() - t0 > PWAIT_LIMIT) {
+                    got = false;
+                    break;
+                }
+            }
+        }
+        if (!__all_sync(0xffffffffu, got)) {
+            if (lane == 0 && !sh.done) {  // a wait ran out
+                sh.dead = 1;
+                atomicExch(&J.ks->kerr, (int)EMUSV_TIMEOUT);
+            }
+            return;
+        }
+        if (j < 0) {
+            if (lane == 0) sh.sigma = q.v;
+            if (lane == 1) sh.scale[0] = q.v;
+        } else {
+            if (lane == 0) sh.ar[j] = q.v;
+            if (lane == 1) sh.ai[j] = q.v;
+            if (lane == 2) {
+                sh.r[j] = q.v;
+                sh.scale[j + 1] = 1.0 / q.v;
+            }
+            if (lane == 3) sh.hn2[j] = q.v;
+            if (lane == 4) sh.flag[j] = (int)q.v;
+        }
+        __syncwarp();
+        __threadfence_block();
+        if (lane == 0) sh.ready = j + 1;
+        __syncwarp();
+    }
+}
+
+// The deciding warps of a CTA: iterations q, q + Q, ... of the job's Q deciding warps.
+template <int CT, bool CL>
+__device__ void p_decider(const PArgs &A, const PJob &J, PShared<CT> &sh, int q, int Q) {
+    const int lane = threadIdx.x & 31;
+    for (int j = q; j < A.limit; j += Q) {
+        int go = 1;
+        if (lane == 0) {
+            const long long t0 = clock64();
+            while (sh.ready <= j) {
+                if (p_decided<CT, CL>(sh, J.x, A.epoch)) {
+                    go = 0;
+                    break;
+                }
+                if (clock64() - t0 > PWAIT_LIMIT) {
+                    sh.dead = 1;
+                    go = 0;
+                    break;
+                }
+                __nanosleep(40);
+            }
+        }
+        if (!__shfl_sync(0xffffffffu, go, 0)) return;
+        __threadfence_block();
+        const int M = j + 3;
+        if (M <= 32) p_conclude<1, CT, CL>(A, J, sh, j);
+        else if (M <= 64) p_conclude<2, CT, CL>(A, J, sh, j);
+        else if (M <= 96) p_conclude<3, CT, CL>(A, J, sh, j);
+        else p_conclude<(KMAX + 2 + 31) / 32, CT, CL>(A, J, sh, j);
+    }
+}
+
+// ------------------------------------------------------------------ the run
+// Cluster jobs: ND deciding warps follow the CT compute threads of every CTA.  Grid jobs (ND =
+// 0): one more CTA decides, so that the compute threads keep 128 registers each.
+template <typename R, bool REALC, int NA, int CT, int ND, bool CL>
+__global__ void __launch_bounds__(CT + 32 * ND, 1) k_lanczos_persist(const __grid_constant__ PArgs A) {
+    typedef typename cvec<R>::T C;
+    constexpr int LB = CT == 256 ? 8 : 9;  // thread bits
+    constexpr int RB = NA == 1 ? 0 : NA == 2 ? 1 : NA == 4 ? 2 : NA == 8 ? 3 : 4;
+    constexpr int GB = CL ? PCL_BITS : PMAXG_BITS;  // CTA bits at most
+    constexpr int CA = NA < (sizeof(R) == 8 ? 2 : 4) ? NA : (sizeof(R) == 8 ? 2 : 4);  // amplitudes at a time
+    extern __shared__ __align__(16) unsigned char psm[];
+    __shared__ PShared<CT> sh;
+    const int S = NA * CT;                  // slots of the arrays below (at least 2^tb)
+    C *us = reinterpret_cast<C *>(psm);     // this CTA's part of v_j (unscaled)
+    C *vps = us + S;                        // cluster jobs: its part of v_{j-1}
+    double *dg = reinterpret_cast<double *>(CL ? vps + S : us + S);  // diagonal minus sigma
+    const int G = 1 << A.gbits;
+    // grid jobs: the compute CTAs of all jobs, then one cluster whose CTA k decides job k
+    const bool decides = !CL && (int)blockIdx.x >= A.njobs << A.gbits;
+    const int r = blockIdx.x & (G - 1);
+    const int jb = decides ? (r < A.njobs ? r : 0) : blockIdx.x >> A.gbits;
+    const PJob &J = A.job[jb];
+    const HamParams &P = A.P;
+    const int n = P.n, tb = A.tbits, nlow = tb < LB ? tb : LB;
+    const int tid = threadIdx.x;
+    KState *ks = J.ks;
+    PExchange *X = J.x;
+    if (tid == 0) {
+        sh.ready = 0;
+        sh.done = 0;
+        sh.dead = 0;
+        mbar_init_count(&sh.bar, CL ? 3 * G : 3 << PGC_BITS);
+        // sigma from the previous finished run (read before anyone overwrites the state)
+        double sg = 0.0;
+        if (J.energy_shift && (ks->status == KS_CONVERGED || ks->status == KS_HAPPY) && ks->iters > 0) {
+            sg = ks->shift + ks->a_re[0];
+            if (!isfinite(sg) || fabs(sg) > 1e12) sg = 0.0;
+        }
+        sh.sigma = sg;
+    }
+    for (int k = tid; k < n; k += blockDim.x) {
+        sh.up_re[k] = P.up_re[k];
+        sh.up_im[k] = P.up_im[k];
+        sh.field[k] = P.field[k];
+    }
+    for (int k = tid; k < n * MAXQ; k += blockDim.x) sh.U[k] = P.U[k];
+    for (int k = tid; k < KMAX; k += blockDim.x) sh.result[k] = 0;
+    __syncthreads();
+    cl_sync_all();  // mbarriers and flags are set before a sibling touches them
+    if constexpr (CL) {
+        if (tid >= CT) {
+            p_decider<CT, CL>(A, J, sh, r + (((tid - CT) >> 5) << A.gbits), ND << A.gbits);
+            cl_sync_all();
+            return;
+        }
+    } else if (decides) {
+        if (r < A.njobs) {
+            if (tid < 32) p_collect<CT>(A, J, sh);
+            else p_decider<CT, CL>(A, J, sh, (tid >> 5) - 1, CT / 32 - 1);
+        }
+        cl_sync_all();
+        return;
+    }
+    const i64 D = i64(1) << n, base = (i64)r << tb;
+    const bool on = tid < (1 << nlow);  // fewer amplitudes than threads on the smallest registers
+    const double sigma = sh.sigma;
+    const C zero = cmake<C>(0.0, 0.0);
+    const C *u0 = reinterpret_cast<const C *>(J.v0) + base;
+    C *bs = reinterpret_cast<C *>(J.basis) + base;  // slot k at bs + k * D
+    double acc[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+        const int l = tid + a * CT;
+        const C v = on ? u0[l] : zero;
+        us[l] = v;
+        if (CL) vps[l] = zero;
+        acc[0] += double(v.x) * double(v.x) + double(v.y) * double(v.y);
+    }
+    {  // diagonal: thread and CTA bits, then the register bits with their crosses
+        const unsigned x = (unsigned)base + tid;
+        double e = -sigma, f[RB > 0 ? RB : 1];
+#pragma unroll
+        for (int k = 0; k < RB; ++k) f[k] = sh.field[LB + k];
+        for (unsigned m = x; m; m &= m - 1) {
+            const int p = __ffs(m) - 1;
+            const double *Up = sh.U + p * MAXQ;
+            e += sh.field[p];
+            for (unsigned q = m & (m - 1); q; q &= q - 1) e += Up[__ffs(q) - 1];
+#pragma unroll
+            for (int k = 0; k < RB; ++k) f[k] += Up[LB + k];
+        }
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            double t = e;
+#pragma unroll
+            for (int k = 0; k < RB; ++k)
+                if ((a >> k) & 1) {
+                    t += f[k];
+#pragma unroll
+                    for (int k2 = k + 1; k2 < RB; ++k2)
+                        if ((a >> k2) & 1) t += sh.U[(LB + k) * MAXQ + LB + k2];
+                }
+            dg[tid + a * CT] = t;
+        }
+    }
+    uint32_t parity = 0;
+    bool stop = false;
+    // every CTA has read the previous state once this exchange is complete
+    bool ok = p_exchange<CT, CL, 1, false>(sh, acc, X, A.epoch, r, A.gbits, parity, false, &stop);
+    const double s0 = sqrt(acc[0]);  // krylov_exp.py:43
+    const bool fine = isfinite(s0) && s0 > 0.0;
+    double sj = 1.0 / s0, sp = 0.0, b = 0.0, vvr = 0.0, vvi = 0.0;
+    if (tid == 0) {
+        sh.scale[0] = sj;
+        if (r == 0) {
+            ks->s0 = s0;
+            ks->shift = sigma;
+            ks->outnorm2 = 0.0;
+            ks->kerr = 0;
+            if (!CL) {
+                rec_put(&X->start[0], sigma, A.epoch);
+                rec_put(&X->start[1], sj, A.epoch);
+            }
+        }
+        if (!fine) {  // decided as iteration 0
+            sh.ar[0] = sh.ai[0] = sh.r[0] = sh.hn2[0] = 0.0;
+            sh.scale[1] = 0.0;
+            sh.flag[0] = KD_NONFINITE;
+            __threadfence_block();
+            sh.ready = 1;
+        }
+    }
+    const unsigned long long e0 = A.epoch + 1;
+    if (!CL && !fine && r == 0 && tid < 5) rec_put(&X->iter[0][tid], tid == 4 ? (double)KD_NONFINITE : 0.0, e0);
+    for (int j = 0; fine && ok && !stop && j < A.limit; ++j) {
+        // grid jobs: CTA 0 looks whether the run is decided, meanwhile
+        PRec vd;
+        vd.e = 0;
+        if (!CL && r == 0 && tid == CT - 1) vd = rec_get(&X->verdict);
+        const C *uj = j == 0 ? reinterpret_cast<const C *>(J.v0) : reinterpret_cast<const C *>(J.basis) + (i64)j * D;
+        // ---------------- A: h = (H - sigma) v_j
+        double hr[NA], hi[NA];
+        acc[0] = acc[1] = acc[2] = 0.0;
+#pragma unroll
+        for (int a0 = 0; a0 < NA; a0 += CA) {
+            // the CTA bits: partners in the other CTAs' parts, in flight during the rest
+            C q[GB][CA];
+#pragma unroll
+            for (int k = 0; k < GB; ++k) {
+                if (k >= A.gbits) {
+#pragma unroll
+                    for (int a = 0; a < CA; ++a) q[k][a] = zero;
+                    continue;
+                }
+                if constexpr (CL) {
+                    const uint32_t pa = cl_addr(us, (uint32_t)(r ^ (1 << k))) + (uint32_t)((tid + a0 * CT) * sizeof(C));
+#pragma unroll
+                    for (int a = 0; a < CA; ++a) q[k][a] = cl_ld(pa + (uint32_t)(a * CT * sizeof(C)), zero);
+                } else {
+                    const C *pp = uj + (base ^ (i64(1) << (tb + k))) + tid + a0 * CT;
+#pragma unroll
+                    for (int a = 0; a < CA; ++a) q[k][a] = __ldcg(pp + a * CT);
+                }
+            }
+            R ar[CA], ai[CA];
+#pragma unroll
+            for (int a = 0; a < CA; ++a) ar[a] = ai[a] = R(0);
+            auto flip = [&](int a, R cr, R ci, const C &w) {
+                if (REALC) {
+                    ar[a] = fmar(cr, w.x, ar[a]);
+                    ai[a] = fmar(cr, w.y, ai[a]);
+                } else {
+                    ar[a] = fmar(cr, w.x, fmar(-ci, w.y, ar[a]));
+                    ai[a] = fmar(cr, w.y, fmar(ci, w.x, ai[a]));
+                }
+            };
+            // thread and register bits: partners in shared memory
+#pragma unroll
+            for (int k = 0; k < LB; ++k) {
+                if (k >= nlow) break;
+                const R cr = R(sh.up_re[k]);
+                R ci = REALC ? R(0) : R(sh.up_im[k]);
+                if (!((tid >> k) & 1)) ci = -ci;
+#pragma unroll
+                for (int a = 0; a < CA; ++a) flip(a, cr, ci, us[(tid ^ (1 << k)) + (a0 + a) * CT]);
+            }
+#pragma unroll
+            for (int k = 0; k < RB; ++k) {
+                const R cr = R(sh.up_re[LB + k]), ci = REALC ? R(0) : R(sh.up_im[LB + k]);
+#pragma unroll
+                for (int a = 0; a < CA; ++a)
+                    flip(a, cr, ((a0 + a) >> k) & 1 ? ci : -ci, us[tid + ((a0 + a) ^ (1 << k)) * CT]);
+            }
+#pragma unroll
+            for (int k = 0; k < GB; ++k) {
+                if (k >= A.gbits) break;
+                const R cr = R(sh.up_re[tb + k]);
+                R ci = REALC ? R(0) : R(sh.up_im[tb + k]);
+                if (!((r >> k) & 1)) ci = -ci;
+#pragma unroll
+                for (int a = 0; a < CA; ++a) flip(a, cr, ci, q[k][a]);
+            }
+#pragma unroll
+            for (int a = 0; a < CA; ++a) {
+                const C v = us[tid + (a0 + a) * CT];
+                const double d = dg[tid + (a0 + a) * CT], vx = double(v.x), vy = double(v.y);
+                const double x = on ? sj * (double(ar[a]) + d * vx) : 0.0;
+                const double y = on ? sj * (double(ai[a]) + d * vy) : 0.0;
+                hr[a0 + a] = x;
+                hi[a0 + a] = y;
+                acc[0] += vx * x + vy * y;
+                acc[1] += vx * y - vy * x;
+                acc[2] += x * x + y * y;
+            }
+        }
+        acc[0] *= sj;
+        acc[1] *= sj;
+        constexpr bool PRE = !CL && NA <= 4;  // v_{j-1} loaded ahead of the exchange
+        const C *up = j == 1 ? u0 : bs + (i64)(j - 1) * D;
+        C vp[PRE ? NA : 1];
+        if (PRE) {
+#pragma unroll
+            for (int a = 0; a < NA; ++a) vp[a] = j > 0 ? __ldcg(up + tid + a * CT) : zero;
+        }
+        bool dummy;
+        ok = p_exchange<CT, CL, 0, false>(sh, acc, X, e0 + 2 * j, r, A.gbits, parity, false, &dummy);
+        if (!ok) break;
+        // ---------------- B: w = h - a v_j - b v_{j-1}
+        const double are = acc[0] - b * vvr, aim = acc[1] - b * vvi;
+        const double car = are * sj, cai = aim * sj, cb = b * sp;
+        const double hn2 = acc[2] + 2.0 * sigma * acc[0] + sigma * sigma;
+        acc[0] = acc[1] = acc[2] = 0.0;
+        C *w = bs + (i64)(j + 1) * D;
+        constexpr int BA = NA < 4 ? NA : 4;
+#pragma unroll
+        for (int a0 = 0; a0 < NA; a0 += BA) {
+            C p[BA];
+#pragma unroll
+            for (int a = 0; a < BA; ++a) {
+                if (CL) p[a] = vps[tid + (a0 + a) * CT];
+                else if (PRE) p[a] = vp[PRE ? a0 + a : 0];
+                else p[a] = j > 0 ? __ldcg(up + tid + (a0 + a) * CT) : zero;
+            }
+#pragma unroll
+            for (int a = 0; a < BA; ++a) {
+                const int l = tid + (a0 + a) * CT;
+                const C v = us[l];
+                const double vx = double(v.x), vy = double(v.y);
+                const double wr = hr[a0 + a] - (car * vx - cai * vy) - cb * double(p[a].x);
+                const double wi = hi[a0 + a] - (car * vy + cai * vx) - cb * double(p[a].y);
+                const C o = on ? cmake<C>(wr, wi) : zero;
+                if (on) w[l] = o;
+                us[l] = o;  // phase A's readers are past the exchange
+                if (CL) vps[l] = v;
+                const double ox = double(o.x), oy = double(o.y);
+                acc[0] += ox * ox + oy * oy;
+                acc[1] += vx * ox + vy * oy;  // <v_j, w>
+                acc[2] += vx * oy - vy * ox;
+            }
+        }
+        acc[1] *= sj;
+        acc[2] *= sj;
+        if (!CL && r == 0 && tid == CT - 1 && vd.e == A.epoch) sh.done = (int)vd.v + 1;
+        ok = p_exchange<CT, CL, 1, true>(sh, acc, X, e0 + 2 * j + 1, r, A.gbits, parity,
+                                         r == 0 && tid == 0 && sh.done, &stop);
+        if (!ok) break;
+        const double rj = sqrt(acc[0]), inv = 1.0 / rj;
+        int flag = KD_OK;
+        if (!isfinite(rj) || !isfinite(hn2) || !isfinite(are) || !isfinite(aim)) flag = KD_NONFINITE;
+        else if (fabs(A.dt) * rj < A.norm_tol) flag = KD_HAPPY;
+        if (!CL && r == 0 && tid < 5)
+            rec_put(&X->iter[j][tid],
+                    tid == 0 ? are : tid == 1 ? aim : tid == 2 ? rj : tid == 3 ? hn2 : (double)flag, e0 + j);
+        if (tid == 0) {
+            sh.scale[j + 1] = inv;
+            if (CL) {
+                sh.ar[j] = are;
+                sh.ai[j] = aim;
+                sh.r[j] = rj;
+                sh.hn2[j] = hn2;
+                sh.flag[j] = flag;
+                __threadfence_block();
+                sh.ready = j + 1;
+            }
+        }
+        sp = sj;
+        sj = inv;
+        b = rj;
+        vvr = acc[1] * inv;  // <v_{j+1}, v_j> = conj(<v_j, w>) / ||w||
+        vvi = -acc[2] * inv;
+        if (flag != KD_OK) break;
+    }
+    // ---------------- the verdict and the combination out = s0 sum_k c_k v_k
+    if (tid == 0) {
+        const long long t0 = clock64();
+        while (ok && !p_decided<CT, CL>(sh, X, A.epoch))
+            if (clock64() - t0 > PWAIT_LIMIT) sh.dead = 1;
+        if (!ok) sh.dead = 1;
+        if (sh.dead) atomicExch(&ks->kerr, (int)EMUSV_TIMEOUT);
+        __threadfence();
+    }
+    compute_sync<CT>();
+    const int st = sh.done - 1;
+    if (!sh.dead && J.out && (st == KS_CONVERGED || st == KS_HAPPY || st == KS_MAXDIM)) {
+        const int nv = __ldcg(&ks->nvec);
+        for (int k = tid; k < nv; k += CT) {
+            const double f = s0 * sh.scale[k];
+            sh.coef[k] = make_double2(f * __ldcg(&ks->c_re[k]), f * __ldcg(&ks->c_im[k]));
+        }
+        compute_sync<CT>();
+        acc[0] = acc[1] = acc[2] = 0.0;
+        C *out = reinterpret_cast<C *>(J.out) + base;
+        constexpr int OA = NA < 4 ? NA : 4, KU = 16 / OA;  // 16 loads in flight
+#pragma unroll
+        for (int a0 = 0; a0 < NA; a0 += OA) {
+            if (!on) break;
+            double re[OA], im[OA];
+#pragma unroll
+            for (int a = 0; a < OA; ++a) {
+                const C v = u0[tid + (a0 + a) * CT];
+                re[a] = sh.coef[0].x * double(v.x) - sh.coef[0].y * double(v.y);
+                im[a] = sh.coef[0].x * double(v.y) + sh.coef[0].y * double(v.x);
+            }
+            for (int k = 1; k < nv; k += KU) {
+                C q[KU][OA];
+#pragma unroll
+                for (int u = 0; u < KU; ++u)
+#pragma unroll
+                    for (int a = 0; a < OA; ++a)
+                        q[u][a] = k + u < nv ? __ldcs(bs + (i64)(k + u) * D + tid + (a0 + a) * CT) : zero;
+#pragma unroll
+                for (int u = 0; u < KU; ++u) {
+                    if (k + u >= nv) break;
+                    const double2 c = sh.coef[k + u];
+#pragma unroll
+                    for (int a = 0; a < OA; ++a) {
+                        re[a] += c.x * double(q[u][a].x) - c.y * double(q[u][a].y);
+                        im[a] += c.x * double(q[u][a].y) + c.y * double(q[u][a].x);
+                    }
+                }
+            }
+#pragma unroll
+            for (int a = 0; a < OA; ++a) {
+                const C o = cmake<C>(re[a], im[a]);
+                out[tid + (a0 + a) * CT] = o;
+                acc[0] += double(o.x) * double(o.x) + double(o.y) * double(o.y);
+            }
+        }
+        ok = p_exchange<CT, CL, 0, false>(sh, acc, X, A.epoch + 4 * KMAX - 1, r, A.gbits, parity, false, &stop);
+        if (r == 0 && tid == 0) {
+            ks->outnorm2 = acc[0];
+            if (!ok) atomicExch(&ks->kerr, (int)EMUSV_TIMEOUT);
+        }
+    }
+    cl_sync_all();  // no CTA leaves while a sibling may still read its shared memory
+}
+
+// ------------------------------------------------------------------ host side
+struct PShape {
+    bool cluster;
+    int gbits, tbits, na_bits;
+};
+// Cluster jobs hold v_j, v_{j-1} and the diagonal in shared memory; 256 compute threads and
+// four deciding warps.  Grid jobs read v_{j-1} from the basis; 512 compute threads, a deciding
+// CTA.
+constexpr int CCT = 256, CND = 4, GCT = 512;
+static size_t persist_smem(const PShape &s, int dtype) {
+    const int lb = s.cluster ? 8 : 9;
+    const size_t es = dtype == EMUSV_C128 ? 16 : 8, slots = size_t(1) << (s.tbits > lb ? s.tbits : lb);
+    return slots * (es * (s.cluster ? 2 : 1) + sizeof(double));
+}
+// One CTA up to 11 qubits (11 qubits on four CTAs: 76 us a step of 16 iterations, on one 82 with
+// three SMs left to others); clusters to 15 (16 qubits on a cluster of 16: 14.6 us an
+// iteration, on the grid 10: the partners' amplitudes come through distributed shared memory
+// at about 18 bytes a clock); the grid to 20, where v_j and the diagonal still fit (20 qubits
+// complex128: 1370 us against 1909 for the streaming passes).
+static PShape persist_shape(int n, int njobs) {
+    PShape s;
+    s.cluster = n <= 15;
+    if (s.cluster) s.gbits = n <= 11 ? 0 : (n == 12 ? 3 : PCL_BITS);
+    else s.gbits = njobs == 2 ? PMAXG_BITS - 1 : PMAXG_BITS;  // side by side on half the CTAs each
+    s.tbits = n - s.gbits;
+    const int lb = s.cluster ? 8 : 9;
+    s.na_bits = s.tbits > lb ? s.tbits - lb : 0;
+    return s;
+}
+// Clusters of a grid job that the current device holds at once (a CTA per SM).
+static int grid_clusters() {
+    static std::atomic<int> cached[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    int n = cached[dev].load();
+    if (n) return n;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1 << PGC_BITS);
+    cfg.blockDim = dim3(GCT);
+    cfg.dynamicSmemBytes = 0;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1 << PGC_BITS;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, k_lanczos_persist<double, true, 1, GCT, 0, false>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+    }
+    cached[dev].store(n);
+    return n;
+}
+static bool shape_fits(const PShape &s, int dtype, int njobs) {
+    return s.na_bits <= 4 && persist_smem(s, dtype) <= 200 * 1024 &&
+           (s.cluster || (njobs << s.gbits >> PGC_BITS) + 1 <= grid_clusters());
+}
+
+bool persist_applies(int dtype, int n) {
+    return n >= 1 && (dtype == EMUSV_C128 || dtype == EMUSV_C64) && shape_fits(persist_shape(n, 1), dtype, 1);
+}
+size_t persist_exchange_bytes() { return (sizeof(PExchange) + 255) / 256 * 256; }
+
+// Epochs of a launch: 4 KMAX consecutive values that no other launch uses.
+static unsigned long long next_epoch() {
+    static std::atomic<unsigned long long> next{
+        ((unsigned long long)std::chrono::steady_clock::now().time_since_epoch().count() << 10) & ~(1ull << 63)};
+    return next.fetch_add(4 * KMAX) & ~(1ull << 63);
+}
+
+template <typename R, bool REALC, int NA>
+static void *pick_na(bool cluster) {
+    return cluster ? reinterpret_cast<void *>(k_lanczos_persist<R, REALC, NA, CCT, CND, true>)
+                   : reinterpret_cast<void *>(k_lanczos_persist<R, REALC, NA, GCT, 0, false>);
+}
+template <typename R, bool REALC>
+static void *pick(const PShape &s) {
+    switch (s.na_bits) {
+    case 0: return pick_na<R, REALC, 1>(s.cluster);
+    case 1: return pick_na<R, REALC, 2>(s.cluster);
+    case 2: return pick_na<R, REALC, 4>(s.cluster);
+    case 3: return pick_na<R, REALC, 8>(s.cluster);
+    default: return pick_na<R, REALC, 16>(s.cluster);
+    }
+}
+
+int persist_launch(const HamParams &P, int dtype, double dt, const PJob *jobs, int njobs, int capacity,
+                   double exp_tol, double norm_tol, int maxdim, cudaStream_t s) {
+    PShape sh = persist_shape(P.n, njobs);
+    int together = njobs;
+    if (!shape_fits(sh, dtype, njobs)) {  // in turn
+        sh = persist_shape(P.n, 1);
+        together = 1;
+    }
+    PArgs A;
+    A.P = P;
+    A.njobs = together;
+    A.gbits = sh.gbits;
+    A.tbits = sh.tbits;
+    A.limit = maxdim < capacity ? maxdim : capacity;
+    A.maxdim = maxdim;
+    A.dt = dt;
+    A.exp_tol = exp_tol;
+    A.norm_tol = norm_tol;
+    const size_t smem = persist_smem(sh, dtype);
+    void *kern = dtype == EMUSV_C128 ? (P.real_coef ? pick<double, true>(sh) : pick<double, false>(sh))
+                                     : (P.real_coef ? pick<float, true>(sh) : pick<float, false>(sh));
+    EMUSV_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (sh.cluster && sh.gbits > 3) EMUSV_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    for (int j0 = 0; j0 < njobs; j0 += together) {
+        for (int j = 0; j < together; ++j) A.job[j] = jobs[j0 + j];
+        A.epoch = next_epoch();
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((together << sh.gbits) + (sh.cluster ? 0 : 1 << PGC_BITS));
+        cfg.blockDim = dim3(sh.cluster ? CCT + 32 * CND : GCT);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1u << (sh.cluster ? sh.gbits : PGC_BITS);
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeCooperative;  // grid jobs wait for one another's CTAs:
+        attr[1].val.cooperative = 1;                  // all resident at once
+        cfg.attrs = attr;
+        cfg.numAttrs = sh.cluster ? 1 : 2;
+        void *args[] = {(void *)&A};
+        ProfScope ps_(PROF_HPSI, s);
+        EMUSV_CHECK(cudaLaunchKernelExC(&cfg, kern, args));
+    }
+    return EMUSV_OK;
+}
+
+}  // namespace emusv
