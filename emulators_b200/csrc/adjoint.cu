@@ -22,6 +22,7 @@
 
 #include "pairsums.cuh"
 #include "persist.cuh"
+#include "tridiag_real.cuh"
 #include "profile.cuh"
 
 namespace emusv {
@@ -92,26 +93,14 @@ static bool carve_adj(void *ws, size_t bytes, int64_t D, size_t es, AdjWorkspace
 // of each basis, coupling 1; double_krylov.py:54-57), rows 0..ms-1.  T (double_krylov.py:
 // 100-113) has size m = j+2 after convergence (last row: T[j+1][j] = ||w_j||, T[j+1][j+1]
 // = 0) or j+1 after a happy breakdown.  One warp per column, Chebyshev form
-// (cheb_expm: the spectrum of B is that of its two blocks).
-__device__ __forceinline__ void adj_block_row(const KState *ks, int kk, int m, double dt,
-                                              double2 &d, double2 &l, double2 &u, double &td,
-                                              double &tr) {
+// (cheb_expm_real: the spectrum of B is that of its two blocks).
+// In units of T the coupling is i/dt; the gradient block's components taken times i make the
+// matrix real (cheb_expm_real) and the wanted block i times its own.
+__device__ __forceinline__ void adj_block_row(const KState *ks, int kk, int m, double &d, double &l, double &u) {
     const int jj = ks->iters - 1;
-    d = l = u = make_double2(0.0, 0.0);
-    td = tr = 0.0;
-    if (kk <= jj) {
-        d = make_double2(dt * ks->a_im[kk], -dt * (ks->a_re[kk] + ks->shift));
-        td = ks->a_re[kk] + ks->shift;
-        tr = fabs(ks->a_im[kk]);
-    }
-    if (kk >= 1) {
-        l = make_double2(0.0, -dt * ks->r[kk - 1]);
-        tr += fabs(ks->r[kk - 1]);
-    }
-    if (kk + 1 <= jj && kk + 1 < m) {
-        u = make_double2(dt * ks->b_im[kk + 1], -dt * ks->b_re[kk + 1]);
-        tr += hypot(ks->b_re[kk + 1], ks->b_im[kk + 1]);
-    }
+    d = kk <= jj ? ks->a_re[kk] + ks->shift : 0.0;
+    l = kk >= 1 ? ks->r[kk - 1] : 0.0;
+    u = kk + 1 <= jj && kk + 1 < m ? ks->b_re[kk + 1] : 0.0;
 }
 
 constexpr int DS_WARPS = 4;
@@ -125,22 +114,20 @@ k_dS(const KState *ks_s, const KState *ks_g, double dt, double2 *dS) {
     const int M = ms + mg;
     const int col = blockIdx.x * DS_WARPS + warp;
     if (col >= mg || M > 32 * ADS_NE) return;
-    double2 d[ADS_NE], l[ADS_NE], u[ADS_NE], y[ADS_NE];
-    double td[ADS_NE], tr[ADS_NE];
+    double d[ADS_NE], l[ADS_NE], u[ADS_NE];
+    double2 y[ADS_NE];
 #pragma unroll
     for (int e = 0; e < ADS_NE; ++e) {
         const int k = lane * ADS_NE + e;
-        d[e] = l[e] = u[e] = make_double2(0.0, 0.0);
-        td[e] = tr[e] = 0.0;
-        if (k < ms) adj_block_row(ks_s, k, ms, dt, d[e], l[e], u[e], td[e], tr[e]);
-        else if (k < M) adj_block_row(ks_g, k - ms, mg, dt, d[e], l[e], u[e], td[e], tr[e]);
-        if (k == 0) tr[e] += 1.0 / fabs(dt);  // the coupling entry 1 in T units
+        d[e] = l[e] = u[e] = 0.0;
+        if (k < ms) adj_block_row(ks_s, k, ms, d[e], l[e], u[e]);
+        else if (k < M) adj_block_row(ks_g, k - ms, mg, d[e], l[e], u[e]);
     }
-    cheb_expm<ADS_NE>(d, l, u, ms, make_double2(1.0, 0.0), ms + col, dt, td, tr, M, y);
+    cheb_expm_real<ADS_NE>(d, l, u, ms, 1.0 / dt, ms + col, dt, M, y);
 #pragma unroll
     for (int e = 0; e < ADS_NE; ++e) {
         const int r = lane * ADS_NE + e;
-        if (r < ms) dS[r * KMAX + col] = y[e];
+        if (r < ms) dS[r * KMAX + col] = make_double2(-y[e].y, y[e].x);  // i y
     }
 }
 

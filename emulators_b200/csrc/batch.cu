@@ -46,8 +46,8 @@
 #include <unordered_map>
 #include <vector>
 
-#include "krylov_device.cuh"
 #include "profile.cuh"
+#include "tridiag_real.cuh"
 
 namespace emusv {
 
@@ -1089,27 +1089,13 @@ __device__ __forceinline__ bool job_ok(const KState *ks) {
 // B = [[A_s, e0 e0^T], [0, A_g]] (A = -i dt T of each basis, the coupling taken as 1:
 // double_krylov.py:54-57 scales it by |state||grad| afterwards), rows 0..ms-1 of y.
 // One warp per column, Chebyshev form (the spectrum of B is that of the two blocks).
-__device__ __forceinline__ void block_row(const KState *ks, int kk, int m, double dt, double2 &d,
-                                          double2 &l, double2 &u, double &td, double &tr) {
+// In units of T the coupling is i/dt; the gradient block's components taken times i make the
+// matrix real (cheb_expm_real) and the wanted block i times its own.
+__device__ __forceinline__ void block_row(const KState *ks, int kk, int m, double &d, double &l, double &u) {
     const int jj = __ldcg(&ks->iters) - 1;  // last Lanczos column; row jj+1 is the appended one
-    d = l = u = make_double2(0.0, 0.0);
-    td = tr = 0.0;
-    if (kk <= jj) {
-        const double ar = __ldcg(&ks->a_re[kk]) + __ldcg(&ks->shift), ai = __ldcg(&ks->a_im[kk]);
-        d = make_double2(dt * ai, -dt * ar);
-        td = ar;
-        tr = fabs(ai);
-    }
-    if (kk >= 1) {
-        const double r = __ldcg(&ks->r[kk - 1]);
-        l = make_double2(0.0, -dt * r);
-        tr += fabs(r);
-    }
-    if (kk + 1 <= jj && kk + 1 < m) {
-        const double br = __ldcg(&ks->b_re[kk + 1]), bi = __ldcg(&ks->b_im[kk + 1]);
-        u = make_double2(dt * bi, -dt * br);
-        tr += hypot(br, bi);
-    }
+    d = kk <= jj ? __ldcg(&ks->a_re[kk]) + __ldcg(&ks->shift) : 0.0;
+    l = kk >= 1 ? __ldcg(&ks->r[kk - 1]) : 0.0;
+    u = kk + 1 <= jj && kk + 1 < m ? __ldcg(&ks->b_re[kk + 1]) : 0.0;
 }
 
 constexpr int DS_NE = 8;  // block matrices up to 256 rows
@@ -1122,23 +1108,21 @@ __global__ void __launch_bounds__(BWARPS * 32) k_batch_dS(const BArgs A, const B
     const int ms = basis_size(kss), mg = basis_size(ksg), M = ms + mg;
     if (col >= mg || M > 32 * DS_NE || ms > D.mmax || mg > D.mmax) return;
     const double dt = A.inst[2 * i].dt;
-    double2 d[DS_NE], l[DS_NE], u[DS_NE], y[DS_NE];
-    double td[DS_NE], tr[DS_NE];
+    double d[DS_NE], l[DS_NE], u[DS_NE];
+    double2 y[DS_NE];
 #pragma unroll
     for (int e = 0; e < DS_NE; ++e) {
         const int k = lane * DS_NE + e;
-        d[e] = l[e] = u[e] = make_double2(0.0, 0.0);
-        td[e] = tr[e] = 0.0;
-        if (k < ms) block_row(kss, k, ms, dt, d[e], l[e], u[e], td[e], tr[e]);
-        else if (k < M) block_row(ksg, k - ms, mg, dt, d[e], l[e], u[e], td[e], tr[e]);
-        if (k == 0) tr[e] += 1.0 / fabs(dt);  // the coupling entry 1 in T units
+        d[e] = l[e] = u[e] = 0.0;
+        if (k < ms) block_row(kss, k, ms, d[e], l[e], u[e]);
+        else if (k < M) block_row(ksg, k - ms, mg, d[e], l[e], u[e]);
     }
-    cheb_expm<DS_NE>(d, l, u, ms, make_double2(1.0, 0.0), ms + col, dt, td, tr, M, y);
+    cheb_expm_real<DS_NE>(d, l, u, ms, 1.0 / dt, ms + col, dt, M, y);
     double2 *out = D.dS + (size_t)i * D.mmax * D.mmax;
 #pragma unroll
     for (int e = 0; e < DS_NE; ++e) {
         const int r = lane * DS_NE + e;
-        if (r < ms) out[r * D.mmax + col] = y[e];
+        if (r < ms) out[r * D.mmax + col] = make_double2(-y[e].y, y[e].x);  // i y
     }
 }
 
