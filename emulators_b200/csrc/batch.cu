@@ -38,6 +38,11 @@
 //    rounds win on batches of uneven registers (256 registers of 12-18 qubits, 150
 //    steps: 0.79 s against 0.92 s), the phases on uniform ones (64 registers of 16 qubits,
 //    the gradient batch's forward).
+//  * where every tile of a batch has a warp of its own the phase engine runs as gangs
+//    (k_batch_gang, below): the same tiles and sums, so the same bits, with the exchanges
+//    inside a register's own warps.  It takes those batches for the forward engine 1 and for
+//    the adjoint's bases: the forward and adjoint sweep of 12 registers of 14 qubits, 10 steps,
+//    complex128: 117 ms by the phase engine, 41 ms by gangs.
 #include <math.h>
 #include <string.h>
 
@@ -46,8 +51,8 @@
 #include <unordered_map>
 #include <vector>
 
+#include "persist_device.cuh"
 #include "profile.cuh"
-#include "tridiag_real.cuh"
 
 namespace emusv {
 
@@ -292,9 +297,9 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // ---------------------------------------------------------------- phase A: H v_j on a tile
+// (returns the tile's ||H v||^2 and <v_j, H v_j>, in every lane)
 template <typename R, int T>
-__device__ bool tile_hpsi(const BArgs &A, const BInst &I, int i, int t, int step, int j,
-                          double sj) {
+__device__ __forceinline__ double3 tile_hpsi_sums(const BArgs &A, const BInst &I, int t, int step, int j, double sj) {
     typedef typename cvec<R>::T C;
     constexpr int AMP = 1 << (T - 5);
     const int lane = threadIdx.x & 31;
@@ -419,19 +424,27 @@ __device__ bool tile_hpsi(const BArgs &A, const BInst &I, int i, int t, int step
     }
     const double s2 = warp_sum((double)h2), s_r = warp_sum(sj * (double)dr),
                  s_i = warp_sum(sj * (double)di);
-    if (lane == 0) {
-        double *pa = A.partA + 4 * (size_t)t;
-        pa[0] = s2;
-        pa[1] = s_r;
-        pa[2] = s_i;
+    return make_double3(s2, s_r, s_i);
+}
+__device__ __forceinline__ void put_part(double *part, int t, double3 s) {
+    if ((threadIdx.x & 31) == 0) {
+        double *p = part + 4 * (size_t)t;
+        p[0] = s.x;
+        p[1] = s.y;
+        p[2] = s.z;
     }
+}
+template <typename R, int T>
+__device__ bool tile_hpsi(const BArgs &A, const BInst &I, int i, int t, int step, int j, double sj) {
+    put_part(A.partA, t, tile_hpsi_sums<R, T>(A, I, t, step, j, sj));
     return tile_done(A.cnt, A.partA, A.sumA, i, I.tile0, I.ntiles);
 }
 
 // ---------------------------------------------------------------- phase B: recurrence
+// (returns the tile's ||w||^2 and <v_j, w>, in every lane)
 template <typename R, int T>
-__device__ bool tile_orth(const BArgs &A, const BInst &I, int i, int t, int j, double car,
-                          double cai, double cb, double sj) {
+__device__ __forceinline__ double3 tile_orth_sums(const BArgs &A, const BInst &I, int t, int j, double car, double cai,
+                                                  double cb, double sj) {
     typedef typename cvec<R>::T C;
     constexpr int AMP = 1 << (T - 5);
     const int lane = threadIdx.x & 31;
@@ -469,17 +482,17 @@ __device__ bool tile_orth(const BArgs &A, const BInst &I, int i, int t, int j, d
     acc0 = warp_sum(acc0);
     acc1 = warp_sum(acc1);
     acc2 = warp_sum(acc2);
-    if (lane == 0) {
-        double *pb = A.partB + 4 * (size_t)t;
-        pb[0] = acc0;
-        pb[1] = acc1;
-        pb[2] = acc2;
-    }
+    return make_double3(acc0, acc1, acc2);
+}
+template <typename R, int T>
+__device__ bool tile_orth(const BArgs &A, const BInst &I, int i, int t, int j, double car, double cai, double cb,
+                          double sj) {
+    put_part(A.partB, t, tile_orth_sums<R, T>(A, I, t, j, car, cai, cb, sj));
     return tile_done(A.cnt + A.ninst, A.partB, A.sumB, i, I.tile0, I.ntiles);
 }
 
 template <typename R, int T>
-__device__ bool tile_norm(const BArgs &A, const BInst &I, int i, int t) {
+__device__ __forceinline__ double tile_norm_sum(const BArgs &A, const BInst &I, int t) {
     typedef typename cvec<R>::T C;
     constexpr int AMP = 1 << (T - 5);
     const int lane = threadIdx.x & 31;
@@ -488,8 +501,12 @@ __device__ bool tile_norm(const BArgs &A, const BInst &I, int i, int t) {
     double nrm = 0.0;
 #pragma unroll 8
     for (int a = 0; a < AMP; ++a) add_sq(nrm, ldcg(u + base + lane + 32 * a));
-    nrm = warp_sum(nrm);
-    if (lane == 0) A.partN[4 * (size_t)t] = nrm;
+    return warp_sum(nrm);
+}
+template <typename R, int T>
+__device__ bool tile_norm(const BArgs &A, const BInst &I, int i, int t) {
+    const double nrm = tile_norm_sum<R, T>(A, I, t);
+    if ((threadIdx.x & 31) == 0) A.partN[4 * (size_t)t] = nrm;
     return tile_done(A.cnt + 2 * A.ninst, A.partN, A.sumN, i, I.tile0, I.ntiles);
 }
 
@@ -882,16 +899,13 @@ __device__ bool job_init(const BArgs &A, int i, int gstep) {
     return __shfl_sync(0xffffffffu, st, 0) == KS_RUNNING;
 }
 
-// Combination tile of step rstep: psi' = s0 sum_k c_k v_k in place for a job whose step
-// ended with a result (optionally also into the history buffer), else (failed) the norm
-// of the kept state; the tile's norm partial.  True for the warp that completes the job.
+// Combination tile of step rstep: psi' = s0 sum_k c_k v_k in place (optionally also into the
+// history buffer); returns the tile's ||psi'||^2.
 template <typename R, int T>
-__device__ bool tile_combine(const BArgs &A, const BInst &I, int i, int t, int rstep) {
+__device__ __forceinline__ double tile_combine_sum(const BArgs &A, const BInst &I, int i, int t, int rstep) {
     typedef typename cvec<R>::T C;
     const int lane = threadIdx.x & 31;
     const KState *ks = A.ks + i;
-    const int st = ld_status(ks);
-    if (st != KS_CONVERGED && st != KS_HAPPY && st != KS_MAXDIM) return tile_norm<R, T>(A, I, i, t);
     const int nvec = __ldcg(&ks->nvec);
     double cr[4], cim[4];
     load_coefs(ks, nvec, false, cr, cim);
@@ -905,7 +919,16 @@ __device__ bool tile_combine(const BArgs &A, const BInst &I, int i, int t, int r
         __syncwarp();
         for (int a = 0; a < AMP; ++a) h[base + lane + 32 * a] = out[base + lane + 32 * a];
     }
-    if (lane == 0) A.partN[4 * (size_t)t] = nrm;
+    return nrm;
+}
+// The combination of a job whose step ended with a result, else (failed) the norm of the kept
+// state; the tile's norm partial.  True for the warp that completes the job.
+template <typename R, int T>
+__device__ bool tile_combine(const BArgs &A, const BInst &I, int i, int t, int rstep) {
+    const int st = ld_status(A.ks + i);
+    if (st != KS_CONVERGED && st != KS_HAPPY && st != KS_MAXDIM) return tile_norm<R, T>(A, I, i, t);
+    const double nrm = tile_combine_sum<R, T>(A, I, i, t, rstep);
+    if ((threadIdx.x & 31) == 0) A.partN[4 * (size_t)t] = nrm;
     return tile_done(A.cnt + 2 * A.ninst, A.partN, A.sumN, i, I.tile0, I.ntiles);
 }
 
@@ -1070,6 +1093,189 @@ __device__ void run_jobs(const BArgs &A) {
 template <typename R, int T, int MINB>
 __global__ void __launch_bounds__(BWARPS * 32, MINB) k_batch_phase(const BArgs A) {
     run_jobs<R, T>(A);
+}
+
+// ---------------------------------------------------------------- gangs
+// The phase engine where every tile of the batch has a warp of its own: a job's warps (a gang:
+// the warps of its own CTAs) go through its phases together, and what a phase waits for is one
+// exchange of the job's own tile sums -- a warp writes its tile's sums as 16-byte records
+// (value, epoch) and reads the records of the job's tiles until each carries the phase's epoch
+// -- instead of a visit that finds the job's next phase published.  The sums are added in the
+// order of inst_sum and the tiles' arithmetic is that of the other schedulers, so the results
+// are theirs to the bit.  The decisions are taken by one warp per job in CTAs of their own
+// while the gang goes on; iterations past the one that ends the step are left unused.
+// Measured: the 12 parameter sets of a 14-qubit ring took 87 us per Lanczos iteration with the
+// visits (1184 warps on 384 tiles and a handful of counters), about 21 us here.
+struct GArgs {
+    BArgs A;
+    PRec *rec;        // per job 7 records a tile (A: 3, B: 3, N: 1) at 7 tile0
+    PRec *jrec;       // per job GANG_JREC: start of a step, verdict, ||w||^2 and <v_j, w> of iteration j
+    const int *cta0;  // [njobs + 1] first CTA of each job's gang
+    int ncompute;     // CTAs of the gangs; the deciding CTAs follow
+};
+constexpr int GANG_JREC = 2 + 3 * KMAX;
+
+// Waits (lanes on their own records) until record r carries epoch e; false once the wait ran
+// out or another warp recorded an error.
+__device__ __forceinline__ bool gang_wait(const BArgs &A, const PRec *r, unsigned long long e, PRec *o) {
+    *o = rec_get<true>(r);
+    if ((o->e & ~PSTOP) == e) return true;
+    const long long t0 = clock64();
+    for (unsigned i = 1;; ++i) {
+        *o = rec_get<true>(r);
+        if ((o->e & ~PSTOP) == e) return true;
+        if ((i & 255u) == 0 && (clock64() - t0 > A.bar_limit || ld_vol(&A.ctl->err))) {
+            atomicCAS(&A.ctl->err, 0, EMUSV_TIMEOUT);
+            return false;
+        }
+    }
+}
+
+// The job's sums over its tiles of NS values a tile (inst_sum's order), from the records at
+// rec; the calling warp's own values and tile.  stop: tile 0's flag goes to every warp.
+template <int NS>
+__device__ __forceinline__ bool gang_exchange(const BArgs &A, PRec *rec, const BInst &I, int tl, unsigned long long e,
+                                              double (&v)[NS], bool stop_in, bool *stop) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    if (lane < NS) {
+        double x = v[0];
+#pragma unroll
+        for (int k = 1; k < NS; ++k)
+            if (lane == k) x = v[k];
+        __threadfence();  // the warp's stores before its records
+        rec_put(rec + lane * I.ntiles + tl, x, e | (stop_in ? PSTOP : 0ull));
+    }
+    bool ok = true, fin = false;
+#pragma unroll
+    for (int k = 0; k < NS; ++k) v[k] = 0.0;
+    for (int t = lane; t < I.ntiles && ok; t += 32) {
+#pragma unroll
+        for (int k = 0; k < NS; ++k) {
+            PRec o;
+            ok = gang_wait(A, rec + k * I.ntiles + t, e, &o) && ok;
+            v[k] += o.v;
+            if (k == 0 && t == 0) fin = (o.e & PSTOP) != 0;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NS; ++k) v[k] = warp_sum(v[k]);
+    *stop = __shfl_sync(0xffffffffu, (int)fin, 0) != 0;
+    return __all_sync(0xffffffffu, ok);
+}
+
+// The deciding warp of job i.
+__device__ void gang_decider(const GArgs &B, int i) {
+    const BArgs &A = B.A;
+    const int lane = threadIdx.x & 31;
+    PRec *jr = B.jrec + (size_t)GANG_JREC * i, o;
+    for (int rstep = 0; rstep < A.run_steps; ++rstep) {
+        const unsigned long long e = 1 + (unsigned long long)rstep;  // the step's epoch
+        if (A.first_step + rstep >= A.inst[i].nsteps) break;         // no step left
+        if (!__all_sync(0xffffffffu, gang_wait(A, jr, e, &o))) return;
+        bool more = job_init(A, i, A.first_step + rstep);
+        for (int j = 0; more; ++j) {
+            o.v = 0.0;
+            const bool got = lane >= 3 || gang_wait(A, jr + 2 + 3 * j + lane, e, &o);
+            if (!__all_sync(0xffffffffu, got)) return;
+            if (lane < 3) A.sumB[4 * (size_t)i + lane] = o.v;
+            __threadfence();
+            __syncwarp();
+            more = job_decide(A, i, j, rstep);
+        }
+        const int st = ld_status(A.ks + i);
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) rec_put(jr + 1, (double)st, e);
+        if (!A.combine || (st != KS_CONVERGED && st != KS_HAPPY && st != KS_MAXDIM)) break;
+    }
+}
+
+template <typename R, int T, int MINB>
+__global__ void __launch_bounds__(BWARPS * 32, MINB) k_batch_gang(const __grid_constant__ GArgs B) {
+    const BArgs &A = B.A;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if ((int)blockIdx.x >= B.ncompute) {
+        const int i = ((int)blockIdx.x - B.ncompute) * BWARPS + warp;
+        if (i < A.ninst) gang_decider(B, i);
+        return;
+    }
+    int lo = 0, hi = A.ninst - 1;  // the job of this CTA
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (__ldg(&B.cta0[mid]) <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
+    }
+    const int i = lo, tl = ((int)blockIdx.x - __ldg(&B.cta0[i])) * BWARPS + warp;
+    const BInst I = A.inst[i];
+    if (tl >= I.ntiles) return;
+    const int t = I.tile0 + tl;
+    const bool lead = tl == 0 && lane == 0;
+    KState *ks = A.ks + i;
+    PRec *ra = B.rec + 7 * (size_t)I.tile0, *rb = ra + 3 * I.ntiles, *rn = ra + 6 * I.ntiles;
+    PRec *jr = B.jrec + (size_t)GANG_JREC * i;
+    unsigned long long ea = 0, eb = 0, en = 0;  // epochs of the three kinds of exchange
+    bool stop = false;
+    int last = BS_IDLE;
+    // failure-path test switch: one sum of job 0 never arrives, its gang's waits run out
+    if (A.test_skip_arrival && i == 0 && tl == 0) return;
+    double nv[1] = {tile_norm_sum<R, T>(A, I, t)};
+    if (!gang_exchange<1>(A, rn, I, tl, ++en, nv, false, &stop)) return;
+    const int limit = A.maxdim < A.capacity ? A.maxdim : A.capacity;
+    for (int rstep = 0; rstep < A.run_steps; ++rstep) {
+        const int gstep = A.first_step + rstep;
+        if (gstep >= I.nsteps) {
+            last = BS_IDLE;
+            break;
+        }
+        const unsigned long long e = 1 + (unsigned long long)rstep;  // the step's epoch
+        if (lead) {
+            A.sumN[4 * (size_t)i] = nv[0];
+            __threadfence();
+            rec_put(jr, 0.0, e);
+        }
+        const double s0 = sqrt(nv[0]);
+        double sn = nv[0], scale = 1.0 / s0, sp = 0.0, b = 0.0, vr = 0.0, vi = 0.0;
+        const bool fine = isfinite(s0) && s0 > 0.0;  // else the decision is KS_NONFINITE
+        for (int j = 0; fine && j < limit; ++j) {
+            // A: H v_j
+            double sj = 1.0 / sqrt(sn);
+            if (!isfinite(sj) || sj <= 0.0) sj = 0.0;
+            const double3 pa = tile_hpsi_sums<R, T>(A, I, t, gstep, j, sj);
+            double a[3] = {pa.x, pa.y, pa.z};
+            if (!gang_exchange<3>(A, ra, I, tl, ++ea, a, false, &stop)) return;
+            // B: w = H v_j - a v_j - b v_{j-1}
+            const double ar = a[1] - b * vr, ai = a[2] - b * vi;
+            if (lead) {  // T_H's column j (read by the decision)
+                ks->a_re[j] = ar;
+                ks->a_im[j] = ai;
+                ks->b_re[j] = b;
+                ks->b_im[j] = 0.0;
+                ks->hn[j] = sqrt(a[0]);
+            }
+            const double3 pb = tile_orth_sums<R, T>(A, I, t, j, ar * scale, ai * scale, b * sp, scale);
+            double w[3] = {pb.x, pb.y, pb.z};
+            if (!gang_exchange<3>(A, rb, I, tl, ++eb, w, lead && rec_get(jr + 1).e == e, &stop)) return;
+            if (tl == 0 && lane < 3) rec_put(jr + 2 + 3 * j + lane, lane == 0 ? w[0] : lane == 1 ? w[1] : w[2], e);
+            if (stop) break;
+            const double r = sqrt(w[0]);  // as krylov_norms
+            sn = w[0];
+            sp = scale;
+            scale = 1.0 / r;
+            b = r;
+            vr = w[1] / r;
+            vi = -w[2] / r;
+        }
+        PRec o;
+        if (!__all_sync(0xffffffffu, gang_wait(A, jr + 1, e, &o))) return;
+        last = (int)o.v;
+        if (!A.combine || (last != KS_CONVERGED && last != KS_HAPPY && last != KS_MAXDIM)) break;
+        nv[0] = tile_combine_sum<R, T>(A, I, i, t, rstep);
+        if (!gang_exchange<1>(A, rn, I, tl, ++en, nv, false, &stop)) return;
+    }
+    if (lead) {
+        const int f = ld_vol(&A.fail[i]);
+        A.status_out[i] = f ? f : (last == BS_IDLE ? KS_CONVERGED : last);
+    }
 }
 
 // ---------------------------------------------------------------- adjoint kernel
@@ -1374,7 +1580,7 @@ static size_t al256(size_t v) { return (v + 255) / 256 * 256; }
 // Workspace layout.  Forward: one job per instance.  Adjoint: jobs 2i (state) and 2i+1
 // (gradient) per instance, plus the adjoint's own arrays.
 struct BLayout {
-    size_t args, ctl, ints, inst, coef, ubits, elow, ks, sums, iters, partA, partB, partN, slots;
+    size_t args, ctl, ints, rec, cta0, inst, coef, ubits, elow, ks, sums, iters, partA, partB, partN, slots;
     size_t dS, escr, E, partC, total;
     int njobs, total_tiles, coef_count, max_steps, mmax, escr_warps;
     long long inst_amps, slot_amps;
@@ -1412,6 +1618,8 @@ static bool layout(int ninst, const int *nq, const int *nsteps, int es, int T, i
     L->ints = off;
     off += sizeof(int) * (12 * (size_t)nj + ninst);
     off = al256(off);
+    L->rec = take(sizeof(PRec) * (7 * (size_t)L->total_tiles + (size_t)GANG_JREC * nj));
+    L->cta0 = take(sizeof(int) * (nj + 1));
     L->inst = take(sizeof(BInst) * nj);
     L->coef = take(sizeof(BCoef) * (coefs > 0 ? coefs : 1));
     L->ubits = take(sizeof(double) * BMAXQ * BMAXQ * ninst);
@@ -1442,12 +1650,13 @@ struct Shape {
 };
 
 // kind 0: forward (lock-step rounds); 1: adjoint rounds; 2: adjoint post-processing;
-// 3: forward (phase engine)
+// 3: forward (phase engine); 4: gangs (forward and the adjoint's bases)
 static void *pick_kernel(int dtype, int T, int kind) {
 #define EMUSV_K(R, TT)                                                                   \
     (kind == 1   ? reinterpret_cast<void *>(k_batch_adj_rounds<R, TT, Shape<R, TT>::MINB>) \
      : kind == 2 ? reinterpret_cast<void *>(k_batch_adj_post<R, TT, Shape<R, TT>::MINB>)   \
      : kind == 3 ? reinterpret_cast<void *>(k_batch_phase<R, TT, Shape<R, TT>::MINB>)      \
+     : kind == 4 ? reinterpret_cast<void *>(k_batch_gang<R, TT, Shape<R, TT>::MINB>)       \
                  : reinterpret_cast<void *>(k_batch<R, TT, Shape<R, TT>::MINB>))
     if (dtype == EMUSV_C64) {
         if (T == 8) return EMUSV_K(float, 8);
@@ -1483,6 +1692,7 @@ struct Prepared {
     BLayout L;
     bool adjoint;
     int engine;  // forward launches: 0 lock-step rounds, 1 phase engine
+    int gang;    // CTAs of the gangs (phase engine and adjoint), 0: more tiles than warps
 };
 static std::mutex g_args_mu;
 static std::unordered_map<const void *, Prepared> g_args;
@@ -1501,7 +1711,7 @@ static int prepare_common(int ninst, const int *nqubits, const int *nsteps, cons
         if (!isfinite(dt[i])) return EMUSV_BAD_ARGUMENT;
     // the shared-memory limits of the kernels the launches may use (host calls, so that a
     // launch recorded into a CUDA graph issues none)
-    for (int kind : {0, 1, 3}) {
+    for (int kind : {0, 1, 3, 4}) {
         const int st = configure_smem(pick_kernel(dtype, T, kind), kernel_smem(dtype, T, kind));
         if (st) return st;
     }
@@ -1641,6 +1851,14 @@ static int prepare_common(int ninst, const int *nqubits, const int *nsteps, cons
         D.partC = reinterpret_cast<double *>(ws + L.partC);
         D.cntC = reinterpret_cast<unsigned *>(ints + 12 * nj);
     }
+    std::vector<int> cta0(nj + 1);
+    for (int J = 0; J < nj; ++J) cta0[J + 1] = cta0[J] + (inst[J].ntiles + BWARPS - 1) / BWARPS;
+    int per_sm = 0;
+    EMUSV_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick_kernel(dtype, T, 4), BWARPS * 32,
+                                                              kernel_smem(dtype, T, 4)));
+    const int deciding = (nj + BWARPS - 1) / BWARPS;
+    P.gang = cta0[nj] + deciding <= per_sm * sm_count() ? cta0[nj] : 0;
+    EMUSV_CHECK(cudaMemcpyAsync(ws + L.cta0, cta0.data(), sizeof(int) * (nj + 1), cudaMemcpyHostToDevice, s));
     EMUSV_CHECK(cudaMemcpyAsync(ws + L.args, &A, sizeof(A), cudaMemcpyHostToDevice, s));
     EMUSV_CHECK(cudaMemcpyAsync(ws + L.inst, inst.data(), sizeof(BInst) * nj, cudaMemcpyHostToDevice, s));
     EMUSV_CHECK(cudaMemcpyAsync(ws + L.coef, coef.data(), sizeof(BCoef) * coef.size(), cudaMemcpyHostToDevice, s));
@@ -1663,14 +1881,16 @@ static int lookup(const void *workspace, bool adjoint, Prepared *out) {
     return EMUSV_OK;
 }
 
+// blocks: the exact grid (it fits), or 0: blocks_per_sm CTAs per SM.
 static int cooperative_launch(void *kern, int blocks_per_sm, void **args, cudaStream_t s,
-                              int *grid_out, int prof_kind = PROF_BATCH, size_t smem = 0) {
-    int per_sm = 0;
-    EMUSV_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BWARPS * 32, smem));
-    if (per_sm < 1) return EMUSV_CUDA_ERROR;
-    const int bps = blocks_per_sm < per_sm ? blocks_per_sm : per_sm;
-    const int grid = bps * sm_count();
-    if (grid_out) *grid_out = grid;
+                              int blocks, int prof_kind = PROF_BATCH, size_t smem = 0) {
+    int grid = blocks;
+    if (!grid) {
+        int per_sm = 0;
+        EMUSV_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BWARPS * 32, smem));
+        if (per_sm < 1) return EMUSV_CUDA_ERROR;
+        grid = (blocks_per_sm < per_sm ? blocks_per_sm : per_sm) * sm_count();
+    }
     ProfScope ps_(prof_kind, s);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
@@ -1684,6 +1904,21 @@ static int cooperative_launch(void *kern, int blocks_per_sm, void **args, cudaSt
     cfg.numAttrs = 1;
     EMUSV_CHECK(cudaLaunchKernelExC(&cfg, kern, args));
     return EMUSV_OK;
+}
+
+// The gangs of a prepared workspace (P.gang > 0); A: the launch's arguments.
+static int gang_launch(int dtype, const Prepared &P, const BArgs &A, unsigned char *ws, cudaStream_t s) {
+    GArgs G;
+    G.A = A;
+    G.rec = reinterpret_cast<PRec *>(ws + P.L.rec);
+    G.jrec = G.rec + 7 * (size_t)A.total_tiles;
+    G.cta0 = reinterpret_cast<const int *>(ws + P.L.cta0);
+    G.ncompute = P.gang;
+    // no record of an earlier launch carries this one's epochs
+    EMUSV_CHECK(cudaMemsetAsync(G.rec, 0, sizeof(PRec) * (7 * (size_t)A.total_tiles + (size_t)GANG_JREC * A.ninst), s));
+    void *args[] = {(void *)&G};
+    return cooperative_launch(pick_kernel(dtype, A.T, 4), 1, args, s, P.gang + (A.ninst + BWARPS - 1) / BWARPS,
+                              PROF_BATCH, kernel_smem(dtype, A.T, 4));
 }
 
 }  // namespace emusv
@@ -1741,8 +1976,9 @@ int emusv_batch_launch_steps(int dtype, int tile_bits, int blocks_per_sm, int fi
     unsigned char *ws = reinterpret_cast<unsigned char *>(workspace);
     // control block, flags, hints and tile counters start at zero
     EMUSV_CHECK(cudaMemsetAsync(ws + P.L.ctl, 0, sizeof(BCtl) + sizeof(int) * 12 * (size_t)A.ninst, s));
+    if (P.engine && P.gang) return gang_launch(dtype, P, A, ws, s);
     void *args[] = {(void *)&A};
-    return cooperative_launch(kern, blocks_per_sm, args, s, nullptr, PROF_BATCH,
+    return cooperative_launch(kern, blocks_per_sm, args, s, 0, PROF_BATCH,
                               kernel_smem(dtype, tile_bits, kind));
 }
 
@@ -1861,8 +2097,9 @@ int emusv_batch_adjoint_launch(int dtype, int tile_bits, int blocks_per_sm, int 
     EMUSV_CHECK(cudaMemsetAsync(ws + P.L.ctl, 0, sizeof(BCtl) + sizeof(int) * 4 * (size_t)nj, s));
     EMUSV_CHECK(cudaMemsetAsync(A.fail, 0, sizeof(int) * (6 * (size_t)nj + D.ninst), s));
     void *args[] = {(void *)&A, (void *)&D};
-    int st = cooperative_launch(k1, blocks_per_sm, args, s, nullptr, PROF_BATCH,
-                                kernel_smem(dtype, tile_bits, 1));
+    const int st = P.gang ? gang_launch(dtype, P, A, ws, s)
+                          : cooperative_launch(k1, blocks_per_sm, args, s, 0, PROF_BATCH,
+                                               kernel_smem(dtype, tile_bits, 1));
     if (st) return st;
     {
         ProfScope ps_(PROF_ADJOINT, s);
@@ -1871,7 +2108,7 @@ int emusv_batch_adjoint_launch(int dtype, int tile_bits, int blocks_per_sm, int 
     }
     EMUSV_CHECK_LAUNCH();
     EMUSV_CHECK(cudaMemsetAsync(ws + P.L.ctl, 0, sizeof(BCtl), s));
-    return cooperative_launch(k3, blocks_per_sm, args, s, nullptr, PROF_ADJOINT);
+    return cooperative_launch(k3, blocks_per_sm, args, s, 0, PROF_ADJOINT);
 }
 
 // Failure-path test switch of a prepared workspace (forward or adjoint): later launches

@@ -338,7 +338,8 @@ int emusv_batch_adjoint_iterations(int ninst, void *workspace, int *iterations_o
 /* Scheduling of a prepared forward batch workspace (no counterpart in the reference):
  * engine 0 (the default) runs every register's Lanczos iterations in lock-step rounds of
  * the whole batch, engine 1 lets each register run its own sequence of phases (norm,
- * H v, recurrence, ..., combination) with no grid barrier.  Results are the same; the
+ * H v, recurrence, ..., combination) with no grid barrier (a batch whose tiles all have a
+ * warp of their own: every register by its own gang of warps).  Results are the same; the
  * faster one depends on the batch (BatchEvolution's autotuner times both).  Host-side
  * only (takes effect at the next launch); EMUSV_BAD_ARGUMENT for an adjoint workspace. */
 int emusv_batch_set_engine(void *workspace, int engine);
