@@ -151,20 +151,27 @@ k_lindblad_jumps(const LindbladJumps J, const void *u_, const double *su_p, void
             di += cnt[e] * J.K[2 * 5 * e + 1];
         }
         double ar = dr * double(ux.x) - di * double(ux.y), ai = dr * double(ux.y) + di * double(ux.x);
-        if (off) {
-            for (int pc = 0; pc < n; ++pc) {
-                const int ij = (int)((row >> pc) & 1u) * 2 + (int)((col >> pc) & 1u);
+        // the other entries: per entry, the qubits of x with its (i, j), two partners at a time
+        // (a loop over the qubits that tested every entry took 22 us at n = 10, this 11.6)
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const int e = ij * 4 + t;
-                    if (!((off >> e) & 1)) continue;
-                    const i64 bits = (i64)(((ij ^ t) >> 1) & 1) << (pc + n) | (i64)((ij ^ t) & 1) << pc;
-                    const C v = u[x ^ bits];
-                    const double kr = J.K[2 * e], ki = J.K[2 * e + 1];
-                    ar += kr * double(v.x) - ki * double(v.y);
-                    ai += kr * double(v.y) + ki * double(v.x);
-                }
+        for (int e = 0; e < 16; ++e) {
+            if (!((off >> e) & 1)) continue;
+            const int ij = e >> 2, fl = (e >> 2) ^ (e & 3);
+            unsigned m = (ij & 2 ? row : ~row) & (ij & 1 ? col : ~col) & low;
+            double sr = 0.0, si = 0.0;
+            auto partner = [&](int p) { return u[x ^ ((i64)(fl >> 1) << (p + n)) ^ ((i64)(fl & 1) << p)]; };
+            while (m) {
+                const int p0 = __ffs(m) - 1;
+                m &= m - 1;
+                const int p1 = __ffs(m) - 1;  // -1: none left
+                m &= m - 1;
+                const C a = partner(p0), b = p1 >= 0 ? partner(p1) : cmake<C>(0.0, 0.0);
+                sr += double(a.x) + double(b.x);
+                si += double(a.y) + double(b.y);
             }
+            const double kr = J.K[2 * e], ki = J.K[2 * e + 1];
+            ar += kr * sr - ki * si;
+            ai += kr * si + ki * sr;
         }
         const C o = out[x];
         // + i su (ar + i ai) = su (-ai + i ar)
