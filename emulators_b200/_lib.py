@@ -181,6 +181,11 @@ def host_f64(t, n: int | None = None, name: str = "parameter") -> np.ndarray:
     as the pulser adapter passes real values in complex128 tensors)."""
     if isinstance(t, torch.Tensor):
         t = t.detach()
+        if t.dtype is torch.float64 and t.device.type == "cpu" and t.is_contiguous():
+            a = t.numpy()  # the adapter's samples: no conversion, no copy
+            if n is not None and a.size != n:
+                raise ValueError(f"{name}: expected {n} values, got {a.size}")
+            return a
         if t.is_complex():
             t = t.real
         a = t.to("cpu", torch.float64).contiguous().numpy()
@@ -201,7 +206,8 @@ def ptr(a) -> int:
 
 
 def stream_of(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    """The handle of the device's current stream (without a Stream object per call)."""
+    return torch._C._cuda_getCurrentRawStream(t.device.index)
 
 
 _scratch: dict = {}

@@ -172,7 +172,10 @@ class Statistics(Observable):
     def apply(self, *, config, state, hamiltonian):
         duration = self.durations[-1]
         if state.data.is_cuda:
-            mem = max(torch.cuda.max_memory_allocated(d) * 1e-6 for d in range(torch.cuda.device_count()))
+            # torch.cuda.max_memory_allocated without flattening every other statistic (0.1 ms
+            # a step, as much as the step itself on a small register)
+            mem = max(torch.cuda.memory_stats_as_nested_dict(d)["allocated_bytes"]["all"]["peak"] * 1e-6
+                      for d in range(torch.cuda.device_count()))
         else:  # pragma: no cover - the package keeps its states on the GPU
             import resource
 
