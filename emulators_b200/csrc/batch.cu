@@ -134,10 +134,9 @@ struct BAdj {
     double2 *dS;            // [ninst][mmax*mmax]: dS[r][k] at r*mmax + k
     unsigned char *E;       // E_k of every instance: [mmax][inst_amps]
     long long inst_amps;
-    double *partC;          // [total job tiles][NCP] contraction partials
+    double *partC;          // contraction partials, rows of NCP (post_row)
     double *grads;          // [ninst][3][BMAXQ] dL/dOmega, dL/ddelta, dL/dphi by qubit
     void *gout;             // packed state gradient exp(+i dt H) g
-    unsigned *cntC;         // [ninst]
     int *astatus;           // [ninst] emusv status of the instance's adjoint
 };
 constexpr int NCP = 6 * BMAXQ;  // per bit: T_re, T_im, U_re, U_im, S_re, S_im
@@ -1341,237 +1340,382 @@ __global__ void __launch_bounds__(BWARPS * 32, MINB) k_batch_adj_rounds(const BA
     run_jobs<R, T>(A);
 }
 
-template <typename R, int T, int MINB>
-__global__ void __launch_bounds__(BWARPS * 32, MINB) k_batch_adj_post(const BArgs A, const BAdj D) {
+// ---------------------------------------------------------------- adjoint post-processing
+// E_k = sum_r dS[r][k] v^s_r for k < mg: a complex matrix product of FP64 operations (8 ms mg an
+// amplitude).  A thread owns PE_X amplitudes and PE_K outputs, so a loaded amplitude feeds PE_K
+// products and a coefficient from shared memory PE_X of them; blocks in y take the groups of
+// outputs, which read the basis again from the L2.  (12 registers of 14 qubits, 45 outputs of 20
+// vectors: 146 us with two blocks an SM, 236 with one; as warps on tiles of 2^9 amplitudes, with
+// the contraction in the same kernel, 384 warps on the whole GPU and 1340 us.)
+constexpr int PE_K = 8, PE_X = 2, PE_T = 256;
+template <typename R>
+__global__ void __launch_bounds__(PE_T, 2) k_post_E(const BArgs A, const BAdj D) {
     typedef typename cvec<R>::T C;
-    constexpr int AMP = 1 << (T - 5);
-    const int lane = threadIdx.x & 31;
-    unsigned ph = 0;
-
-    // ---------------- E_k = sum_r dS[r][k] v^s_r (state tiles); g_out (gradient tiles)
-    for (int t = next_tile(A.ctl, ph); t < A.total_tiles; t = next_tile(A.ctl, ph)) {
-        const int J = inst_of_tile(A, t), i = J >> 1;
-        const KState *kss = A.ks + 2 * i, *ksg = A.ks + 2 * i + 1;
-        const BInst I = A.inst[J];
-        const long long base = (long long)(t - I.tile0) << T;
-        if (!job_ok(kss) || !job_ok(ksg)) {
-            if ((J & 1) && __ldcg(&ksg->s0) == 0.0) {  // exp(+i dt H) 0 = 0
-                C *o = reinterpret_cast<C *>(D.gout) + I.off0 + base + lane;
-                for (int a = 0; a < AMP; ++a) o[32 * a] = cmake<C>(0.0, 0.0);
-            }
-            continue;
-        }
-        const int ms = basis_size(kss), mg = basis_size(ksg);
-        if (J & 1) {  // state gradient from the gradient basis
-            double cr[4], cim[4];
-            const int nvec = __ldcg(&ksg->nvec);
-            load_coefs(ksg, nvec, true, cr, cim);
-            tile_lincomb<R, T>(A, I, t, nvec, cr, cim, reinterpret_cast<C *>(D.gout) + I.off0);
-            continue;
-        }
-        const double2 *dS = D.dS + (size_t)i * D.mmax * D.mmax;
-        // KC outputs per pass over the state basis: every loaded amplitude feeds KC MACs
-        constexpr int KC = 16;
-        for (int k0 = 0; k0 < mg; k0 += KC) {
-            const int kn = mg - k0 < KC ? mg - k0 : KC;
-            for (int a = 0; a < AMP; ++a) {
-                double er[KC], ei[KC];
+    __shared__ double2 cf[KMAX][PE_K];
+    const int i = blockIdx.z, k0 = blockIdx.y * PE_K;
+    const KState *kss = A.ks + 2 * i, *ksg = kss + 1;
+    if (!job_ok(kss) || !job_ok(ksg)) return;
+    const int ms = basis_size(kss), mg = basis_size(ksg);
+    const BInst I = A.inst[2 * i];
+    const long long x0 = (long long)blockIdx.x * PE_T * PE_X + threadIdx.x, len = 1LL << I.n;
+    if (k0 >= mg || (long long)blockIdx.x * PE_T * PE_X >= len) return;
+    const double2 *dS = D.dS + (size_t)i * D.mmax * D.mmax;
+    for (int e = threadIdx.x; e < ms * PE_K; e += PE_T) {
+        const int r = e / PE_K, kk = e % PE_K;
+        const double sc = kss->scale[r];
+        const double2 d = k0 + kk < mg ? dS[(size_t)r * D.mmax + k0 + kk] : make_double2(0.0, 0.0);
+        cf[r][kk] = make_double2(sc * d.x, sc * d.y);
+    }
+    __syncthreads();
+    double er[PE_X][PE_K], ei[PE_X][PE_K];
 #pragma unroll
-                for (int kk = 0; kk < KC; ++kk) er[kk] = ei[kk] = 0.0;
-                const long long x = base + lane + 32 * a;
+    for (int a = 0; a < PE_X; ++a)
+#pragma unroll
+        for (int kk = 0; kk < PE_K; ++kk) er[a][kk] = ei[a][kk] = 0.0;
 #pragma unroll 4
-                for (int r = 0; r < ms; ++r) {
-                    const double sc = __ldcg(&kss->scale[r]);
-                    const C v = ldcg(vec_ptr<C>(A, r, I) + x);
-                    const double vx = sc * double(v.x), vy = sc * double(v.y);
-                    const double2 *drow = dS + (size_t)r * D.mmax + k0;
+    for (int r = 0; r < ms; ++r) {
+        const C *v = vec_ptr<C>(A, r, I);
+        double vx[PE_X], vy[PE_X];
 #pragma unroll
-                    for (int kk = 0; kk < KC; ++kk) {
-                        if (kk < kn) {
-                            const double2 d = drow[kk];
-                            er[kk] += d.x * vx - d.y * vy;
-                            ei[kk] += d.x * vy + d.y * vx;
-                        }
-                    }
-                }
+        for (int a = 0; a < PE_X; ++a) {
+            const long long x = x0 + a * PE_T;
+            const C q = x < len ? ldcg(v + x) : cmake<C>(0.0, 0.0);
+            vx[a] = double(q.x);
+            vy[a] = double(q.y);
+        }
 #pragma unroll
-                for (int kk = 0; kk < KC; ++kk) {
-                    if (kk < kn) {
-                        C *Ek = reinterpret_cast<C *>(D.E + (size_t)(k0 + kk) * D.inst_amps * sizeof(C)) + I.off0;
-                        Ek[x] = cmake<C>(er[kk], ei[kk]);
-                    }
-                }
+        for (int kk = 0; kk < PE_K; ++kk) {
+            const double2 d = cf[r][kk];
+#pragma unroll
+            for (int a = 0; a < PE_X; ++a) {
+                er[a][kk] = fma(d.x, vx[a], fma(-d.y, vy[a], er[a][kk]));
+                ei[a][kk] = fma(d.x, vy[a], fma(d.y, vx[a], ei[a][kk]));
             }
         }
     }
-    if (!grid_sync(A, ph)) return;
+#pragma unroll
+    for (int kk = 0; kk < PE_K; ++kk) {
+        if (k0 + kk >= mg) break;
+        C *Ek = reinterpret_cast<C *>(D.E + (size_t)(k0 + kk) * D.inst_amps * sizeof(C)) + I.off0;
+#pragma unroll
+        for (int a = 0; a < PE_X; ++a)
+            if (x0 + a * PE_T < len) Ek[x0 + a * PE_T] = cmake<C>(er[a][kk], ei[a][kk]);
+    }
+}
 
-    // ---------------- contractions over state tiles; the last tile of an instance turns
-    // its sums into the step's gradients (torch.py:324-353)
-    for (int t = next_tile(A.ctl, ph); t < A.total_tiles; t = next_tile(A.ctl, ph)) {
-        const int J = inst_of_tile(A, t), i = J >> 1;
-        if (J & 1) continue;
-        const KState *kss = A.ks + 2 * i, *ksg = A.ks + 2 * i + 1;
-        const BInst I = A.inst[J], IG = A.inst[J + 1];
-        const int n = I.n;
-        const long long base = (long long)(t - I.tile0) << T;
-        double acc[6] = {0, 0, 0, 0, 0, 0};  // lane p: T, U, S sums of bit p
-        const bool ok = job_ok(kss) && job_ok(ksg);
-        if (ok) {
-            const int mg = basis_size(ksg);
-            double rr[AMP], ri[AMP];
-#pragma unroll
-            for (int a = 0; a < AMP; ++a) rr[a] = ri[a] = 0.0;
-            for (int k = 0; k < mg; ++k) {
-                const double gs = __ldcg(&ksg->scale[k]);
-                const C *gk = vec_ptr<C>(A, k, IG) + base + lane;
-                const C *Ek = reinterpret_cast<const C *>(D.E + (size_t)k * D.inst_amps * sizeof(C)) + I.off0;
-                double gr[AMP], gi[AMP];
-                C e[AMP];
-#pragma unroll
-                for (int a = 0; a < AMP; ++a) {
-                    const C g = ldcg(gk + 32 * a);
-                    gr[a] = gs * double(g.x);
-                    gi[a] = -gs * double(g.y);  // conj
-                    e[a] = ldcg(Ek + base + lane + 32 * a);
-                    rr[a] += gr[a] * double(e[a].x) - gi[a] * double(e[a].y);
-                    ri[a] += gr[a] * double(e[a].y) + gi[a] * double(e[a].x);
-                }
-                // per bit p: sum conj(G) E(x^p) and its part with x_p = 1; the partner is
-                // in another lane (p < 5), another register (p < T, compile-time index so
-                // e[] stays in registers) or another tile (p >= T)
-                auto bit_sums = [&](int p, double tr, double ti, double ur, double ui) {
-                    tr = warp_sum(tr);
-                    ti = warp_sum(ti);
-                    ur = warp_sum(ur);
-                    ui = warp_sum(ui);
-                    if (lane == p) {
-                        acc[0] += tr;
-                        acc[1] += ti;
-                        acc[2] += ur;
-                        acc[3] += ui;
-                    }
-                };
-                auto term = [&](int a, const C &w, bool bit, double &tr, double &ti, double &ur,
-                                double &ui) {
-                    const double pr = gr[a] * double(w.x) - gi[a] * double(w.y);
-                    const double pi = gr[a] * double(w.y) + gi[a] * double(w.x);
-                    tr += pr;
-                    ti += pi;
-                    if (bit) {
-                        ur += pr;
-                        ui += pi;
-                    }
-                };
-                if constexpr (AMP <= 16 && MINB == 1) {  // unrolled: e[] stays in registers
-#pragma unroll
-                    for (int p = 0; p < 5; ++p) {
-                        double tr = 0, ti = 0, ur = 0, ui = 0;
-#pragma unroll
-                        for (int a = 0; a < AMP; ++a)
-                            term(a, shfl_c(e[a], 1 << p), (lane >> p) & 1, tr, ti, ur, ui);
-                        bit_sums(p, tr, ti, ur, ui);
-                    }
-#pragma unroll
-                    for (int p = 5; p < T; ++p) {
-                        double tr = 0, ti = 0, ur = 0, ui = 0;
-#pragma unroll
-                        for (int a = 0; a < AMP; ++a)
-                            term(a, e[a ^ (1 << (p - 5))], (a >> (p - 5)) & 1, tr, ti, ur, ui);
-                        bit_sums(p, tr, ti, ur, ui);
-                    }
-                } else {  // the unrolled form would not fit the register budget
-                    for (int p = 0; p < T; ++p) {
-                        double tr = 0, ti = 0, ur = 0, ui = 0;
-#pragma unroll
-                        for (int a = 0; a < AMP; ++a) {
-                            if (p < 5) term(a, shfl_c(e[a], 1 << p), (lane >> p) & 1, tr, ti, ur, ui);
-                            else term(a, e[a ^ (1 << (p - 5))], (a >> (p - 5)) & 1, tr, ti, ur, ui);
-                        }
-                        bit_sums(p, tr, ti, ur, ui);
-                    }
-                }
-                for (int p = T; p < n; ++p) {
-                    double tr = 0, ti = 0, ur = 0, ui = 0;
-                    const bool bit = (base >> p) & 1;
-#pragma unroll
-                    for (int a = 0; a < AMP; ++a)
-                        term(a, ldcg(Ek + (base ^ (1LL << p)) + lane + 32 * a), bit, tr, ti, ur, ui);
-                    bit_sums(p, tr, ti, ur, ui);
-                }
-            }
-            for (int p = 0; p < n; ++p) {  // S_pp = sum over x with bit p of rho(x)
-                double sr = 0, si = 0;
-#pragma unroll
-                for (int a = 0; a < AMP; ++a) {
-                    const long long x = base + lane + 32 * a;
-                    if ((x >> p) & 1) {
-                        sr += rr[a];
-                        si += ri[a];
-                    }
-                }
-                sr = warp_sum(sr);
-                si = warp_sum(si);
-                if (lane == p) {
-                    acc[4] += sr;
-                    acc[5] += si;
-                }
-            }
-        }
-        double *pc = D.partC + (size_t)t * NCP;
-        if (lane < n)
-#pragma unroll
-            for (int c = 0; c < 6; ++c) pc[6 * lane + c] = acc[c];
-        // count the tile; the instance's last tile finalises
-        unsigned old = 0;
-        if (lane == 0) {
-            __threadfence();
-            old = atomicAdd(&D.cntC[i], 1u);
-        }
-        old = __shfl_sync(0xffffffffu, old, 0);
-        if (old != (unsigned)I.ntiles - 1) continue;
-        __threadfence();
-        if (lane == 0) D.cntC[i] = 0;
-        double *g = D.grads + (size_t)i * 3 * BMAXQ;
-        if (!ok) {  // a zero gradient (or a failed basis): no parameter gradient
-            const bool zero = __ldcg(&ksg->s0) == 0.0;
-            if (lane < n) g[lane] = g[BMAXQ + lane] = g[2 * BMAXQ + lane] = 0.0;
-            if (lane == 0) {
-                int e = EMUSV_OK;
-                if (!zero) {
-                    e = EMUSV_NONFINITE;
-                    for (const KState *k2 : {kss, ksg}) {
-                        const int st = ld_status(k2);
-                        if (st == KS_MAXDIM) e = EMUSV_NOT_CONVERGED;  // double_krylov.py:107-110
-                        if (st == BS_CAPACITY) e = EMUSV_WORKSPACE_TOO_SMALL;
-                    }
-                }
-                D.astatus[i] = e;
-            }
-            continue;
-        }
-        double sum[6] = {0, 0, 0, 0, 0, 0};  // lane p: instance sums of bit p
-        if (lane < n)
-            for (int tt = 0; tt < I.ntiles; ++tt)
-#pragma unroll
-                for (int c = 0; c < 6; ++c) sum[c] += __ldcg(D.partC + (size_t)(I.tile0 + tt) * NCP + 6 * lane + c);
-        if (lane < n) {
-            const int p = lane, q = n - 1 - p;  // bit p is qubit q
-            const BCoef &cf = A.coef[I.coef0 + D.step];
-            const double dt = I.dt, c = __ldcg(&kss->s0) * __ldcg(&ksg->s0);
-            const double Ure = sum[2], Uim = sum[3], Dre = sum[0] - sum[2], Dim = sum[1] - sum[3];
-            // Re(-i dt c <.>) for a flip with coefficient a on |1><0| and conj(a) on |0><1|
-            auto flip = [&](double ar, double ai) {
-                const double im = ar * Uim + ai * Ure + ar * Dim - ai * Dre;
-                return dt * c * im;
-            };
-            const double om = cf.om[p], phv = cf.ph[p];
-            g[q] = flip(0.5 * cos(phv), 0.5 * sin(phv));                     // DHDOmegaSparse
-            g[BMAXQ + q] = dt * c * (-sum[5]);                              // DHDDeltaSparse: -n
-            g[2 * BMAXQ + q] = flip(-0.5 * om * sin(phv), 0.5 * om * cos(phv));  // DHDPhiSparse
-        }
-        if (lane == 0) D.astatus[i] = EMUSV_OK;
+// g_out = exp(+i dt H) g from the gradient's own basis: the sums of tile_lincomb, a thread per
+// amplitude: 38 us at 12 registers of 14 qubits, 206 with a warp per tile.
+template <typename R>
+__global__ void __launch_bounds__(PE_T) k_post_gout(const BArgs A, const BAdj D) {
+    typedef typename cvec<R>::T C;
+    __shared__ double2 cf[KMAX + 2];
+    const int i = blockIdx.y;
+    const KState *kss = A.ks + 2 * i, *ksg = kss + 1;
+    const BInst I = A.inst[2 * i + 1];
+    const long long x = (long long)blockIdx.x * PE_T + threadIdx.x;
+    if (x >= 1LL << I.n) return;  // whole blocks: registers have 2^8 amplitudes or more
+    C *out = reinterpret_cast<C *>(D.gout) + I.off0;
+    if (!job_ok(kss) || !job_ok(ksg)) {
+        if (__ldcg(&ksg->s0) == 0.0) out[x] = cmake<C>(0.0, 0.0);  // exp(+i dt H) 0 = 0
+        return;
     }
+    const int nvec = __ldcg(&ksg->nvec);
+    for (int k = threadIdx.x; k < nvec; k += PE_T) {  // as load_coefs, conjugated
+        const double f = __ldcg(&ksg->s0) * __ldcg(&ksg->scale[k]);
+        cf[k] = make_double2(f * __ldcg(&ksg->c_re[k]), -(f * __ldcg(&ksg->c_im[k])));
+    }
+    __syncthreads();
+    double re = 0.0, im = 0.0;
+    constexpr int U = 8;  // loads in flight
+    for (int k0 = 0; k0 < nvec; k0 += U) {
+        C b[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            b[u] = k0 + u < nvec ? ldcg(vec_ptr<C>(A, k0 + u, I) + x) : cmake<C>(0.0, 0.0);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (k0 + u >= nvec) break;
+            const double c_r = cf[k0 + u].x, c_i = cf[k0 + u].y;
+            re += c_r * double(b[u].x) - c_i * double(b[u].y);
+            im += c_r * double(b[u].y) + c_i * double(b[u].x);
+        }
+    }
+    out[x] = cmake<C>(re, im);
+}
+
+// The contractions sum_k conj(G_k(x)) E_k(x ^ bit p): per bit p the sum T over all x and its
+// part U over x with bit p set, and S_pp = sum_x x_p rho(x), rho = sum_k conj(G_k) E_k.  A block
+// takes 2^tb consecutive amplitudes (tb = min(n, PC_TB)) and every gridDim.y-th k; a thread owns
+// NA amplitudes throughout and keeps its sums in registers until the end (its bits do not
+// change), one block reduction in all.  Low bits: the partners of E_k's tile from shared
+// memory, the next tile loaded meanwhile.  High bits (k_post_high): products with partner
+// tiles, PC_H bits a block.  Rows of NCP sums at partC; k_post_finish adds them.  138 + 92 + 5 us
+// at 12 registers of 14 qubits; each kernel reads the 110 MB of E and of G about once.
+constexpr int PC_T = 256, PC_TB = 10, PC_H = 4, PC_KS = 4;  // PC_KS: most blocks of one tile
+// Row of an instance's block: instances of fewer than 2^PC_TB amplitudes have one block each.
+__device__ __forceinline__ double *post_row(const BAdj &D, const BInst &I, int i, int block) {
+    return D.partC + ((size_t)((I.off0 >> PC_TB) + i) * PC_KS + block) * NCP;
+}
+__device__ __forceinline__ bool post_block(const BArgs &A, int i, BInst *I, BInst *IG, int *mg) {
+    const KState *kss = A.ks + 2 * i, *ksg = kss + 1;
+    if (!job_ok(kss) || !job_ok(ksg)) return false;
+    *I = A.inst[2 * i];
+    *IG = A.inst[2 * i + 1];
+    *mg = basis_size(ksg);
+    return (long long)blockIdx.x << (I->n < PC_TB ? I->n : PC_TB) < 1LL << I->n;
+}
+
+template <typename R>
+__global__ void __launch_bounds__(PC_T, 2) k_post_low(const BArgs A, const BAdj D) {
+    typedef typename cvec<R>::T C;
+    constexpr int NA = 1 << (PC_TB - 8), NV = 4 * PC_TB + 2 * PC_TB + 2, NWP = PC_T / 32;
+    __shared__ C tile[2][1 << PC_TB];
+    __shared__ double red[NWP][NV];
+    const int i = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    BInst I, IG;
+    int mg;
+    if (!post_block(A, i, &I, &IG, &mg)) return;
+    const KState *ksg = A.ks + 2 * i + 1;
+    const int n = I.n, tb = n < PC_TB ? n : PC_TB;
+    const long long base = (long long)blockIdx.x << tb;
+    const C zero = cmake<C>(0.0, 0.0);
+    // amplitudes tid + 256 a < 2^tb; sums of the thread bits, of the register bits by the bit
+    // (0, 1), rho
+    double Tr[8], Ti[8], Qr[NA / 2][2], Qi[NA / 2][2], rr[NA], ri[NA];
+#pragma unroll
+    for (int p = 0; p < 8; ++p) Tr[p] = Ti[p] = 0.0;
+#pragma unroll
+    for (int q = 0; q < NA / 2; ++q) Qr[q][0] = Qr[q][1] = Qi[q][0] = Qi[q][1] = 0.0;
+#pragma unroll
+    for (int a = 0; a < NA; ++a) rr[a] = ri[a] = 0.0;
+    auto Ek = [&](int k) { return reinterpret_cast<const C *>(D.E + (size_t)k * D.inst_amps * sizeof(C)) + I.off0 + base; };
+    C en[NA], gn[NA];
+    auto fetch = [&](int k) {
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            const bool on = tid + a * PC_T < (1 << tb);
+            en[a] = on ? ldcg(Ek(k) + tid + a * PC_T) : zero;
+            gn[a] = on ? ldcg(vec_ptr<C>(A, k, IG) + base + tid + a * PC_T) : zero;
+        }
+    };
+    int buf = 0;
+    if ((int)blockIdx.y < mg) fetch(blockIdx.y);
+    for (int k = blockIdx.y; k < mg; k += gridDim.y, buf ^= 1) {
+        const double gs = __ldcg(&ksg->scale[k]);
+        double gr[NA], gi[NA];
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            gr[a] = gs * double(gn[a].x);
+            gi[a] = -gs * double(gn[a].y);  // conj
+            tile[buf][tid + a * PC_T] = en[a];
+        }
+        __syncthreads();  // (the other buffer's readers are past this barrier's predecessor)
+        if (k + (int)gridDim.y < mg) fetch(k + gridDim.y);
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            const C w = tile[buf][tid + a * PC_T];
+            rr[a] += gr[a] * double(w.x) - gi[a] * double(w.y);
+            ri[a] += gr[a] * double(w.y) + gi[a] * double(w.x);
+        }
+#pragma unroll
+        for (int p = 0; p < 8; ++p) {
+            if (p >= tb) break;
+#pragma unroll
+            for (int a = 0; a < NA; ++a) {
+                const C w = tile[buf][(tid ^ (1 << p)) + a * PC_T];
+                Tr[p] += gr[a] * double(w.x) - gi[a] * double(w.y);
+                Ti[p] += gr[a] * double(w.y) + gi[a] * double(w.x);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < NA / 2; ++q) {
+            if (8 + q >= tb) break;
+#pragma unroll
+            for (int a = 0; a < NA; ++a) {
+                const int bit = (a >> q) & 1;
+                const C w = tile[buf][tid + (a ^ (1 << q)) * PC_T];
+                Qr[q][bit] += gr[a] * double(w.x) - gi[a] * double(w.y);
+                Qi[q][bit] += gr[a] * double(w.y) + gi[a] * double(w.x);
+            }
+        }
+    }
+    // block sums: bit p: T, U at 4 p; S at 4 PC_TB + 2 p; the total of rho last
+    auto put = [&](int v, double x) {
+        x = warp_sum(x);
+        if (lane == 0) red[warp][v] = x;
+    };
+    double sr = 0.0, si = 0.0;
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+        sr += rr[a];
+        si += ri[a];
+    }
+#pragma unroll
+    for (int p = 0; p < PC_TB; ++p) {
+        const bool bit = p < 8 && ((tid >> p) & 1);
+        double t[2], u[2], q[2];
+        if (p < 8) {
+            t[0] = Tr[p < 8 ? p : 0];
+            t[1] = Ti[p < 8 ? p : 0];
+            u[0] = bit ? t[0] : 0.0;
+            u[1] = bit ? t[1] : 0.0;
+            q[0] = bit ? sr : 0.0;
+            q[1] = bit ? si : 0.0;
+        } else {
+            const int r = p - 8;
+            u[0] = Qr[r][1];
+            u[1] = Qi[r][1];
+            t[0] = Qr[r][0] + u[0];
+            t[1] = Qi[r][0] + u[1];
+            q[0] = q[1] = 0.0;
+#pragma unroll
+            for (int a = 0; a < NA; ++a)
+                if ((a >> r) & 1) {
+                    q[0] += rr[a];
+                    q[1] += ri[a];
+                }
+        }
+        put(4 * p, t[0]);
+        put(4 * p + 1, t[1]);
+        put(4 * p + 2, u[0]);
+        put(4 * p + 3, u[1]);
+        put(4 * PC_TB + 2 * p, q[0]);
+        put(4 * PC_TB + 2 * p + 1, q[1]);
+    }
+    put(NV - 2, sr);
+    put(NV - 1, si);
+    __syncthreads();
+    double *row = post_row(D, I, i, blockIdx.x * gridDim.y + blockIdx.y);
+    for (int v = tid; v < 6 * n; v += PC_T) {  // row: 6 values a bit: T, U, S
+        const int p = v / 6, c = v - 6 * p;
+        double x = 0.0;
+        if (p < tb) {
+            const int at = c < 4 ? 4 * p + c : 4 * PC_TB + 2 * p + c - 4;
+            for (int w = 0; w < NWP; ++w) x += red[w][at];
+        } else if (c >= 4) {  // a bit of the block: all of rho or nothing
+            if ((base >> p) & 1)
+                for (int w = 0; w < NWP; ++w) x += red[w][NV - 2 + c - 4];
+        } else {
+            continue;  // k_post_high's
+        }
+        row[v] = x;
+    }
+}
+
+template <typename R>
+__global__ void __launch_bounds__(PC_T) k_post_high(const BArgs A, const BAdj D, int ksplit) {
+    typedef typename cvec<R>::T C;
+    constexpr int NA = 1 << (PC_TB - 8), NWP = PC_T / 32;
+    __shared__ double red[NWP][2 * PC_H];
+    const int i = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ky = blockIdx.y % ksplit, p0 = PC_TB + (blockIdx.y / ksplit) * PC_H;
+    BInst I, IG;
+    int mg;
+    if (!post_block(A, i, &I, &IG, &mg) || p0 >= I.n) return;
+    const KState *ksg = A.ks + 2 * i + 1;
+    const int n = I.n, np = n - p0 < PC_H ? n - p0 : PC_H;
+    const long long base = (long long)blockIdx.x << PC_TB;
+    double Tr[PC_H], Ti[PC_H];
+#pragma unroll
+    for (int q = 0; q < PC_H; ++q) Tr[q] = Ti[q] = 0.0;
+    for (int k = ky; k < mg; k += ksplit) {
+        const double gs = __ldcg(&ksg->scale[k]);
+        const C *G = vec_ptr<C>(A, k, IG) + base + tid;
+        const C *E = reinterpret_cast<const C *>(D.E + (size_t)k * D.inst_amps * sizeof(C)) + I.off0 + tid;
+        C g[NA], w[PC_H][NA];
+#pragma unroll
+        for (int a = 0; a < NA; ++a) g[a] = ldcg(G + a * PC_T);
+#pragma unroll
+        for (int q = 0; q < PC_H; ++q)
+#pragma unroll
+            for (int a = 0; a < NA; ++a)
+                w[q][a] = q < np ? ldcg(E + (base ^ (1LL << (p0 + q))) + a * PC_T) : cmake<C>(0.0, 0.0);
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            const double gr = gs * double(g[a].x), gi = -gs * double(g[a].y);
+#pragma unroll
+            for (int q = 0; q < PC_H; ++q) {
+                Tr[q] += gr * double(w[q][a].x) - gi * double(w[q][a].y);
+                Ti[q] += gr * double(w[q][a].y) + gi * double(w[q][a].x);
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < PC_H; ++q) {
+        const double x = warp_sum(Tr[q]), y = warp_sum(Ti[q]);
+        if (lane == 0) {
+            red[warp][2 * q] = x;
+            red[warp][2 * q + 1] = y;
+        }
+    }
+    __syncthreads();
+    double *row = post_row(D, I, i, blockIdx.x * ksplit + ky);
+    if (tid < 4 * np) {
+        const int q = tid >> 2, c = tid & 3, p = p0 + q;
+        double x = 0.0;
+        for (int w = 0; w < NWP; ++w) x += red[w][2 * q + (c & 1)];
+        row[6 * p + c] = c < 2 || ((base >> p) & 1) ? x : 0.0;
+    }
+}
+
+// The step's gradients of instance i from its rows (torch.py:324-353).
+constexpr int PF_G = 4;  // groups of rows summed side by side
+__global__ void __launch_bounds__(128 * PF_G) k_post_finish(const BArgs A, const BAdj D, int ksplit) {
+    __shared__ double part[PF_G][128];
+    const int i = blockIdx.x, v = threadIdx.x & 127, gq = threadIdx.x >> 7;
+    const KState *kss = A.ks + 2 * i, *ksg = kss + 1;
+    const BInst I = A.inst[2 * i];
+    const int n = I.n, p = threadIdx.x;
+    double *g = D.grads + (size_t)i * 3 * BMAXQ;
+    if (!job_ok(kss) || !job_ok(ksg)) {  // a zero gradient (or a failed basis): no parameter gradient
+        const bool zero = __ldcg(&ksg->s0) == 0.0;
+        if (p < n) g[p] = g[BMAXQ + p] = g[2 * BMAXQ + p] = 0.0;
+        if (p == 0) {
+            int e = EMUSV_OK;
+            if (!zero) {
+                e = EMUSV_NONFINITE;
+                for (const KState *k2 : {kss, ksg}) {
+                    const int st = ld_status(k2);
+                    if (st == KS_MAXDIM) e = EMUSV_NOT_CONVERGED;  // double_krylov.py:107-110
+                    if (st == BS_CAPACITY) e = EMUSV_WORKSPACE_TOO_SMALL;
+                }
+            }
+            D.astatus[i] = e;
+        }
+        return;
+    }
+    static_assert(NCP <= 128, "a thread per value of a row");
+    const int rows = (n > PC_TB ? 1 << (n - PC_TB) : 1) * ksplit;
+    double t = 0.0;
+    if (v < 6 * n) {
+        const double *q = post_row(D, I, i, 0) + v;
+#pragma unroll 8
+        for (int r = gq; r < rows; r += PF_G) t += __ldcg(q + (size_t)r * NCP);
+    }
+    part[gq][v] = t;
+    __syncthreads();
+    if (p >= n) return;
+    double sum[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+        sum[c] = 0.0;
+#pragma unroll
+        for (int k = 0; k < PF_G; ++k) sum[c] += part[k][6 * p + c];
+    }
+    const int q = n - 1 - p;  // bit p is qubit q
+    const BCoef &cf = A.coef[I.coef0 + D.step];
+    const double dt = I.dt, c = __ldcg(&kss->s0) * __ldcg(&ksg->s0);
+    const double Ure = sum[2], Uim = sum[3], Dre = sum[0] - sum[2], Dim = sum[1] - sum[3];
+    // Re(-i dt c <.>) for a flip with coefficient a on |1><0| and conj(a) on |0><1|
+    auto flip = [&](double ar, double ai) {
+        const double im = ar * Uim + ai * Ure + ar * Dim - ai * Dre;
+        return dt * c * im;
+    };
+    const double om = cf.om[p], phv = cf.ph[p];
+    g[q] = flip(0.5 * cos(phv), 0.5 * sin(phv));                         // DHDOmegaSparse
+    g[BMAXQ + q] = dt * c * (-sum[5]);                                   // DHDDeltaSparse: -n
+    g[2 * BMAXQ + q] = flip(-0.5 * om * sin(phv), 0.5 * om * cos(phv));  // DHDPhiSparse
+    if (p == 0) D.astatus[i] = EMUSV_OK;
 }
 
 // ---------------------------------------------------------------- host side
@@ -1611,12 +1755,11 @@ static bool layout(int ninst, const int *nq, const int *nsteps, int es, int T, i
     L->args = take(sizeof(BArgs));
     // control block and integer flags, contiguous so that a launch clears them in one go:
     // per job the phase engine's state and take words (two ints each, 8-byte aligned after
-    // the 32-byte control block), hint, polled, fail, status, ranB, cnt[3], then the
-    // adjoint's counters
+    // the 32-byte control block), hint, polled, fail, status, ranB, cnt[3]
     L->ctl = off;
     off += sizeof(BCtl);
     L->ints = off;
-    off += sizeof(int) * (12 * (size_t)nj + ninst);
+    off += sizeof(int) * 12 * (size_t)nj;
     off = al256(off);
     L->rec = take(sizeof(PRec) * (7 * (size_t)L->total_tiles + (size_t)GANG_JREC * nj));
     L->cta0 = take(sizeof(int) * (nj + 1));
@@ -1636,7 +1779,7 @@ static bool layout(int ninst, const int *nq, const int *nsteps, int es, int T, i
     if (adjoint) {
         L->dS = take(sizeof(double2) * ninst * (size_t)L->mmax * L->mmax);
         L->E = take((size_t)L->mmax * (size_t)amps * es);
-        L->partC = take(sizeof(double) * NCP * (size_t)L->total_tiles);
+        L->partC = take(sizeof(double) * NCP * PC_KS * ((size_t)(amps >> PC_TB) + ninst));
     }
     L->total = off;
     return true;
@@ -1649,12 +1792,11 @@ struct Shape {
     static constexpr int MINB = (sizeof(R) == 4 ? T >= 10 : T >= 9) ? 1 : 2;
 };
 
-// kind 0: forward (lock-step rounds); 1: adjoint rounds; 2: adjoint post-processing;
-// 3: forward (phase engine); 4: gangs (forward and the adjoint's bases)
+// kind 0: forward (lock-step rounds); 1: adjoint rounds; 3: forward (phase engine);
+// 4: gangs (forward and the adjoint's bases)
 static void *pick_kernel(int dtype, int T, int kind) {
 #define EMUSV_K(R, TT)                                                                   \
     (kind == 1   ? reinterpret_cast<void *>(k_batch_adj_rounds<R, TT, Shape<R, TT>::MINB>) \
-     : kind == 2 ? reinterpret_cast<void *>(k_batch_adj_post<R, TT, Shape<R, TT>::MINB>)   \
      : kind == 3 ? reinterpret_cast<void *>(k_batch_phase<R, TT, Shape<R, TT>::MINB>)      \
      : kind == 4 ? reinterpret_cast<void *>(k_batch_gang<R, TT, Shape<R, TT>::MINB>)       \
                  : reinterpret_cast<void *>(k_batch<R, TT, Shape<R, TT>::MINB>))
@@ -1670,11 +1812,9 @@ static void *pick_kernel(int dtype, int T, int kind) {
     return nullptr;
 }
 
-// Dynamic shared memory of a kernel kind: the H v phase's partner-tile stages (kinds 0
-// and 1; the post-processing kernel has none).  Set as the kernel's limit before its
-// occupancy is queried or it is launched.
+// Dynamic shared memory of a kernel kind: the H v phase's partner-tile stages.  Set as the
+// kernel's limit before its occupancy is queried or it is launched.
 static size_t kernel_smem(int dtype, int T, int kind) {
-    if (kind == 2) return 0;
     const size_t es = dtype == EMUSV_C128 ? 16 : 8;
     return (size_t)BWARPS * PSTAGES * (es << T);
 }
@@ -1692,6 +1832,7 @@ struct Prepared {
     BLayout L;
     bool adjoint;
     int engine;  // forward launches: 0 lock-step rounds, 1 phase engine
+    int nmax;    // qubits of the largest instance
     int gang;    // CTAs of the gangs (phase engine and adjoint), 0: more tiles than warps
 };
 static std::mutex g_args_mu;
@@ -1849,7 +1990,6 @@ static int prepare_common(int ninst, const int *nqubits, const int *nsteps, cons
         D.E = ws + L.E;
         D.inst_amps = L.inst_amps;
         D.partC = reinterpret_cast<double *>(ws + L.partC);
-        D.cntC = reinterpret_cast<unsigned *>(ints + 12 * nj);
     }
     std::vector<int> cta0(nj + 1);
     for (int J = 0; J < nj; ++J) cta0[J + 1] = cta0[J] + (inst[J].ntiles + BWARPS - 1) / BWARPS;
@@ -1857,6 +1997,8 @@ static int prepare_common(int ninst, const int *nqubits, const int *nsteps, cons
     EMUSV_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick_kernel(dtype, T, 4), BWARPS * 32,
                                                               kernel_smem(dtype, T, 4)));
     const int deciding = (nj + BWARPS - 1) / BWARPS;
+    P.nmax = 0;
+    for (int i = 0; i < ninst; ++i) P.nmax = nqubits[i] > P.nmax ? nqubits[i] : P.nmax;
     P.gang = cta0[nj] + deciding <= per_sm * sm_count() ? cta0[nj] : 0;
     EMUSV_CHECK(cudaMemcpyAsync(ws + L.cta0, cta0.data(), sizeof(int) * (nj + 1), cudaMemcpyHostToDevice, s));
     EMUSV_CHECK(cudaMemcpyAsync(ws + L.args, &A, sizeof(A), cudaMemcpyHostToDevice, s));
@@ -1864,7 +2006,7 @@ static int prepare_common(int ninst, const int *nqubits, const int *nsteps, cons
     EMUSV_CHECK(cudaMemcpyAsync(ws + L.coef, coef.data(), sizeof(BCoef) * coef.size(), cudaMemcpyHostToDevice, s));
     EMUSV_CHECK(cudaMemcpyAsync(ws + L.ubits, ub.data(), sizeof(double) * ub.size(), cudaMemcpyHostToDevice, s));
     EMUSV_CHECK(cudaMemcpyAsync(ws + L.elow, elow.data(), sizeof(double) * elow.size(), cudaMemcpyHostToDevice, s));
-    EMUSV_CHECK(cudaMemsetAsync(ws + L.ctl, 0, sizeof(BCtl) + sizeof(int) * (12 * (size_t)nj + ninst), s));
+    EMUSV_CHECK(cudaMemsetAsync(ws + L.ctl, 0, sizeof(BCtl) + sizeof(int) * 12 * (size_t)nj, s));
     EMUSV_CHECK(cudaStreamSynchronize(s));  // the host tables go out of scope
     {
         std::lock_guard<std::mutex> g(g_args_mu);
@@ -2071,7 +2213,7 @@ int emusv_batch_adjoint_prepare(int ninst, const int *nqubits, const int *nsteps
 int emusv_batch_adjoint_launch(int dtype, int tile_bits, int blocks_per_sm, int step,
                                const void *states, const void *grad_in, void *grad_out,
                                double *grads_dev, int *status_dev, void *workspace, void *stream) {
-    void *k1 = pick_kernel(dtype, tile_bits, 1), *k3 = pick_kernel(dtype, tile_bits, 2);
+    void *k1 = pick_kernel(dtype, tile_bits, 1);
     Prepared P;
     if (!k1 || !workspace || !states || !grad_in || !grad_out || !grads_dev || !status_dev ||
         blocks_per_sm < 1 || lookup(workspace, true, &P))
@@ -2095,7 +2237,7 @@ int emusv_batch_adjoint_launch(int dtype, int tile_bits, int blocks_per_sm, int 
     // hints carry from one step to the next)
     const int nj = A.ninst;
     EMUSV_CHECK(cudaMemsetAsync(ws + P.L.ctl, 0, sizeof(BCtl) + sizeof(int) * 4 * (size_t)nj, s));
-    EMUSV_CHECK(cudaMemsetAsync(A.fail, 0, sizeof(int) * (6 * (size_t)nj + D.ninst), s));
+    EMUSV_CHECK(cudaMemsetAsync(A.fail, 0, sizeof(int) * 6 * (size_t)nj, s));
     void *args[] = {(void *)&A, (void *)&D};
     const int st = P.gang ? gang_launch(dtype, P, A, ws, s)
                           : cooperative_launch(k1, blocks_per_sm, args, s, 0, PROF_BATCH,
@@ -2107,8 +2249,34 @@ int emusv_batch_adjoint_launch(int dtype, int tile_bits, int blocks_per_sm, int 
         k_batch_dS<<<grid, BWARPS * 32, 0, s>>>(A, D);
     }
     EMUSV_CHECK_LAUNCH();
-    EMUSV_CHECK(cudaMemsetAsync(ws + P.L.ctl, 0, sizeof(BCtl), s));
-    return cooperative_launch(k3, blocks_per_sm, args, s, 0, PROF_ADJOINT);
+    {
+        ProfScope ps_(PROF_ADJOINT, s);
+        const int ni = D.ninst;
+        const long long len = 1LL << P.nmax;
+        // one block a tile of 2^PC_TB amplitudes, or several that share its k where the tiles
+        // alone leave SMs without two blocks
+        const int tiles = P.nmax > PC_TB ? 1 << (P.nmax - PC_TB) : 1;
+        int ks = 1;
+        while (ks < PC_KS && (long long)tiles * ni * ks < 2 * sm_count()) ks *= 2;
+        const dim3 ge((unsigned)((len + PE_T * PE_X - 1) / (PE_T * PE_X)), (D.mmax + PE_K - 1) / PE_K, ni);
+        const dim3 gl(tiles, ks, ni);
+        const dim3 gh(tiles, ks * ((P.nmax - PC_TB + PC_H - 1) / PC_H), ni);
+        const dim3 go((unsigned)((len + PE_T - 1) / PE_T), ni);
+        if (dtype == EMUSV_C64) {
+            k_post_E<float><<<ge, PE_T, 0, s>>>(A, D);
+            k_post_gout<float><<<go, PE_T, 0, s>>>(A, D);
+            k_post_low<float><<<gl, PC_T, 0, s>>>(A, D);
+            if (P.nmax > PC_TB) k_post_high<float><<<gh, PC_T, 0, s>>>(A, D, ks);
+        } else {
+            k_post_E<double><<<ge, PE_T, 0, s>>>(A, D);
+            k_post_gout<double><<<go, PE_T, 0, s>>>(A, D);
+            k_post_low<double><<<gl, PC_T, 0, s>>>(A, D);
+            if (P.nmax > PC_TB) k_post_high<double><<<gh, PC_T, 0, s>>>(A, D, ks);
+        }
+        k_post_finish<<<ni, 128 * PF_G, 0, s>>>(A, D, ks);
+    }
+    EMUSV_CHECK_LAUNCH();
+    return EMUSV_OK;
 }
 
 // Failure-path test switch of a prepared workspace (forward or adjoint): later launches
