@@ -42,7 +42,7 @@
 //    (k_batch_gang, below): the same tiles and sums, so the same bits, with the exchanges
 //    inside a register's own warps.  It takes those batches for the forward engine 1 and for
 //    the adjoint's bases: the forward and adjoint sweep of 12 registers of 14 qubits, 10 steps,
-//    complex128: 117 ms by the phase engine, 41 ms by gangs.
+//    complex128: 117 ms by the phase engine, 23 ms by gangs.
 #include <math.h>
 #include <string.h>
 
@@ -296,19 +296,35 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // ---------------------------------------------------------------- phase A: H v_j on a tile
-// (returns the tile's ||H v||^2 and <v_j, H v_j>, in every lane)
-template <typename R, int T>
-__device__ __forceinline__ double3 tile_hpsi_sums(const BArgs &A, const BInst &I, int t, int step, int j, double sj) {
-    typedef typename cvec<R>::T C;
-    constexpr int AMP = 1 << (T - 5);
+// The partner tiles of the bits above the tile go through the warp's shared-memory stages by
+// cp.async: PSTAGES partner tiles in flight and no registers held by the copies, the first ones
+// issued before the tile's own terms.
+// (p < 0: the tile itself)
+template <typename C, int T>
+__device__ __forceinline__ void partner_issue(const C *u, long long base, int p, int st) {
     const int lane = threadIdx.x & 31;
-    const int n = I.n;
-    const long long base = (long long)(t - I.tile0) << T;
-    const BCoef &cf = A.coef[I.coef0 + step];  // step: absolute
+    const char *src = reinterpret_cast<const char *>(u + (p < 0 ? base : base ^ (1LL << p)));
+    char *dst = reinterpret_cast<char *>(hpsi_stages<C, T>() + ((size_t)st << T));
+    constexpr int CP = (int)(sizeof(C) << T) / (16 * 32);  // 16-byte copies per lane
+#pragma unroll
+    for (int m = 0; m < CP; ++m) cp_async16(dst + 16 * (lane + 32 * m), src + 16 * (lane + 32 * m));
+    cp_async_commit();
+}
+template <typename C, int T>
+__device__ __forceinline__ void partners_begin(const C *u, long long base, int n) {
+    for (int q = 0; q < PSTAGES - 1; ++q) {
+        if (q < n - T) partner_issue<C, T>(u, base, T + q, q);
+        else cp_async_commit();  // empty groups keep the group count uniform
+    }
+}
+
+// The tile's diagonal: the energy of the high bits and the lane bits' fields, and the register
+// bits' fields (fields of the low bits include the high bits' pairs).
+template <int T>
+__device__ __forceinline__ void tile_diag(const BArgs &A, const BInst &I, const BCoef &cf, long long base,
+                                          double &dlane, double (&freg)[T - 5]) {
+    const int lane = threadIdx.x & 31, n = I.n;
     const double *Ub = A.Ubits + (size_t)I.pidx * BMAXQ * BMAXQ;
-    const C *u = vec_ptr<C>(A, j, I);
-    C *out = vec_ptr<C>(A, j + 1, I);
-    // per-tile diagonal terms: fields of the low bits including the high bits' pairs
     double fl = 0.0;  // lane p < T: effective field of low bit p
     if (lane < T) {
         fl = __ldg(&cf.field[lane]);
@@ -325,21 +341,28 @@ __device__ __forceinline__ double3 tile_hpsi_sums(const BArgs &A, const BInst &I
         }
         eh = warp_sum(eh);
     }
-    double dlane = eh;  // + lane-bit fields
+    dlane = eh;  // + lane-bit fields
 #pragma unroll
     for (int p = 0; p < 5; ++p) {
         const double f = __shfl_sync(0xffffffffu, fl, p);
         if ((lane >> p) & 1) dlane += f;
     }
-    double freg[T - 5];
 #pragma unroll
     for (int k = 0; k < T - 5; ++k) freg[k] = __shfl_sync(0xffffffffu, fl, 5 + k);
-    const double *El = A.Elow + ((size_t)I.pidx << T);
+}
 
-    C v[AMP];
-    R ar[AMP], ai[AMP];
-#pragma unroll
-    for (int a = 0; a < AMP; ++a) v[a] = ldcg(u + base + lane + 32 * a);
+// (ar, ai) = H v on the tile from its amplitudes v and the partner tiles of u, begun by
+// partners_begin.
+template <typename R, int T>
+__device__ __forceinline__ void tile_hpsi_acc(const BArgs &A, const BInst &I, const BCoef &cf, long long base,
+                                              double dlane, const double (&freg)[T - 5],
+                                              const typename cvec<R>::T *u,
+                                              const typename cvec<R>::T (&v)[1 << (T - 5)],
+                                              R (&ar)[1 << (T - 5)], R (&ai)[1 << (T - 5)]) {
+    typedef typename cvec<R>::T C;
+    constexpr int AMP = 1 << (T - 5);
+    const int lane = threadIdx.x & 31;
+    const double *El = A.Elow + ((size_t)I.pidx << T);
 #pragma unroll
     for (int a = 0; a < AMP; ++a) {
         double d = dlane + __ldg(&El[lane + 32 * a]);
@@ -379,44 +402,36 @@ __device__ __forceinline__ double3 tile_hpsi_sums(const BArgs &A, const BInst &I
             cfma(bit ? ucr : dcr, bit ? uci : dci, v[a ^ (1 << k)], ar[a], ai[a]);
         }
     }
-    // bits above the tile: the partner tiles, staged through the warp's shared-memory
-    // stages by cp.async (PSTAGES partner tiles in flight and no registers held by the
-    // copies), then read back in the lanes' amplitude layout
-    C *stage0 = hpsi_stages<C, T>();
-    auto issue = [&](int p, int st) {
-        const char *src = reinterpret_cast<const char *>(u + (base ^ (1LL << p)));
-        char *dst = reinterpret_cast<char *>(stage0 + ((size_t)st << T));
-        constexpr int CP = (int)(sizeof(C) << T) / (16 * 32);  // 16-byte copies per lane
-#pragma unroll
-        for (int m = 0; m < CP; ++m) cp_async16(dst + 16 * (lane + 32 * m), src + 16 * (lane + 32 * m));
-        cp_async_commit();
-    };
-    const int np = n - T;
-    for (int q = 0; q < PSTAGES - 1; ++q) {
-        if (q < np) issue(T + q, q);
-        else cp_async_commit();  // empty groups keep the group count uniform
-    }
+    // bits above the tile, the partner tiles read back in the lanes' amplitude layout
+    const int np = I.n - T;
     for (int q = 0; q < np; ++q) {
         const int qn = q + PSTAGES - 1;  // into the stage read in iteration q - 1
-        if (qn < np) issue(T + qn, qn % PSTAGES);
+        if (qn < np) partner_issue<C, T>(u, base, T + qn, qn % PSTAGES);
         else cp_async_commit();
         cp_async_wait<PSTAGES - 1>();  // this lane's copies of partner tile q landed
         __syncwarp();                  // and every lane's
         const int p = T + q;
         R cr, ci;
         coef(p, (int)((base >> p) & 1), cr, ci);
-        const C *w = stage0 + ((size_t)(q % PSTAGES) << T) + lane;
+        const C *w = hpsi_stages<C, T>() + ((size_t)(q % PSTAGES) << T) + lane;
 #pragma unroll
         for (int a = 0; a < AMP; ++a) cfma(cr, ci, w[32 * a], ar[a], ai[a]);
         __syncwarp();  // the stage is read before it is refilled
     }
     cp_async_wait<0>();
-    // H v = sj * H stored_j; partials ||Hv||^2 and <v_j, Hv> = sj^2 <stored, H stored>
+}
+
+// H v = sj * H stored_j in place of (ar, ai); the tile's ||Hv||^2 and <v_j, Hv> = sj^2 <stored,
+// H stored>, in every lane.
+template <typename R, int AMP>
+__device__ __forceinline__ double3 hpsi_sums(double sj, const typename cvec<R>::T (&v)[AMP], R (&ar)[AMP],
+                                             R (&ai)[AMP]) {
     R h2 = 0, dr = 0, di = 0;
 #pragma unroll
     for (int a = 0; a < AMP; ++a) {
         const R hr = (R)sj * ar[a], hi = (R)sj * ai[a];
-        out[base + lane + 32 * a] = cmake<C>(hr, hi);
+        ar[a] = hr;
+        ai[a] = hi;
         h2 = fma(hr, hr, fma(hi, hi, h2));
         dr = fma((R)v[a].x, hr, fma((R)v[a].y, hi, dr));
         di = fma((R)v[a].x, hi, fma(-(R)v[a].y, hr, di));
@@ -424,6 +439,29 @@ __device__ __forceinline__ double3 tile_hpsi_sums(const BArgs &A, const BInst &I
     const double s2 = warp_sum((double)h2), s_r = warp_sum(sj * (double)dr),
                  s_i = warp_sum(sj * (double)di);
     return make_double3(s2, s_r, s_i);
+}
+
+template <typename R, int T>
+__device__ __forceinline__ double3 tile_hpsi_sums(const BArgs &A, const BInst &I, int t, int step, int j, double sj) {
+    typedef typename cvec<R>::T C;
+    constexpr int AMP = 1 << (T - 5);
+    const int lane = threadIdx.x & 31;
+    const long long base = (long long)(t - I.tile0) << T;
+    const BCoef &cf = A.coef[I.coef0 + step];  // step: absolute
+    const C *u = vec_ptr<C>(A, j, I);
+    C *out = vec_ptr<C>(A, j + 1, I);
+    partners_begin<C, T>(u, base, I.n);
+    double dlane, freg[T - 5];
+    tile_diag<T>(A, I, cf, base, dlane, freg);
+    C v[AMP];
+    R ar[AMP], ai[AMP];
+#pragma unroll
+    for (int a = 0; a < AMP; ++a) v[a] = ldcg(u + base + lane + 32 * a);
+    tile_hpsi_acc<R, T>(A, I, cf, base, dlane, freg, u, v, ar, ai);
+    const double3 s = hpsi_sums<R, AMP>(sj, v, ar, ai);
+#pragma unroll
+    for (int a = 0; a < AMP; ++a) out[base + lane + 32 * a] = cmake<C>(ar[a], ai[a]);
+    return s;
 }
 __device__ __forceinline__ void put_part(double *part, int t, double3 s) {
     if ((threadIdx.x & 31) == 0) {
@@ -440,6 +478,23 @@ __device__ bool tile_hpsi(const BArgs &A, const BInst &I, int i, int t, int step
 }
 
 // ---------------------------------------------------------------- phase B: recurrence
+// One amplitude of w = H v_j - a v_j - b v_{j-1}; adds its ||w||^2 and <v_j, w>.  Every product
+// and sum is written out, so that all schedulers round alike.
+template <typename C>
+__device__ __forceinline__ C orth_amp(C h, C q, C pv, double car, double cai, double cb, double sj, double &acc0,
+                                      double &acc1, double &acc2) {
+    const double qx = q.x, qy = q.y;
+    const double tr = fma(car, qx, -__dmul_rn(cai, qy)), ti = fma(car, qy, __dmul_rn(cai, qx));
+    const double wr = fma(-cb, double(pv.x), __dsub_rn(double(h.x), tr));
+    const double wi = fma(-cb, double(pv.y), __dsub_rn(double(h.y), ti));
+    const C o = cmake<C>(wr, wi);
+    const double orr = double(o.x), oi = double(o.y);
+    const double vr = __dmul_rn(sj, qx), vi = __dmul_rn(sj, qy);
+    acc0 = __dadd_rn(acc0, fma(orr, orr, __dmul_rn(oi, oi)));
+    acc1 = __dadd_rn(acc1, fma(vr, orr, __dmul_rn(vi, oi)));
+    acc2 = __dadd_rn(acc2, fma(vr, oi, -__dmul_rn(vi, orr)));
+    return o;
+}
 // (returns the tile's ||w||^2 and <v_j, w>, in every lane)
 template <typename R, int T>
 __device__ __forceinline__ double3 tile_orth_sums(const BArgs &A, const BInst &I, int t, int j, double car, double cai,
@@ -465,17 +520,7 @@ __device__ __forceinline__ double3 tile_orth_sums(const BArgs &A, const BInst &I
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
             const long long x = base + lane + 32 * (a0 + c);
-            double wr = double(h[c].x) - (car * double(q[c].x) - cai * double(q[c].y));
-            double wi = double(h[c].y) - (car * double(q[c].y) + cai * double(q[c].x));
-            wr -= cb * double(pv[c].x);
-            wi -= cb * double(pv[c].y);
-            const C o = cmake<C>(wr, wi);
-            w[x] = o;
-            const double orr = double(o.x), oi = double(o.y);
-            const double vr = sj * double(q[c].x), vi = sj * double(q[c].y);
-            acc0 += orr * orr + oi * oi;
-            acc1 += vr * orr + vi * oi;
-            acc2 += vr * oi - vi * orr;
+            w[x] = orth_amp(h[c], q[c], pv[c], car, cai, cb, sj, acc0, acc1, acc2);
         }
     }
     acc0 = warp_sum(acc0);
@@ -689,7 +734,8 @@ __device__ __forceinline__ void load_coefs(const KState *ks, int nvec, bool conj
 }
 
 // out(tile) = sum_k coef_k stored_k(tile) over k < nvec; returns the tile's ||out||^2.
-template <typename R, int T>
+// KU vectors' loads are in flight at a time; the order of the sums is that of k.
+template <typename R, int T, int KU = 1>
 __device__ double tile_lincomb(const BArgs &A, const BInst &I, int t, int nvec, const double (&cr)[4],
                                const double (&cim)[4], typename cvec<R>::T *out) {
     typedef typename cvec<R>::T C;
@@ -702,20 +748,29 @@ __device__ double tile_lincomb(const BArgs &A, const BInst &I, int t, int nvec, 
         double re[CH], im[CH];
 #pragma unroll
         for (int c = 0; c < CH; ++c) re[c] = im[c] = 0.0;
-        for (int k = 0; k < nvec; ++k) {
-            const int src = k & 31, blk = k >> 5;
-            const double vr = blk == 0 ? cr[0] : blk == 1 ? cr[1] : blk == 2 ? cr[2] : cr[3];
-            const double vi = blk == 0 ? cim[0] : blk == 1 ? cim[1] : blk == 2 ? cim[2] : cim[3];
-            const double c_r = __shfl_sync(0xffffffffu, vr, src);
-            const double c_i = __shfl_sync(0xffffffffu, vi, src);
-            const C *vk = vec_ptr<C>(A, k, I) + base + lane;
-            C b[CH];
+        for (int k0 = 0; k0 < nvec; k0 += KU) {
+            C b[KU][CH];
 #pragma unroll
-            for (int c = 0; c < CH; ++c) b[c] = ldcg(vk + 32 * (a0 + c));
+            for (int u = 0; u < KU; ++u) {
+                if (k0 + u >= nvec) break;
+                const C *vk = vec_ptr<C>(A, k0 + u, I) + base + lane;
 #pragma unroll
-            for (int c = 0; c < CH; ++c) {
-                re[c] += c_r * double(b[c].x) - c_i * double(b[c].y);
-                im[c] += c_r * double(b[c].y) + c_i * double(b[c].x);
+                for (int c = 0; c < CH; ++c) b[u][c] = ldcg(vk + 32 * (a0 + c));
+            }
+#pragma unroll
+            for (int u = 0; u < KU; ++u) {
+                const int k = k0 + u, src = k & 31, blk = k >> 5;
+                if (k >= nvec) break;
+                const double vr = blk == 0 ? cr[0] : blk == 1 ? cr[1] : blk == 2 ? cr[2] : cr[3];
+                const double vi = blk == 0 ? cim[0] : blk == 1 ? cim[1] : blk == 2 ? cim[2] : cim[3];
+                const double c_r = __shfl_sync(0xffffffffu, vr, src);
+                const double c_i = __shfl_sync(0xffffffffu, vi, src);
+#pragma unroll
+                for (int c = 0; c < CH; ++c) {
+                    const double bx = b[u][c].x, by = b[u][c].y;
+                    re[c] = __dadd_rn(re[c], fma(c_r, bx, -__dmul_rn(c_i, by)));
+                    im[c] = __dadd_rn(im[c], fma(c_r, by, __dmul_rn(c_i, bx)));
+                }
             }
         }
 #pragma unroll
@@ -900,7 +955,7 @@ __device__ bool job_init(const BArgs &A, int i, int gstep) {
 
 // Combination tile of step rstep: psi' = s0 sum_k c_k v_k in place (optionally also into the
 // history buffer); returns the tile's ||psi'||^2.
-template <typename R, int T>
+template <typename R, int T, int KU = 1>
 __device__ __forceinline__ double tile_combine_sum(const BArgs &A, const BInst &I, int i, int t, int rstep) {
     typedef typename cvec<R>::T C;
     const int lane = threadIdx.x & 31;
@@ -909,7 +964,7 @@ __device__ __forceinline__ double tile_combine_sum(const BArgs &A, const BInst &
     double cr[4], cim[4];
     load_coefs(ks, nvec, false, cr, cim);
     C *out = vec_ptr<C>(A, 0, I);
-    const double nrm = tile_lincomb<R, T>(A, I, t, nvec, cr, cim, out);
+    const double nrm = tile_lincomb<R, T, KU>(A, I, t, nvec, cr, cim, out);
     if (A.hist && ((rstep + 1) % A.hist_every) == 0) {  // the new tile into the history slot
         constexpr int AMP = 1 << (T - 5);
         const long long base = (long long)(t - I.tile0) << T;
@@ -1101,91 +1156,339 @@ __global__ void __launch_bounds__(BWARPS * 32, MINB) k_batch_phase(const BArgs A
 // (value, epoch) and reads the records of the job's tiles until each carries the phase's epoch
 // -- instead of a visit that finds the job's next phase published.  The sums are added in the
 // order of inst_sum and the tiles' arithmetic is that of the other schedulers, so the results
-// are theirs to the bit.  The decisions are taken by one warp per job in CTAs of their own
-// while the gang goes on; iterations past the one that ends the step are left unused.
-// Measured: the 12 parameter sets of a 14-qubit ring took 87 us per Lanczos iteration with the
-// visits (1184 warps on 384 tiles and a handful of counters), about 21 us here.
+// are theirs to the bit.  A warp keeps its tile of v_j, and of H v_j between the phases, in
+// registers: a phase loads only the partner tiles and v_{j-1}.  The decisions are taken by warps
+// of their own (gang_decider) while the gang goes on; iterations past the one that ends the step
+// are left unused.
+// Measured per Lanczos iteration of 12 registers of 14 qubits: 87 us with the visits (1184 warps
+// on 384 tiles and a handful of counters), 12 here: H v 5.6, recurrence 2.2, the exchanges 1.1
+// and 1.8, the rest between them.
 struct GArgs {
     BArgs A;
     PRec *rec;        // per job 7 records a tile (A: 3, B: 3, N: 1) at 7 tile0
     PRec *jrec;       // per job GANG_JREC: start of a step, verdict, ||w||^2 and <v_j, w> of iteration j
     const int *cta0;  // [njobs + 1] first CTA of each job's gang
     int ncompute;     // CTAs of the gangs; the deciding CTAs follow
+    int width;        // deciding warps of a job, a power of two up to BWARPS
 };
 constexpr int GANG_JREC = 2 + 3 * KMAX;
 
 // Waits (lanes on their own records) until record r carries epoch e; false once the wait ran
-// out or another warp recorded an error.
+// out or another warp recorded an error.  Polls are relaxed loads, one acquire load at the end:
+// every acquire empties the SM's first-level cache, and the polls of a CTA's waiting warps kept
+// the one still at work from its loads and shuffles (its recurrence took 7 us instead of 1).
 __device__ __forceinline__ bool gang_wait(const BArgs &A, const PRec *r, unsigned long long e, PRec *o) {
+    *o = rec_get<false>(r);
+    if ((o->e & ~PSTOP) != e) {
+        const long long t0 = clock64();
+        for (unsigned i = 1;; ++i) {
+            *o = rec_get<false>(r);
+            if ((o->e & ~PSTOP) == e) break;
+            if ((i & 255u) == 0 && (clock64() - t0 > A.bar_limit || ld_vol(&A.ctl->err))) {
+                atomicCAS(&A.ctl->err, 0, EMUSV_TIMEOUT);
+                return false;
+            }
+        }
+    }
     *o = rec_get<true>(r);
-    if ((o->e & ~PSTOP) == e) return true;
+    return true;
+}
+
+// A CTA's view of its job's exchanges (two, in turn: a warp may still read the last one).
+struct GShare {
+    double v[2][3];
+    int ok[2], stop[2];
+};
+
+// The job's sums over its tiles of NS values a tile (inst_sum's order), from the records at
+// rec; the calling warp's own values and tile.  stop: tile 0's flag goes to every warp.
+// DATA: the warps' stores before the exchange are visible to every warp after it.  Warp 0 waits
+// for the records and hands the sums to the CTA's nw warps: with every warp polling, the polls
+// of those that waited filled the SM's load path and the one still at work took up to 7 us
+// longer.  mute: the warp's records stay out (failure-path test).
+template <int NS, bool DATA = true>
+__device__ __forceinline__ bool gang_exchange(const BArgs &A, GShare &S, unsigned &turn, int nw, PRec *rec,
+                                              const BInst &I, int tl, unsigned long long e, double (&v)[NS],
+                                              bool stop_in, bool *stop, bool mute) {
+    const int lane = threadIdx.x & 31, p = turn++ & 1;
+    __syncwarp();
+    if (lane < NS && !mute) {
+        double x = v[0];
+#pragma unroll
+        for (int k = 1; k < NS; ++k)
+            if (lane == k) x = v[k];
+        if (DATA) __threadfence();
+        rec_put(rec + lane * I.ntiles + tl, x, e | (stop_in ? PSTOP : 0ull));
+    }
+    if (threadIdx.x < 32) {
+        bool ok = true, fin = false;
+        double s[NS];
+#pragma unroll
+        for (int k = 0; k < NS; ++k) s[k] = 0.0;
+        const long long t0 = clock64();
+        for (int t = lane; t < I.ntiles && ok; t += 32) {
+            PRec o[NS];
+            for (unsigned i = 1;; ++i) {
+                bool all = true;
+#pragma unroll
+                for (int k = 0; k < NS; ++k) o[k] = rec_get<false>(rec + k * I.ntiles + t);
+#pragma unroll
+                for (int k = 0; k < NS; ++k) all = all && (o[k].e & ~PSTOP) == e;
+                if (all) break;
+                if ((i & 255u) == 0 && (clock64() - t0 > A.bar_limit || ld_vol(&A.ctl->err))) {
+                    atomicCAS(&A.ctl->err, 0, EMUSV_TIMEOUT);
+                    ok = false;
+                    break;
+                }
+            }
+            if (DATA) o[0] = rec_get<true>(rec + t);
+#pragma unroll
+            for (int k = 0; k < NS; ++k) s[k] += o[k].v;
+            if (t == 0) fin = (o[0].e & PSTOP) != 0;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < NS; ++k) {
+            s[k] = warp_sum(s[k]);
+            if (lane == 0) S.v[p][k] = s[k];
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (lane == 0) {
+            S.ok[p] = ok;
+            S.stop[p] = fin;
+        }
+    }
+    asm volatile("bar.sync 1, %0;" ::"r"(32 * nw) : "memory");
+#pragma unroll
+    for (int k = 0; k < NS; ++k) v[k] = S.v[p][k];
+    *stop = S.stop[p] != 0;
+    return S.ok[p] != 0;
+}
+
+// The deciding warps of a job, B.width of them in one CTA.  The iterations of a step are dealt
+// out in turn: warp `sub` tests those with j = sub (mod width), so tests of several iterations
+// run side by side (a test of a 45-vector basis takes 30 us, an iteration of a 14-qubit gang
+// 10).  The step ends at the earliest iteration whose test says so (job_decide's rules): a warp
+// that finds an end waits for the tests of the earlier iterations.  When the first test of a
+// step already converges, the untested iterations are dealt out the same way.
+struct GDec {
+    int begin;  // 2 epoch + (the step runs): the step's state is set up
+    int over;   // epoch of the last step decided, its outcome in st
+    int st, hint;
+    int term;   // earliest iteration found to end the step
+    int fb;     // > 0: the first test, of iteration fb, converged
+    int next[BWARPS], fbdone[BWARPS], at[BWARPS];  // per warp: next iteration it tests; its share done; epoch
+    double ferr[BWARPS];                           // error estimate of its share's end
+};
+constexpr int GDEC_C = 2 * (KMAX + 2);  // a warp's coefficients (real, imaginary) in shared memory
+__device__ __forceinline__ double *gang_scratch() {
+    extern __shared__ __align__(16) unsigned char bsm[];
+    return reinterpret_cast<double *>(bsm);  // deciding CTAs have no partner tiles
+}
+static_assert(BWARPS * GDEC_C * sizeof(double) <= (size_t)BWARPS * PSTAGES * (sizeof(float2) << 8),
+              "the coefficients fit the smallest kernel's shared memory");
+
+template <typename F>
+__device__ __forceinline__ bool gang_until(const BArgs &A, F done) {  // bounded wait, warp-uniform
+    if (__any_sync(0xffffffffu, done())) return true;
     const long long t0 = clock64();
     for (unsigned i = 1;; ++i) {
-        *o = rec_get<true>(r);
-        if ((o->e & ~PSTOP) == e) return true;
-        if ((i & 255u) == 0 && (clock64() - t0 > A.bar_limit || ld_vol(&A.ctl->err))) {
+        if (__any_sync(0xffffffffu, done())) return true;
+        if ((i & 255u) == 0 && __any_sync(0xffffffffu, clock64() - t0 > A.bar_limit || ld_vol(&A.ctl->err))) {
             atomicCAS(&A.ctl->err, 0, EMUSV_TIMEOUT);
             return false;
         }
     }
 }
-
-// The job's sums over its tiles of NS values a tile (inst_sum's order), from the records at
-// rec; the calling warp's own values and tile.  stop: tile 0's flag goes to every warp.
-template <int NS>
-__device__ __forceinline__ bool gang_exchange(const BArgs &A, PRec *rec, const BInst &I, int tl, unsigned long long e,
-                                              double (&v)[NS], bool stop_in, bool *stop) {
-    const int lane = threadIdx.x & 31;
+__device__ __forceinline__ int sh_at(const int *p) { return *reinterpret_cast<const volatile int *>(p); }
+__device__ __forceinline__ int sh_get(const int *p) { return __shfl_sync(0xffffffffu, sh_at(p), 0); }  // uniform
+__device__ __forceinline__ void sh_put(int *p, int v) {  // after the warp's earlier writes
     __syncwarp();
-    if (lane < NS) {
-        double x = v[0];
-#pragma unroll
-        for (int k = 1; k < NS; ++k)
-            if (lane == k) x = v[k];
-        __threadfence();  // the warp's stores before its records
-        rec_put(rec + lane * I.ntiles + tl, x, e | (stop_in ? PSTOP : 0ull));
+    if ((threadIdx.x & 31) == 0) {
+        __threadfence_block();
+        *reinterpret_cast<volatile int *>(p) = v;
     }
-    bool ok = true, fin = false;
-#pragma unroll
-    for (int k = 0; k < NS; ++k) v[k] = 0.0;
-    for (int t = lane; t < I.ntiles && ok; t += 32) {
-#pragma unroll
-        for (int k = 0; k < NS; ++k) {
-            PRec o;
-            ok = gang_wait(A, rec + k * I.ntiles + t, e, &o) && ok;
-            v[k] += o.v;
-            if (k == 0 && t == 0) fin = (o.e & PSTOP) != 0;
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < NS; ++k) v[k] = warp_sum(v[k]);
-    *stop = __shfl_sync(0xffffffffu, (int)fin, 0) != 0;
-    return __all_sync(0xffffffffu, ok);
+    __syncwarp();
 }
 
-// The deciding warp of job i.
-__device__ void gang_decider(const GArgs &B, int i) {
+__device__ __noinline__ void gang_decider(const GArgs &B, int i, int sub, GDec *G, double *cbase) {
     const BArgs &A = B.A;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, W = B.width;
+    KState *ks = A.ks + i;
+    double *const c = cbase + (size_t)sub * GDEC_C;
+    const double dt = A.inst[i].dt;
     PRec *jr = B.jrec + (size_t)GANG_JREC * i, o;
+    auto eval = [&](int jj) { return krylov_eval(ks, jj, dt, c, c + KMAX + 2); };
+    if (sub == 0) sh_put(&G->hint, A.hint[i]);
     for (int rstep = 0; rstep < A.run_steps; ++rstep) {
-        const unsigned long long e = 1 + (unsigned long long)rstep;  // the step's epoch
-        if (A.first_step + rstep >= A.inst[i].nsteps) break;         // no step left
-        if (!__all_sync(0xffffffffu, gang_wait(A, jr, e, &o))) return;
-        bool more = job_init(A, i, A.first_step + rstep);
-        for (int j = 0; more; ++j) {
+        const int e = 1 + rstep;                              // the step's epoch
+        if (A.first_step + rstep >= A.inst[i].nsteps) break;  // no step left
+        // every warp has left the step before; then the step's state
+        sh_put(&G->at[sub], e);
+        if (sub == 0) {
+            if (!gang_until(A, [&] { return __all_sync(0xffffffffu, lane >= W || sh_at(&G->at[lane]) == e); })) return;
+            if (!__all_sync(0xffffffffu, gang_wait(A, jr, e, &o))) return;
+            const bool more = job_init(A, i, A.first_step + rstep);
+            if (lane < W) {
+                *reinterpret_cast<volatile int *>(&G->next[lane]) = lane;
+                *reinterpret_cast<volatile int *>(&G->fbdone[lane]) = 0;
+            }
+            if (lane == 0) {
+                G->term = 1 << 30;
+                G->fb = 0;
+            }
+            __syncwarp();
+            if (!more) {
+                const int st = ld_status(ks);
+                __threadfence();
+                __syncwarp();
+                if (lane == 0) {
+                    G->st = st;
+                    rec_put(jr + 1, (double)st, e);
+                }
+                sh_put(&G->over, e);
+            }
+            __threadfence_block();
+            sh_put(&G->begin, 2 * e + (more ? 1 : 0));
+        } else if (!gang_until(A, [&] { return sh_get(&G->begin) >> 1 == e; })) {
+            return;
+        }
+        __threadfence_block();
+        const int hint = sh_get(&G->hint);
+        bool redo = false;  // the warp's coefficients were overwritten by its share
+        // the warp's share of the iterations before the first test
+        auto share = [&](int jmax) {
+            for (int jj = sub; jj < jmax && jj < sh_get(&G->term); jj += W) {
+                const double err = eval(jj);
+                if (err < A.exp_tol) {
+                    if (lane == 0) {
+                        G->ferr[sub] = err;
+                        atomicMin(&G->term, jj);
+                    }
+                    break;
+                }
+            }
+            redo = true;
+            sh_put(&G->fbdone[sub], 1);
+        };
+        auto asked = [&] { return sh_get(&G->fb) > 0 && !sh_get(&G->fbdone[sub]); };
+        // waits for `done` (uniform), taking the share when it is asked for; false: the launch failed
+        auto wait = [&](auto done) {
+            for (;;) {
+                bool ask = false;
+                if (!gang_until(A, [&] { ask = asked(); return done() || ask; })) return false;
+                __threadfence_block();
+                if (!ask) return true;
+                share(sh_get(&G->fb));
+            }
+        };
+        auto over = [&] { return sh_get(&G->over) == e; };
+        // every iteration before j tested without an end (then true), or an earlier end
+        auto stands = [&](int j, bool *alone) {
+            bool all = false;
+            if (!wait([&] {
+                    all = __all_sync(0xffffffffu, lane >= W || lane == sub || sh_at(&G->next[lane]) > j);
+                    return all || sh_get(&G->term) < j || over();
+                }))
+                return false;
+            *alone = !(over() || sh_get(&G->term) < j);
+            return *alone || wait(over);  // an earlier one: its warp ends the step
+        };
+        for (int j = 0; !over(); ++j) {
+            // the sums of iteration j, or the step's end
+            bool have = lane >= 3;
             o.v = 0.0;
-            const bool got = lane >= 3 || gang_wait(A, jr + 2 + 3 * j + lane, e, &o);
-            if (!__all_sync(0xffffffffu, got)) return;
-            if (lane < 3) A.sumB[4 * (size_t)i + lane] = o.v;
+            if (!wait([&] {
+                    if (!have) {
+                        o = rec_get<false>(jr + 2 + 3 * j + lane);
+                        have = (o.e & ~PSTOP) == (unsigned long long)e;
+                    }
+                    return __all_sync(0xffffffffu, have) || over();
+                }))
+                return;
+            if (!__all_sync(0xffffffffu, have)) break;
+            if (lane < 3) o = rec_get<true>(jr + 2 + 3 * j + lane);
+            __syncwarp();
+            // (every warp writes the same norms)
+            const int flag = krylov_norms(ks, j, __shfl_sync(0xffffffffu, o.v, 0), __shfl_sync(0xffffffffu, o.v, 1),
+                                          __shfl_sync(0xffffffffu, o.v, 2), dt, A.norm_tol);
+            if ((j & (W - 1)) != sub) continue;
+            const bool poll = j + 1 >= hint || j + 1 >= A.maxdim;
+            const bool first = poll && (j == 0 || !(j >= hint || j >= A.maxdim));
+            int st = KS_RUNNING, jc = j;
+            double err = 0.0;
+            const double *cw = c;  // the ending iteration's coefficients
+            if (flag == KD_NONFINITE) {
+                st = KS_NONFINITE;
+            } else if (flag == KD_HAPPY) {
+                st = KS_HAPPY;
+            } else {
+                if (poll) {
+                    redo = false;
+                    err = eval(j);
+                    if ((err < A.exp_tol || err != err) && first && j > 0) {
+                        bool alone;
+                        if (!stands(j, &alone)) return;
+                        if (!alone) break;
+                        sh_put(&G->fb, j);
+                        share(j);
+                        if (!gang_until(A, [&] { return __all_sync(0xffffffffu, lane >= W || sh_at(&G->fbdone[lane])); }))
+                            return;
+                        __threadfence_block();
+                        const int t = sh_get(&G->term);
+                        if (t < j) {
+                            jc = t;
+                            err = *reinterpret_cast<const volatile double *>(&G->ferr[t & (W - 1)]);
+                            cw = cbase + (size_t)(t & (W - 1)) * GDEC_C;
+                            redo = false;
+                        }
+                    }
+                    if (err < A.exp_tol) st = KS_CONVERGED;
+                    else if (j + 1 >= A.maxdim) st = KS_MAXDIM;
+                }
+                if (st == KS_RUNNING && j + 2 > A.capacity) st = BS_CAPACITY;
+            }
+            if (st == KS_RUNNING) {
+                sh_put(&G->next[sub], j + W);
+                continue;
+            }
+            // an end: it stands once every earlier iteration is tested
+            if (lane == 0) atomicMin(&G->term, jc);
+            __syncwarp();
+            if (jc == j) {
+                bool alone;
+                if (!stands(j, &alone)) return;
+                if (!alone) break;
+                if (st == KS_HAPPY) krylov_happy(ks, j + 1, dt);
+                else if (poll && redo && st != KS_NONFINITE) eval(j);
+            }
+            if (st != KS_HAPPY && st != KS_NONFINITE && poll)
+                for (int k = lane; k <= jc + 1; k += 32) {
+                    ks->c_re[k] = cw[k];
+                    ks->c_im[k] = cw[KMAX + 2 + k];
+                }
+            const int iters = st == KS_CONVERGED || st == KS_MAXDIM || st == KS_HAPPY || st == KS_NONFINITE || poll
+                                  ? jc + 1 : 0;
+            if (lane == 0) {
+                ks->err = err;
+                ks->nvec = st == KS_HAPPY ? j + 1 : jc + 2;
+                ks->iters = iters;
+                ks->status = st;
+                if (st == KS_NONFINITE || st == BS_CAPACITY) A.fail[i] = st;
+                A.iters_out[(size_t)i * A.max_steps + rstep] = iters;
+                const int h = iters > 3 ? iters - 3 : 0;  // poll a little early
+                A.hint[i] = h;
+                G->hint = h;
+                G->st = st;
+            }
             __threadfence();
             __syncwarp();
-            more = job_decide(A, i, j, rstep);
+            if (lane == 0) rec_put(jr + 1, (double)st, e);
+            sh_put(&G->over, e);
+            break;
         }
-        const int st = ld_status(A.ks + i);
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) rec_put(jr + 1, (double)st, e);
+        __threadfence_block();
+        const int st = sh_get(&G->st);
         if (!A.combine || (st != KS_CONVERGED && st != KS_HAPPY && st != KS_MAXDIM)) break;
     }
 }
@@ -1195,8 +1498,12 @@ __global__ void __launch_bounds__(BWARPS * 32, MINB) k_batch_gang(const __grid_c
     const BArgs &A = B.A;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if ((int)blockIdx.x >= B.ncompute) {
-        const int i = ((int)blockIdx.x - B.ncompute) * BWARPS + warp;
-        if (i < A.ninst) gang_decider(B, i);
+        __shared__ GDec dec[BWARPS];
+        const int per = BWARPS / B.width, g = warp / B.width, i = ((int)blockIdx.x - B.ncompute) * per + g;
+        for (int k = threadIdx.x; k < (int)(sizeof(dec) / sizeof(int)); k += BWARPS * 32)
+            reinterpret_cast<int *>(dec)[k] = 0;
+        __syncthreads();
+        if (i < A.ninst) gang_decider(B, i, warp % B.width, &dec[g], gang_scratch() + (size_t)g * B.width * GDEC_C);
         return;
     }
     int lo = 0, hi = A.ninst - 1;  // the job of this CTA
@@ -1204,10 +1511,16 @@ __global__ void __launch_bounds__(BWARPS * 32, MINB) k_batch_gang(const __grid_c
         const int mid = (lo + hi + 1) >> 1;
         if (__ldg(&B.cta0[mid]) <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
     }
-    const int i = lo, tl = ((int)blockIdx.x - __ldg(&B.cta0[i])) * BWARPS + warp;
+    const int i = lo, tl0 = ((int)blockIdx.x - __ldg(&B.cta0[i])) * BWARPS, tl = tl0 + warp;
     const BInst I = A.inst[i];
     if (tl >= I.ntiles) return;
+    const int nw = I.ntiles - tl0 < BWARPS ? I.ntiles - tl0 : BWARPS;  // warps of this CTA
+    __shared__ GShare S;
+    unsigned turn = 0;
     const int t = I.tile0 + tl;
+    typedef typename cvec<R>::T C;
+    constexpr int AMP = 1 << (T - 5);
+    const long long base = (long long)tl << T;
     const bool lead = tl == 0 && lane == 0;
     KState *ks = A.ks + i;
     PRec *ra = B.rec + 7 * (size_t)I.tile0, *rb = ra + 3 * I.ntiles, *rn = ra + 6 * I.ntiles;
@@ -1216,9 +1529,9 @@ __global__ void __launch_bounds__(BWARPS * 32, MINB) k_batch_gang(const __grid_c
     bool stop = false;
     int last = BS_IDLE;
     // failure-path test switch: one sum of job 0 never arrives, its gang's waits run out
-    if (A.test_skip_arrival && i == 0 && tl == 0) return;
+    const bool mute = A.test_skip_arrival && i == 0 && tl == 0;
     double nv[1] = {tile_norm_sum<R, T>(A, I, t)};
-    if (!gang_exchange<1>(A, rn, I, tl, ++en, nv, false, &stop)) return;
+    if (!gang_exchange<1>(A, S, turn, nw, rn, I, tl, ++en, nv, false, &stop, mute)) return;
     const int limit = A.maxdim < A.capacity ? A.maxdim : A.capacity;
     for (int rstep = 0; rstep < A.run_steps; ++rstep) {
         const int gstep = A.first_step + rstep;
@@ -1235,13 +1548,28 @@ __global__ void __launch_bounds__(BWARPS * 32, MINB) k_batch_gang(const __grid_c
         const double s0 = sqrt(nv[0]);
         double sn = nv[0], scale = 1.0 / s0, sp = 0.0, b = 0.0, vr = 0.0, vi = 0.0;
         const bool fine = isfinite(s0) && s0 > 0.0;  // else the decision is KS_NONFINITE
+        // the warp's tile of v_j stays in its registers, and H v_j from A to B
+        const BCoef &cf = A.coef[I.coef0 + gstep];
+        double dlane, freg[T - 5];
+        tile_diag<T>(A, I, cf, base, dlane, freg);
+        C v[AMP];
+#pragma unroll
+        for (int a = 0; a < AMP; ++a) v[a] = ldcg(vec_ptr<C>(A, 0, I) + base + lane + 32 * a);
         for (int j = 0; fine && j < limit; ++j) {
             // A: H v_j
             double sj = 1.0 / sqrt(sn);
             if (!isfinite(sj) || sj <= 0.0) sj = 0.0;
-            const double3 pa = tile_hpsi_sums<R, T>(A, I, t, gstep, j, sj);
+            const C *u = vec_ptr<C>(A, j, I);
+            partners_begin<C, T>(u, base, I.n);
+            R hr[AMP], hi[AMP];
+            tile_hpsi_acc<R, T>(A, I, cf, base, dlane, freg, u, v, hr, hi);
+            const double3 pa = hpsi_sums<R, AMP>(sj, v, hr, hi);
+            if (j > 0) partner_issue<C, T>(vec_ptr<C>(A, j - 1, I), base, -1, 0);  // v_{j-1}'s tile, for B
             double a[3] = {pa.x, pa.y, pa.z};
-            if (!gang_exchange<3>(A, ra, I, tl, ++ea, a, false, &stop)) return;
+            if (!gang_exchange<3, false>(A, S, turn, nw, ra, I, tl, ++ea, a, false, &stop, mute)) {
+                cp_async_wait<0>();
+                return;
+            }
             // B: w = H v_j - a v_j - b v_{j-1}
             const double ar = a[1] - b * vr, ai = a[2] - b * vi;
             if (lead) {  // T_H's column j (read by the decision)
@@ -1251,9 +1579,20 @@ __global__ void __launch_bounds__(BWARPS * 32, MINB) k_batch_gang(const __grid_c
                 ks->b_im[j] = 0.0;
                 ks->hn[j] = sqrt(a[0]);
             }
-            const double3 pb = tile_orth_sums<R, T>(A, I, t, j, ar * scale, ai * scale, b * sp, scale);
-            double w[3] = {pb.x, pb.y, pb.z};
-            if (!gang_exchange<3>(A, rb, I, tl, ++eb, w, lead && rec_get(jr + 1).e == e, &stop)) return;
+            cp_async_wait<0>();
+            __syncwarp();
+            double w[3] = {0.0, 0.0, 0.0};
+            C *wv = vec_ptr<C>(A, j + 1, I) + base + lane;
+            const double car = ar * scale, cai = ai * scale, cb = b * sp;
+#pragma unroll
+            for (int c = 0; c < AMP; ++c) {
+                const C pv = j > 0 ? hpsi_stages<C, T>()[lane + 32 * c] : cmake<C>(0.0, 0.0);
+                v[c] = orth_amp(cmake<C>(hr[c], hi[c]), v[c], pv, car, cai, cb, scale, w[0], w[1], w[2]);
+                wv[32 * c] = v[c];
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) w[c] = warp_sum(w[c]);
+            if (!gang_exchange<3>(A, S, turn, nw, rb, I, tl, ++eb, w, lead && rec_get<false>(jr + 1).e == e, &stop, mute)) return;
             if (tl == 0 && lane < 3) rec_put(jr + 2 + 3 * j + lane, lane == 0 ? w[0] : lane == 1 ? w[1] : w[2], e);
             if (stop) break;
             const double r = sqrt(w[0]);  // as krylov_norms
@@ -1264,12 +1603,21 @@ __global__ void __launch_bounds__(BWARPS * 32, MINB) k_batch_gang(const __grid_c
             vr = w[1] / r;
             vi = -w[2] / r;
         }
-        PRec o;
-        if (!__all_sync(0xffffffffu, gang_wait(A, jr + 1, e, &o))) return;
-        last = (int)o.v;
+        const int p = turn++ & 1;
+        if (warp == 0) {
+            PRec o;
+            const bool ok = __all_sync(0xffffffffu, gang_wait(A, jr + 1, e, &o));
+            if (lane == 0) {
+                S.v[p][0] = o.v;
+                S.ok[p] = ok;
+            }
+        }
+        asm volatile("bar.sync 1, %0;" ::"r"(32 * nw) : "memory");
+        if (!S.ok[p]) return;
+        last = (int)S.v[p][0];
         if (!A.combine || (last != KS_CONVERGED && last != KS_HAPPY && last != KS_MAXDIM)) break;
-        nv[0] = tile_combine_sum<R, T>(A, I, i, t, rstep);
-        if (!gang_exchange<1>(A, rn, I, tl, ++en, nv, false, &stop)) return;
+        nv[0] = tile_combine_sum<R, T, MINB == 1 ? 4 : 2>(A, I, i, t, rstep);
+        if (!gang_exchange<1>(A, S, turn, nw, rn, I, tl, ++en, nv, false, &stop, mute)) return;
     }
     if (lead) {
         const int f = ld_vol(&A.fail[i]);
@@ -1436,8 +1784,9 @@ __global__ void __launch_bounds__(PE_T) k_post_gout(const BArgs A, const BAdj D)
         for (int u = 0; u < U; ++u) {
             if (k0 + u >= nvec) break;
             const double c_r = cf[k0 + u].x, c_i = cf[k0 + u].y;
-            re += c_r * double(b[u].x) - c_i * double(b[u].y);
-            im += c_r * double(b[u].y) + c_i * double(b[u].x);
+            const double bx = b[u].x, by = b[u].y;
+            re = __dadd_rn(re, fma(c_r, bx, -__dmul_rn(c_i, by)));
+            im = __dadd_rn(im, fma(c_r, by, __dmul_rn(c_i, bx)));
         }
     }
     out[x] = cmake<C>(re, im);
@@ -1833,6 +2182,7 @@ struct Prepared {
     bool adjoint;
     int engine;  // forward launches: 0 lock-step rounds, 1 phase engine
     int nmax;    // qubits of the largest instance
+    int width;   // deciding warps of a gang
     int gang;    // CTAs of the gangs (phase engine and adjoint), 0: more tiles than warps
 };
 static std::mutex g_args_mu;
@@ -1996,10 +2346,13 @@ static int prepare_common(int ninst, const int *nqubits, const int *nsteps, cons
     int per_sm = 0;
     EMUSV_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick_kernel(dtype, T, 4), BWARPS * 32,
                                                               kernel_smem(dtype, T, 4)));
-    const int deciding = (nj + BWARPS - 1) / BWARPS;
+    // as many deciding warps a job as fit beside the gangs
+    P.width = BWARPS;
+    auto deciding = [&] { return (nj * P.width + BWARPS - 1) / BWARPS; };
+    while (P.width > 1 && cta0[nj] + deciding() > per_sm * sm_count()) P.width /= 2;
     P.nmax = 0;
     for (int i = 0; i < ninst; ++i) P.nmax = nqubits[i] > P.nmax ? nqubits[i] : P.nmax;
-    P.gang = cta0[nj] + deciding <= per_sm * sm_count() ? cta0[nj] : 0;
+    P.gang = cta0[nj] + deciding() <= per_sm * sm_count() ? cta0[nj] : 0;
     EMUSV_CHECK(cudaMemcpyAsync(ws + L.cta0, cta0.data(), sizeof(int) * (nj + 1), cudaMemcpyHostToDevice, s));
     EMUSV_CHECK(cudaMemcpyAsync(ws + L.args, &A, sizeof(A), cudaMemcpyHostToDevice, s));
     EMUSV_CHECK(cudaMemcpyAsync(ws + L.inst, inst.data(), sizeof(BInst) * nj, cudaMemcpyHostToDevice, s));
@@ -2056,10 +2409,11 @@ static int gang_launch(int dtype, const Prepared &P, const BArgs &A, unsigned ch
     G.jrec = G.rec + 7 * (size_t)A.total_tiles;
     G.cta0 = reinterpret_cast<const int *>(ws + P.L.cta0);
     G.ncompute = P.gang;
+    G.width = P.width;
     // no record of an earlier launch carries this one's epochs
     EMUSV_CHECK(cudaMemsetAsync(G.rec, 0, sizeof(PRec) * (7 * (size_t)A.total_tiles + (size_t)GANG_JREC * A.ninst), s));
     void *args[] = {(void *)&G};
-    return cooperative_launch(pick_kernel(dtype, A.T, 4), 1, args, s, P.gang + (A.ninst + BWARPS - 1) / BWARPS,
+    return cooperative_launch(pick_kernel(dtype, A.T, 4), 1, args, s, P.gang + (A.ninst * P.width + BWARPS - 1) / BWARPS,
                               PROF_BATCH, kernel_smem(dtype, A.T, 4));
 }
 

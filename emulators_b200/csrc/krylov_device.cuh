@@ -400,12 +400,12 @@ __device__ __forceinline__ void load_rows(const KState *ks, int m, double dt, do
 // Extended exponential of iteration jj: exp of the (jj+3) x (jj+3) matrix
 // [[A, 0, 0], [l e_jj^T, 0, 0], [0, 1, 0]] (A = -i dt T_H of size jj+1, l = -i dt r_jj)
 // applied to e_0 = (y, x1, x2) (krylov_exp.py:77-78); writes the coefficients
-// c[0..jj+1] = (y, x1) and returns the Expokit error estimate (krylov_exp.py:81-84).
+// c[0..jj+1] = (y, x1) to c_re, c_im and returns the Expokit error estimate (krylov_exp.py:81-84).
 // One warp, Chebyshev form.
 // NE entries per lane: the smallest layout that holds the jj + 3 rows (the work of every
 // Chebyshev term scales with NE; each entry's arithmetic is the same in every layout).
 template <int NE>
-static __device__ __noinline__ double krylov_eval_ne(KState *ks, int jj, double dt) {
+static __device__ __noinline__ double krylov_eval_ne(const KState *ks, int jj, double dt, double *c_re, double *c_im) {
     const int lane = threadIdx.x & 31;
     const int m = jj + 1, M = m + 2;
     double2 d[NE], l[NE], u[NE], y[NE];
@@ -433,20 +433,23 @@ static __device__ __noinline__ double krylov_eval_ne(KState *ks, int jj, double 
     for (int e = 0; e < NE; ++e) {
         const int k = lane * NE + e;
         if (k <= m) {  // c[m] = x1 multiplies v_{jj+1} (krylov_exp.py:88-90)
-            ks->c_re[k] = y[e].x;
-            ks->c_im[k] = y[e].y;
+            c_re[k] = y[e].x;
+            c_im[k] = y[e].y;
         }
     }
     __syncwarp();
     return err1 < err2 ? err1 : (err1 * err2 / (err1 - err2));  // krylov_exp.py:84
 }
-static __device__ double krylov_eval(KState *ks, int jj, double dt) {
+static __device__ double krylov_eval(const KState *ks, int jj, double dt, double *c_re, double *c_im) {
     constexpr int NEMAX = (KMAX + 2 + 31) / 32;
     const int M = jj + 3;
-    if (M <= 32) return krylov_eval_ne<1>(ks, jj, dt);
-    if (M <= 64) return krylov_eval_ne<2>(ks, jj, dt);
-    if (M <= 96) return krylov_eval_ne<3>(ks, jj, dt);
-    return krylov_eval_ne<NEMAX>(ks, jj, dt);
+    if (M <= 32) return krylov_eval_ne<1>(ks, jj, dt, c_re, c_im);
+    if (M <= 64) return krylov_eval_ne<2>(ks, jj, dt, c_re, c_im);
+    if (M <= 96) return krylov_eval_ne<3>(ks, jj, dt, c_re, c_im);
+    return krylov_eval_ne<NEMAX>(ks, jj, dt, c_re, c_im);
+}
+static __device__ double krylov_eval(KState *ks, int jj, double dt) {
+    return krylov_eval(ks, jj, dt, ks->c_re, ks->c_im);
 }
 
 // Decide iteration j of a Lanczos run from the FP64 sums v = ||w_j||^2 and
