@@ -1372,6 +1372,7 @@ __device__ __noinline__ void gang_decider(const GArgs &B, int i, int sub, GDec *
             sh_put(&G->fbdone[sub], 1);
         };
         auto asked = [&] { return sh_get(&G->fb) > 0 && !sh_get(&G->fbdone[sub]); };
+        auto over = [&] { return sh_get(&G->over) == e; };
         // waits for `done` (uniform), taking the share when it is asked for; false: the launch failed
         auto wait = [&](auto done) {
             for (;;) {
@@ -1380,9 +1381,10 @@ __device__ __noinline__ void gang_decider(const GArgs &B, int i, int sub, GDec *
                 __threadfence_block();
                 if (!ask) return true;
                 share(sh_get(&G->fb));
+                // its coefficients stay until the first test's warp has chosen
+                if (!gang_until(A, [&] { return over() || sh_get(&G->fb) == 0; })) return false;
             }
         };
-        auto over = [&] { return sh_get(&G->over) == e; };
         // every iteration before j tested without an end (then true), or an earlier end
         auto stands = [&](int j, bool *alone) {
             bool all = false;
@@ -1441,6 +1443,8 @@ __device__ __noinline__ void gang_decider(const GArgs &B, int i, int sub, GDec *
                             err = *reinterpret_cast<const volatile double *>(&G->ferr[t & (W - 1)]);
                             cw = cbase + (size_t)(t & (W - 1)) * GDEC_C;
                             redo = false;
+                        } else {
+                            sh_put(&G->fb, 0);
                         }
                     }
                     if (err < A.exp_tol) st = KS_CONVERGED;
