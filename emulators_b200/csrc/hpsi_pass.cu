@@ -173,6 +173,25 @@ static int launch_high(PassParams P, int hpos, const PassArgs &A, const void *pa
     return EMUSV_OK;
 }
 
+// Rows of pass H twice (w = 1) or four times (w = 2) as wide, for as many group bits fewer: the
+// widest that still cover `bits` bits of the G that 64-byte rows take.  A pass that reads the
+// partial sums beside the values took 336 us on 64-byte rows, 280 on 128-byte and 275 on 256-byte
+// ones (three streams of 512 MB: 4.8, 5.8 and 5.9 TB/s); one that reads the values alone reaches
+// 6.5 on 64-byte rows already.
+static int wider_rows(int bits, int G) { return bits <= G - 2 ? 2 : bits <= G - 1 ? 1 : 0; }
+
+// One strided pass over the bits [top - (TB - CMIN - w), top).
+template <typename R, bool REALC, int EPI, int CMIN, bool CHUNKF = false>
+static int launch_high_rows(int w, const PassParams &P, int top, const PassArgs &A, const void *part, cudaStream_t s,
+                            int *grid_out, int hskip = PassShape<R>::TB) {
+    constexpr int G = PassShape<R>::TB - CMIN;
+    if constexpr (CMIN == PassShape<R>::CMIN) {
+        if (w == 2) return launch_high<R, REALC, EPI, CMIN + 2, CHUNKF>(P, top - G + 2, A, part, s, grid_out, hskip);
+        if (w == 1) return launch_high<R, REALC, EPI, CMIN + 1, CHUNKF>(P, top - G + 1, A, part, s, grid_out, hskip);
+    }
+    return launch_high<R, REALC, EPI, CMIN, CHUNKF>(P, top - G, A, part, s, grid_out, hskip);
+}
+
 // H v in two or three streaming passes: L (bits 0..TB-1, diagonal), then strided passes
 // over groups of G = TB - CMIN bits: the final one over the top G bits [n - G, n), and,
 // when n - TB > G, one before it over [n - 2G, n - G).  Group bits below TB (covered by
@@ -205,12 +224,13 @@ static int run_passes_c(const HamParams &H, const HpsiArgs &HA, cudaStream_t s) 
     }
     A.out = HA.part_buf;
     if ((st = launch_low<R, REALC, EPI_PARTIAL, NOISY>(P, A, s))) return st;
+    const int w = CMIN < PassShape<R>::CMIN ? 0 : wider_rows(rem > G ? (rem + 1) / 2 : rem, G);
     if (rem > G) {
-        if ((st = launch_high<R, REALC, EPI_PARTIAL, CMIN>(P, n - 2 * G, A, HA.part_buf, s, nullptr)))
+        if ((st = launch_high_rows<R, REALC, EPI_PARTIAL, CMIN>(w, P, n - (G - w), A, HA.part_buf, s, nullptr)))
             return st;
     }
     A.out = HA.out;
-    return launch_high<R, REALC, EPI_STORE, CMIN>(P, n - G, A, HA.part_buf, s, nullptr);
+    return launch_high_rows<R, REALC, EPI_STORE, CMIN>(w, P, n, A, HA.part_buf, s, nullptr);
 }
 
 // 64-byte rows (PassShape CMIN) where two H passes cover the bits above pass L, else
@@ -405,10 +425,14 @@ static int lz_high_t(const HamParams &H, const void *u, void *part, double *part
         *nblocks_out = g2;
         return EMUSV_OK;
     }
+    P.hcf = CMIN;
     if (rem > G) {
-        if ((st = launch_high<R, REALC, EPI_X_FIRST, CMIN>(P, n - 2 * G, A, nullptr, s, &g1, TBL))) return st;
+        // the second group's rows as wide as the first leaves room for
+        const int w = wider_rows(rem - G, G);
+        const int g2b = G - w;
+        if ((st = launch_high<R, REALC, EPI_X_FIRST, CMIN>(P, n - g2b - G, A, nullptr, s, &g1, TBL))) return st;
         A.partials = partials + (size_t)g1 * NRED;
-        if ((st = launch_high<R, REALC, EPI_X_ADD, CMIN, true>(P, n - G, A, part, s, &g2, TBL))) return st;
+        if ((st = launch_high_rows<R, REALC, EPI_X_ADD, CMIN, true>(w, P, n, A, part, s, &g2, TBL))) return st;
     } else {
         if ((st = launch_high<R, REALC, EPI_X_FIRST, CMIN, true>(P, n - G, A, nullptr, s, &g2, TBL)))
             return st;

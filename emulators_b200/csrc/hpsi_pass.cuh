@@ -55,6 +55,7 @@ constexpr int PBMAX_ALL = 3;  // largest cluster (2^3 CTAs) either pass uses
 struct PassParams {
     int n;
     int real_coef;
+    int hcf;  // pass H: chunk bits whose flips it applies
     // coefficients by bit position: "up" = target bit 1, "dn" = target bit 0
     float fup_re[MAXQ], fup_im[MAXQ], fdn_re[MAXQ], fdn_im[MAXQ];
     double dup_re[MAXQ], dup_im[MAXQ], ddn_re[MAXQ], ddn_im[MAXQ];
@@ -554,7 +555,7 @@ k_pass_high(const PassParams P, PassArgs A, const __grid_constant__ PassHighMaps
         cci[r] = bit ? Coef<R>::uim(P, cpos + r) : Coef<R>::dim(P, cpos + r);
     }
     // tile bits whose flips this pass applies: group bits at or above P.hskip
-    uint32_t apply = CHUNKF ? (1u << c) - 1u : 0u;
+    uint32_t apply = CHUNKF ? (1u << P.hcf) - 1u : 0u;
     for (int k = c; k < TB; ++k)
         if (hpos + k - c >= P.hskip) apply |= 1u << k;
     // coefficients of the shared-memory bits (direction fixed by the thread's own bits);
