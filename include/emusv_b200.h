@@ -128,7 +128,8 @@ size_t emusv_krylov_workspace_bytes(int nqubits, int dtype, int basis_capacity);
  * Convergence is tested on the device at every iteration, as the reference does; the
  * host reads the device's decision from iteration `krylov_dim_hint` on (0: every
  * iteration), so the hint only saves host synchronisations and never moves the stopping
- * iteration.
+ * iteration.  Registers of up to 20 qubits run the whole step in one launch and do not use
+ * the hint.
  * The workspace carries one value from call to call: the previous step's energy, which
  * the next step subtracts from H inside H*psi (same basis and coefficients; less
  * complex64 rounding of the diagonal).  Zero the workspace once before its first call.
