@@ -265,7 +265,8 @@ template <> struct LzShape<double> {
 };
 
 // The chunk bits of the pass H rows of this register (the bits the recurrence pass L
-// leaves out): 64-byte rows where two H passes cover the bits above pass L, else 32-byte.
+// leaves out): 64-byte rows where two H passes cover the bits above pass L, else 32-byte; the
+// last pass's rows may be wider (wider_rows) and then hold more bits than it applies.
 template <typename R> static int lz_chunk_bits(int n) {
     constexpr int TB = PassShape<R>::TB, CMIN = PassShape<R>::CMIN, TBL = LzShape<R>::TB;
     return n - TBL <= 2 * (TB - CMIN) ? CMIN : CMIN - 1;
