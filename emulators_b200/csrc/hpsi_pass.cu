@@ -178,25 +178,65 @@ static int launch_high(PassParams P, int hpos, const PassArgs &A, const void *pa
 // partial sums beside the values took 336 us on 64-byte rows, 280 on 128-byte and 275 on 256-byte
 // ones (three streams of 512 MB: 4.8, 5.8 and 5.9 TB/s); one that reads the values alone reaches
 // 6.5 on 64-byte rows already.
-static int wider_rows(int bits, int G) { return bits <= G - 2 ? 2 : bits <= G - 1 ? 1 : 0; }
+static constexpr int wider_rows(int bits, int G) { return bits <= G - 2 ? 2 : bits <= G - 1 ? 1 : 0; }
 
-// One strided pass over the bits [top - (TB - CMIN - w), top).
-template <typename R, bool REALC, int EPI, int CMIN, bool CHUNKF = false>
-static int launch_high_rows(int w, const PassParams &P, int top, const PassArgs &A, const void *part, cudaStream_t s,
-                            int *grid_out, int hskip = PassShape<R>::TB) {
-    constexpr int G = PassShape<R>::TB - CMIN;
-    if constexpr (CMIN == PassShape<R>::CMIN) {
-        if (w == 2) return launch_high<R, REALC, EPI, CMIN + 2, CHUNKF>(P, top - G + 2, A, part, s, grid_out, hskip);
-        if (w == 1) return launch_high<R, REALC, EPI, CMIN + 1, CHUNKF>(P, top - G + 1, A, part, s, grid_out, hskip);
+// The strided passes over the bits [skip, n), in launch order: pass k takes the rows of width
+// w[k] and the bits [top[k] - (G - w[k]), top[k]), and leaves out those below skip.  Only 64-byte
+// rows (rows64) come wider.  With `both`, all passes share the width; else only the second of two,
+// which reads the partial sums, is wider.
+struct RowPlan {
+    int passes, top[2], w[2];
+};
+static constexpr RowPlan row_plan(int n, int skip, int G, bool rows64, bool both) {
+    const int bits = n - skip;
+    RowPlan p = {};
+    p.passes = bits > G ? 2 : 1;
+    const int last = p.passes - 1;
+    if (rows64 && both) {
+        p.w[0] = p.w[last] = wider_rows(p.passes == 2 ? (bits + 1) / 2 : bits, G);
+    } else if (rows64 && p.passes == 2) {
+        p.w[1] = wider_rows(bits - G, G);
     }
-    return launch_high<R, REALC, EPI, CMIN, CHUNKF>(P, top - G, A, part, s, grid_out, hskip);
+    p.top[last] = n;
+    if (p.passes == 2) p.top[0] = n - (G - p.w[1]);
+    return p;
+}
+// Does every register up to EMUSV_MAX_QUBITS have each bit from skip on in exactly one pass, and
+// no pass below its rows?
+static constexpr bool row_plans_cover(int tb, int cmin, int skip, bool both) {
+    for (int n = skip + 1; n <= EMUSV_MAX_QUBITS; ++n) {
+        const bool rows64 = n - skip <= 2 * (tb - cmin);
+        const int c = rows64 ? cmin : cmin - 1, G = tb - c;
+        const RowPlan p = row_plan(n, skip, G, rows64, both);
+        if (n - skip > 2 * G) return false;
+        for (int k = 0; k < p.passes; ++k)
+            if (p.top[k] - (G - p.w[k]) < c + p.w[k]) return false;
+        for (int bit = skip; bit < n; ++bit) {
+            int times = 0;
+            for (int k = 0; k < p.passes; ++k) times += bit < p.top[k] && bit >= p.top[k] - (G - p.w[k]);
+            if (times != 1) return false;
+        }
+    }
+    return true;
+}
+
+// Pass k of a plan.
+template <typename R, bool REALC, int EPI, int CMIN, bool CHUNKF = false>
+static int launch_high_rows(const RowPlan &plan, int k, const PassParams &P, const PassArgs &A, const void *part,
+                            cudaStream_t s, int *grid_out, int hskip = PassShape<R>::TB) {
+    constexpr int G = PassShape<R>::TB - CMIN;
+    const int w = plan.w[k], lo = plan.top[k] - (G - w);
+    if constexpr (CMIN == PassShape<R>::CMIN) {
+        if (w == 2) return launch_high<R, REALC, EPI, CMIN + 2, CHUNKF>(P, lo, A, part, s, grid_out, hskip);
+        if (w == 1) return launch_high<R, REALC, EPI, CMIN + 1, CHUNKF>(P, lo, A, part, s, grid_out, hskip);
+    }
+    if (w) return EMUSV_BAD_ARGUMENT;
+    return launch_high<R, REALC, EPI, CMIN, CHUNKF>(P, lo, A, part, s, grid_out, hskip);
 }
 
 // H v in two or three streaming passes: L (bits 0..TB-1, diagonal), then strided passes
-// over groups of G = TB - CMIN bits: the final one over the top G bits [n - G, n), and,
-// when n - TB > G, one before it over [n - 2G, n - G).  Group bits below TB (covered by
-// pass L) are skipped, so every H pass keeps the compile-time chunk of CMIN bits.  The
-// partial sums live in HA.part_buf (which may be HA.out: every pass reads a tile before
+// over groups of at most G = TB - CMIN bits (row_plan).  Group bits below TB (covered by
+// pass L) are skipped, so every H pass keeps a compile-time chunk.  The partial sums live in HA.part_buf (which may be HA.out: every pass reads a tile before
 // writing it).
 template <typename R, bool REALC, int CMIN, bool NOISY>
 static int run_passes_c(const HamParams &H, const HpsiArgs &HA, cudaStream_t s) {
@@ -224,13 +264,13 @@ static int run_passes_c(const HamParams &H, const HpsiArgs &HA, cudaStream_t s) 
     }
     A.out = HA.part_buf;
     if ((st = launch_low<R, REALC, EPI_PARTIAL, NOISY>(P, A, s))) return st;
-    const int w = CMIN < PassShape<R>::CMIN ? 0 : wider_rows(rem > G ? (rem + 1) / 2 : rem, G);
-    if (rem > G) {
-        if ((st = launch_high_rows<R, REALC, EPI_PARTIAL, CMIN>(w, P, n - (G - w), A, HA.part_buf, s, nullptr)))
-            return st;
+    static_assert(row_plans_cover(TB, PassShape<R>::CMIN, TB, true), "each bit above pass L in one pass");
+    const RowPlan plan = row_plan(n, TB, G, CMIN == PassShape<R>::CMIN, true);
+    if (plan.passes == 2) {
+        if ((st = launch_high_rows<R, REALC, EPI_PARTIAL, CMIN>(plan, 0, P, A, HA.part_buf, s, nullptr))) return st;
     }
     A.out = HA.out;
-    return launch_high_rows<R, REALC, EPI_STORE, CMIN>(w, P, n, A, HA.part_buf, s, nullptr);
+    return launch_high_rows<R, REALC, EPI_STORE, CMIN>(plan, plan.passes - 1, P, A, HA.part_buf, s, nullptr);
 }
 
 // 64-byte rows (PassShape CMIN) where two H passes cover the bits above pass L, else
@@ -427,15 +467,14 @@ static int lz_high_t(const HamParams &H, const void *u, void *part, double *part
         return EMUSV_OK;
     }
     P.hcf = CMIN;
-    if (rem > G) {
-        // the second group's rows as wide as the first leaves room for
-        const int w = wider_rows(rem - G, G);
-        const int g2b = G - w;
-        if ((st = launch_high<R, REALC, EPI_X_FIRST, CMIN>(P, n - g2b - G, A, nullptr, s, &g1, TBL))) return st;
+    static_assert(row_plans_cover(TB, PassShape<R>::CMIN, TBL, false), "each bit above the tile in one pass");
+    const RowPlan plan = row_plan(n, TBL, G, CMIN == PassShape<R>::CMIN, false);
+    if (plan.passes == 2) {
+        if ((st = launch_high<R, REALC, EPI_X_FIRST, CMIN>(P, plan.top[0] - G, A, nullptr, s, &g1, TBL))) return st;
         A.partials = partials + (size_t)g1 * NRED;
-        if ((st = launch_high_rows<R, REALC, EPI_X_ADD, CMIN, true>(w, P, n, A, part, s, &g2, TBL))) return st;
+        if ((st = launch_high_rows<R, REALC, EPI_X_ADD, CMIN, true>(plan, 1, P, A, part, s, &g2, TBL))) return st;
     } else {
-        if ((st = launch_high<R, REALC, EPI_X_FIRST, CMIN, true>(P, n - G, A, nullptr, s, &g2, TBL)))
+        if ((st = launch_high<R, REALC, EPI_X_FIRST, CMIN, true>(P, plan.top[0] - G, A, nullptr, s, &g2, TBL)))
             return st;
     }
     *nblocks_out = g1 + g2;
