@@ -201,8 +201,8 @@ static constexpr RowPlan row_plan(int n, int skip, int G, bool rows64, bool both
     if (p.passes == 2) p.top[0] = n - (G - p.w[1]);
     return p;
 }
-// Does every register up to EMUSV_MAX_QUBITS have each bit from skip on in exactly one pass, and
-// no pass below its rows?
+// Does every register up to EMUSV_MAX_QUBITS have each bit from skip on in exactly one pass, no
+// pass below its rows and no wider 32-byte rows?
 static constexpr bool row_plans_cover(int tb, int cmin, int skip, bool both) {
     for (int n = skip + 1; n <= EMUSV_MAX_QUBITS; ++n) {
         const bool rows64 = n - skip <= 2 * (tb - cmin);
@@ -210,7 +210,7 @@ static constexpr bool row_plans_cover(int tb, int cmin, int skip, bool both) {
         const RowPlan p = row_plan(n, skip, G, rows64, both);
         if (n - skip > 2 * G) return false;
         for (int k = 0; k < p.passes; ++k)
-            if (p.top[k] - (G - p.w[k]) < c + p.w[k]) return false;
+            if ((p.w[k] && !rows64) || p.top[k] - (G - p.w[k]) < c + p.w[k]) return false;
         for (int bit = skip; bit < n; ++bit) {
             int times = 0;
             for (int k = 0; k < p.passes; ++k) times += bit < p.top[k] && bit >= p.top[k] - (G - p.w[k]);
