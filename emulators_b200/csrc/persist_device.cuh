@@ -273,7 +273,7 @@ __device__ __noinline__ void p_conclude(const PRun &A, PShared<CT> &sh, int j) {
         }
         if (ext) extend_rows<NE>(m, sh.r[j], A.dt, l);
         cheb_expm_real<NE>(d, l, u, -1, 0.0, 0, A.dt, ext ? m + 2 : m, y, &sh.done);
-        if (sh.done) return;
+        if (__any_sync(0xffffffffu, sh.done)) return;
         if (ext) err = expokit_error<NE>(y, m, A.dt, sqrt(fmax(0.0, sh.hn2[j])));
     }
     int st = KS_RUNNING, nvec = j + 2;

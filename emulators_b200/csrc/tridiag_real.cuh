@@ -86,7 +86,8 @@ static __device__ void cheb_expm_real(const double (&d)[NE], const double (&l)[N
     double jk1 = 0.0, jk = 1e-280, S = 0.0;  // J~_{k+1}, J~_k, normalisation sum
     double kd = K;                           // k
     for (int k = K; k >= 1; --k, kd -= 1.0) {
-        if (abandon && (k & 7) == 0 && *abandon) return;
+        // the whole warp or none of it: another warp may set the word between two lanes' loads
+        if (abandon && (k & 7) == 0 && __any_sync(0xffffffffu, *abandon)) return;
         if ((k & 1) == 0) S += 2.0 * jk;
         if (k <= N) {  // b_k = 2 (-i sgn)^k J~_k e_col + 2 X b_{k+1} - b_{k+2}
             double xr[NE], xi[NE];
