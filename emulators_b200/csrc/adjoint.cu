@@ -333,6 +333,8 @@ int emusv_adjoint_step(int nqubits, int dtype, double dt, const double *omegas,
                          tolerance, max_krylov_dim, 0, false, s, &run);
         if (st || (st = read_heads(ks2, 2, s, h))) return st;
     }
+    for (const KHead &k : h)
+        if (k.status == KS_TIMEOUT) return EMUSV_TIMEOUT;  // the norms below may be missing
     const double s0[2] = {h[0].s0, h[1].s0};
     if (s0[0] == 0.0 || s0[1] == 0.0) {  // a zero state or gradient: dU|s><g| = 0
         for (int i = 0; i < n; ++i) {
@@ -346,7 +348,6 @@ int emusv_adjoint_step(int nqubits, int dtype, double dt, const double *omegas,
     for (const KHead &k : h) {
         if (k.status == KS_RUNNING) return EMUSV_WORKSPACE_TOO_SMALL;
         if (k.status == KS_MAXDIM) return EMUSV_NOT_CONVERGED;  // double_krylov.py:107-110
-        if (k.status == KS_TIMEOUT) return EMUSV_TIMEOUT;
         if (k.status != KS_CONVERGED && k.status != KS_HAPPY) return EMUSV_NONFINITE;
     }
     // size of the gradient basis (the dS columns)

@@ -652,6 +652,11 @@ int emusv_krylov_step(int nqubits, int dtype, double dt, const double *omegas,
     return h.status == KS_MAXDIM ? EMUSV_NOT_CONVERGED : EMUSV_OK;
 }
 
+int emusv_krylov_set_wait_test(long long wait_cycles, int withhold) {
+    persist_set_wait_test(wait_cycles, withhold);
+    return EMUSV_OK;
+}
+
 int emusv_vec_dot(int64_t len, int dtype, const void *a, const void *b, double *res_dev,
                   void *scratch, size_t scratch_bytes, void *stream) {
     if (len < 1 || !a || !b || !res_dev || !scratch ||

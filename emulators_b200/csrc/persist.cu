@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(CT + 32 * ND, 1) k_lanczos_persist(const __gri
         sh.ready = 0;
         sh.done = 0;
         sh.dead = 0;
+        sh.lost = 0;
         mbar_init_count(&sh.bar, CL ? 3 * G : 3 << PGC_BITS);
         // sigma from the previous finished run (read before anyone overwrites the state)
         double sg = 0.0;
@@ -56,7 +57,7 @@ __global__ void __launch_bounds__(CT + 32 * ND, 1) k_lanczos_persist(const __gri
     for (int k = tid; k < KMAX; k += blockDim.x) sh.result[k] = 0;
     __syncthreads();
     cl_sync_all();  // mbarriers and flags are set before a sibling touches them
-    const PRun run = {ks, X, A.epoch, A.gbits, A.limit, A.maxdim, A.dt, A.exp_tol, PWAIT_LIMIT};
+    const PRun run = {ks, X, A.epoch, A.gbits, A.limit, A.maxdim, A.dt, A.exp_tol, A.wait};
     if constexpr (CL) {
         if (tid >= CT) {
             p_decider<CT, CL>(run, sh, r + (((tid - CT) >> 5) << A.gbits), ND << A.gbits);
@@ -115,8 +116,11 @@ __global__ void __launch_bounds__(CT + 32 * ND, 1) k_lanczos_persist(const __gri
     }
     uint32_t parity = 0;
     bool stop = false;
+    // failure-path test: this CTA's sums stay out, so its siblings' waits for them run out, and in
+    // its end its own wait for the verdict
+    const bool mute = A.withhold && jb == 0 && r == G - 1;
     // every CTA has read the previous state once this exchange is complete
-    bool ok = p_exchange<CT, CL, 1, false>(sh, acc, X, A.epoch, r, A.gbits, parity, false, &stop);
+    bool ok = mute || p_exchange<CT, CL, 1, false>(sh, acc, X, A.epoch, r, A.gbits, parity, false, &stop, A.wait);
     const double s0 = sqrt(acc[0]);  // krylov_exp.py:43
     const bool fine = isfinite(s0) && s0 > 0.0;
     double sj = 1.0 / s0, sp = 0.0, b = 0.0, vvr = 0.0, vvi = 0.0;
@@ -127,12 +131,13 @@ __global__ void __launch_bounds__(CT + 32 * ND, 1) k_lanczos_persist(const __gri
             ks->shift = sigma;
             ks->outnorm2 = 0.0;
             ks->kerr = 0;
+            ks->status = KS_RUNNING;
             if (!CL) {
                 rec_put(&X->start[0], sigma, A.epoch);
                 rec_put(&X->start[1], sj, A.epoch);
             }
         }
-        if (!fine) {  // decided as iteration 0
+        if (!fine && !mute) {  // decided as iteration 0
             sh.ar[0] = sh.ai[0] = sh.r[0] = sh.hn2[0] = 0.0;
             sh.scale[1] = 0.0;
             sh.flag[0] = KD_NONFINITE;
@@ -141,8 +146,8 @@ __global__ void __launch_bounds__(CT + 32 * ND, 1) k_lanczos_persist(const __gri
         }
     }
     const unsigned long long e0 = A.epoch + 1;
-    if (!CL && !fine && r == 0 && tid < 5) rec_put(&X->iter[0][tid], tid == 4 ? (double)KD_NONFINITE : 0.0, e0);
-    for (int j = 0; fine && ok && !stop && j < A.limit; ++j) {
+    if (!CL && !fine && !mute && r == 0 && tid < 5) rec_put(&X->iter[0][tid], tid == 4 ? (double)KD_NONFINITE : 0.0, e0);
+    for (int j = 0; fine && ok && !mute && !stop && j < A.limit; ++j) {
         // grid jobs: CTA 0 looks whether the run is decided, meanwhile
         PRec vd;
         vd.e = 0;
@@ -233,7 +238,7 @@ __global__ void __launch_bounds__(CT + 32 * ND, 1) k_lanczos_persist(const __gri
             for (int a = 0; a < NA; ++a) vp[a] = j > 0 ? __ldcg(up + tid + a * CT) : zero;
         }
         bool dummy;
-        ok = p_exchange<CT, CL, 0, false>(sh, acc, X, e0 + 2 * j, r, A.gbits, parity, false, &dummy);
+        ok = p_exchange<CT, CL, 0, false>(sh, acc, X, e0 + 2 * j, r, A.gbits, parity, false, &dummy, A.wait);
         if (!ok) break;
         // ---------------- B: w = h - a v_j - b v_{j-1}
         const double are = acc[0] - b * vvr, aim = acc[1] - b * vvi;
@@ -272,7 +277,7 @@ __global__ void __launch_bounds__(CT + 32 * ND, 1) k_lanczos_persist(const __gri
         acc[2] *= sj;
         if (!CL && r == 0 && tid == CT - 1 && vd.e == A.epoch) sh.done = (int)vd.v + 1;
         ok = p_exchange<CT, CL, 1, true>(sh, acc, X, e0 + 2 * j + 1, r, A.gbits, parity,
-                                         r == 0 && tid == 0 && sh.done, &stop);
+                                         r == 0 && tid == 0 && sh.done, &stop, A.wait);
         if (!ok) break;
         const double rj = sqrt(acc[0]), inv = 1.0 / rj;
         int flag = KD_OK;
@@ -304,14 +309,17 @@ __global__ void __launch_bounds__(CT + 32 * ND, 1) k_lanczos_persist(const __gri
     if (tid == 0) {
         const long long t0 = clock64();
         while (ok && !p_decided<CT, CL>(sh, X, A.epoch))
-            if (clock64() - t0 > PWAIT_LIMIT) sh.dead = 1;
-        if (!ok) sh.dead = 1;
-        if (sh.dead) atomicExch(&ks->kerr, (int)EMUSV_TIMEOUT);
+            if (clock64() - t0 > A.wait) ok = false;
+        sh.verdict = ok ? sh.done : 0;  // not decided: a deciding warp gave up
+        if (!sh.verdict) {
+            sh.dead = 1;
+            atomicExch(&ks->kerr, (int)EMUSV_TIMEOUT);
+        }
         __threadfence();
     }
     compute_sync<CT>();
-    const int st = sh.done - 1;
-    if (!sh.dead && J.out && (st == KS_CONVERGED || st == KS_HAPPY || st == KS_MAXDIM)) {
+    const int st = sh.verdict - 1;
+    if (J.out && (st == KS_CONVERGED || st == KS_HAPPY || st == KS_MAXDIM)) {
         const int nv = __ldcg(&ks->nvec);
         for (int k = tid; k < nv; k += CT) {
             const double f = s0 * sh.scale[k];
@@ -356,7 +364,8 @@ __global__ void __launch_bounds__(CT + 32 * ND, 1) k_lanczos_persist(const __gri
                 acc[0] += double(o.x) * double(o.x) + double(o.y) * double(o.y);
             }
         }
-        ok = p_exchange<CT, CL, 0, false>(sh, acc, X, A.epoch + 4 * KMAX - 1, r, A.gbits, parity, false, &stop);
+        ok = p_exchange<CT, CL, 0, false>(sh, acc, X, A.epoch + 4 * KMAX - 1, r, A.gbits, parity, false, &stop,
+                                           A.wait);
         if (r == 0 && tid == 0) {
             ks->outnorm2 = acc[0];
             if (!ok) atomicExch(&ks->kerr, (int)EMUSV_TIMEOUT);
@@ -428,6 +437,14 @@ bool persist_applies(int dtype, int n) {
 }
 size_t persist_exchange_bytes() { return (sizeof(PExchange) + 255) / 256 * 256; }
 
+// Failure-path test switch of the calling thread (emusv_krylov_set_wait_test).
+static thread_local long long tl_wait = PWAIT_LIMIT;
+static thread_local int tl_withhold = 0;
+void persist_set_wait_test(long long wait_cycles, int withhold) {
+    tl_wait = wait_cycles > 0 ? wait_cycles : PWAIT_LIMIT;
+    tl_withhold = withhold ? 1 : 0;
+}
+
 // Epochs of a launch: 4 KMAX consecutive values that no other launch uses.
 static unsigned long long next_epoch() {
     static std::atomic<unsigned long long> next{
@@ -469,6 +486,8 @@ int persist_launch(const HamParams &P, int dtype, double dt, const PJob *jobs, i
     A.dt = dt;
     A.exp_tol = exp_tol;
     A.norm_tol = norm_tol;
+    A.wait = tl_wait;
+    A.withhold = tl_withhold;
     const size_t smem = persist_smem(sh, dtype);
     void *kern = dtype == EMUSV_C128 ? (P.real_coef ? pick<double, true>(sh) : pick<double, false>(sh))
                                      : (P.real_coef ? pick<float, true>(sh) : pick<float, false>(sh));

@@ -30,8 +30,9 @@
 // CTA, 1.5-1.8 in a cluster, 3.1-3.8 through the L2 with 32 clusters of four (4.9-6.4 when 128
 // CTAs read each other's records).
 //
-// Every wait is bounded (about 2 s of SM clock): on a timeout the CTA records EMUSV_TIMEOUT in
-// the run's state and the job's CTAs return.
+// Every wait is bounded (PArgs::wait): on a timeout the CTA records EMUSV_TIMEOUT in the run's state
+// and the job's CTAs return.  Whether a wait ran out is decided by the warps that wait and handed
+// to the CTA through a barrier, so its threads always leave together.
 #pragma once
 
 #include "krylov_device.cuh"
@@ -42,7 +43,7 @@ constexpr int PMAXG_BITS = 7;      // CTAs per job: at most 128
 constexpr int PMAXG = 1 << PMAXG_BITS;
 constexpr int PCL_BITS = 4;        // CTAs of a cluster job: at most 16
 constexpr int PGC_BITS = 2;        // CTAs per cluster of a grid job: 4 (33 such clusters fit the GPU)
-constexpr long long PWAIT_LIMIT = 4000000000LL;  // SM clock cycles a wait lasts at most
+constexpr long long PWAIT_LIMIT = 4000000000LL;  // SM clock cycles a wait lasts at most (about 2 s)
 
 struct __align__(16) PRec {  // written and read as one 16-byte access
     double v;
@@ -74,11 +75,14 @@ struct PArgs {
     int limit, maxdim;       // iterations computed at most (basis slots), max_krylov_dim
     double dt, exp_tol, norm_tol;
     unsigned long long epoch;  // the launch's first epoch
+    long long wait;            // clock cycles a wait lasts at most
+    int withhold;              // failure-path test: the last CTA of job 0 sends no sums
 };
 
 // Host side (persist.cu).
 bool persist_applies(int dtype, int n);
 size_t persist_exchange_bytes();
+void persist_set_wait_test(long long wait_cycles, int withhold);
 // Runs 1 or 2 jobs of the same operator; the caller reads their states afterwards.
 int persist_launch(const HamParams &P, int dtype, double dt, const PJob *jobs, int njobs, int capacity,
                    double exp_tol, double norm_tol, int maxdim, cudaStream_t s);

@@ -32,14 +32,14 @@ constexpr unsigned long long PSTOP = 1ull << 63;  // epoch flag: the run was dec
 
 // Waits until the record carries the epoch; false on a timeout.
 template <bool ACQUIRE = false>
-__device__ __forceinline__ bool rec_wait(const PRec *r, unsigned long long e, PRec *o) {
+__device__ __forceinline__ bool rec_wait(const PRec *r, unsigned long long e, PRec *o, long long limit) {
     *o = rec_get<ACQUIRE>(r);
     if ((o->e & ~PSTOP) == e) return true;
     const long long t0 = clock64();
     for (unsigned i = 1;; ++i) {
         *o = rec_get<ACQUIRE>(r);
         if ((o->e & ~PSTOP) == e) return true;
-        if ((i & 255u) == 0 && clock64() - t0 > PWAIT_LIMIT) return false;
+        if ((i & 255u) == 0 && clock64() - t0 > limit) return false;
     }
 }
 
@@ -78,7 +78,7 @@ __device__ __forceinline__ void mbar_init_count(uint64_t *bar, uint32_t count) {
 __device__ __forceinline__ void cl_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ bool cl_wait(uint64_t *bar, uint32_t parity, long long limit = PWAIT_LIMIT) {
+__device__ __forceinline__ bool cl_wait(uint64_t *bar, uint32_t parity, long long limit) {
     const long long t0 = clock64();
     for (unsigned i = 1;; ++i) {
         uint32_t ok;
@@ -97,7 +97,7 @@ __device__ __forceinline__ void cl_sync_all() {
 template <int CT> struct PShared {
     double red[2][CT / 32][3];      // the warps' sums, alternating between exchanges
     double xs[2][3][1 << PCL_BITS]; // the cluster's CTAs' sums of phases A and B
-    double part[3];                 // grid jobs: the sums
+    double part[3];                 // the job's sums of the last exchange
     double up_re[MAXQ], up_im[MAXQ], field[MAXQ];
     double U[MAXQ * MAXQ];
     // the run's scalars, every CTA's own copy
@@ -110,6 +110,9 @@ template <int CT> struct PShared {
     volatile int ready;             // iterations whose scalars are here
     volatile int done;              // the run's status + 1 once it is decided
     volatile int dead;              // a wait of this CTA ran out
+    int lost;                       // a wait for the job's sums ran out (set by the warps that wait,
+                                    // read by the compute warps after the exchange's barrier)
+    int verdict;                    // `done` as the compute warps act on it, 0 after a timeout
     int fin[2];
     double sigma;
 };
@@ -120,11 +123,10 @@ template <int CT> __device__ __forceinline__ void compute_sync() {  // the compu
 
 // The sums of v[0..2] over the job's compute threads, in every thread, in a fixed order; a
 // barrier of the job (ordering global stores before it for grid jobs when PUBLISH).  PH 0:
-// phase A, 1: phase B.  *stop: CTA 0's flag.  False on a timeout.
+// phase A, 1: phase B.  *stop: CTA 0's flag.  False, in every thread of the CTA alike, on a timeout.
 template <int CT, bool CL, int PH, bool PUBLISH>
 __device__ __forceinline__ bool p_exchange(PShared<CT> &sh, double (&v)[3], PExchange *X, unsigned long long e, int r,
-                                           int gbits, uint32_t &parity, bool stop_in, bool *stop,
-                                           long long wait = PWAIT_LIMIT) {
+                                           int gbits, uint32_t &parity, bool stop_in, bool *stop, long long wait) {
     constexpr int NW = CT / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, G = 1 << gbits;
 #pragma unroll
@@ -155,25 +157,22 @@ __device__ __forceinline__ bool p_exchange(PShared<CT> &sh, double (&v)[3], PExc
         return true;
     }
     if constexpr (CL) {
-        // every CTA receives every CTA's sums (and CTA 0's flag), then the phase completes
+        // every CTA receives every CTA's sums (and CTA 0's flag), then the phase completes; one warp
+        // per sum waits for it
         const int fin = __shfl_sync(0xffffffffu, (int)stop_in, 0);
-        if (warp < 3 && lane < G) {
-            cl_st(cl_addr(&sh.xs[PH][warp][r], lane), block_total(warp));
-            if (warp == 0 && r == 0)
-                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cl_addr(&sh.fin[PH], lane)), "r"(fin)
-                             : "memory");
-            cl_arrive(cl_addr(&sh.bar, lane));
-        }
-        const bool ok = cl_wait(&sh.bar, parity, wait);
-        parity ^= 1u;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
+        if (warp < 3) {
+            if (lane < G) {
+                cl_st(cl_addr(&sh.xs[PH][warp][r], lane), block_total(warp));
+                if (warp == 0 && r == 0)
+                    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cl_addr(&sh.fin[PH], lane)), "r"(fin)
+                                 : "memory");
+                cl_arrive(cl_addr(&sh.bar, lane));
+            }
+            if (!cl_wait(&sh.bar, parity, wait)) sh.lost = 1;
             double t = 0.0;
-            for (int g = 0; g < G; g += 2) t += sh.xs[PH][k][g] + sh.xs[PH][k][g + 1];
-            v[k] = t;
+            for (int g = 0; g < G; g += 2) t += sh.xs[PH][warp][g] + sh.xs[PH][warp][g + 1];
+            if (lane == 0) sh.part[warp] = t;
         }
-        *stop = sh.fin[PH] != 0;
-        return ok;
     } else {
         // clusters of PGC CTAs first: their sums meet in the cluster's first CTA, which writes
         // the cluster's records; every CTA reads all clusters' records, one a lane
@@ -187,32 +186,32 @@ __device__ __forceinline__ bool p_exchange(PShared<CT> &sh, double (&v)[3], PExc
             }
             bool ok = true;
             if ((r & (PGC - 1)) == 0 && lane == 0) {
-                ok = cl_wait(&sh.bar, parity);
+                ok = cl_wait(&sh.bar, parity, wait);
                 double t = 0.0;
 #pragma unroll
                 for (int g = 0; g < PGC; ++g) t += sh.xs[PH][warp][g];
                 if (PUBLISH) __threadfence();  // the cluster's stores before its record
-                rec_put(&recs[warp][r >> PGC_BITS], t, e | (stop_in ? PSTOP : 0ull));
+                if (ok) rec_put(&recs[warp][r >> PGC_BITS], t, e | (stop_in ? PSTOP : 0ull));
             }
             __syncwarp();
             double t = 0.0;
             if (lane < (G >> PGC_BITS)) {
                 PRec o;
-                ok = rec_wait<PUBLISH>(&recs[warp][lane], e, &o) && ok;
+                ok = rec_wait<PUBLISH>(&recs[warp][lane], e, &o, wait) && ok;
                 t = o.v;
                 if (warp == 0 && lane == 0) sh.fin[PH] = (o.e & PSTOP) != 0;
             }
             t = warp_sum(t);
             if (lane == 0) sh.part[warp] = t;
-            if (!ok) sh.dead = 1;
+            if (!ok) sh.lost = 1;
         }
-        parity ^= 1u;
-        compute_sync<CT>();
-#pragma unroll
-        for (int k = 0; k < 3; ++k) v[k] = sh.part[k];
-        *stop = sh.fin[PH] != 0;
-        return sh.dead == 0;
     }
+    parity ^= 1u;
+    compute_sync<CT>();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[k] = sh.part[k];
+    *stop = sh.fin[PH] != 0;
+    return sh.lost == 0;
 }
 
 // ------------------------------------------------------------------ decisions

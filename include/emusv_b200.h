@@ -144,6 +144,14 @@ int emusv_krylov_step(int nqubits, int dtype, double dt, const double *omegas,
                       void *workspace, size_t workspace_bytes, emusv_krylov_info *info,
                       void *stream);
 
+/* Failure-path test switch of the calling thread's one-launch runs (emusv_krylov_step and
+ * emusv_adjoint_step, registers of up to 20 qubits; no counterpart in the reference, whose loop has
+ * no device-side waits): their waits last at most wait_cycles SM clock cycles (<= 0 restores the
+ * default, about 2 s), and with withhold != 0 one CTA never sends its sums, so every wait for them
+ * runs out, all CTAs return and the call gives EMUSV_TIMEOUT; the device stays usable.  Off by
+ * default; for tests.  Host-side only (takes effect at the next call). */
+int emusv_krylov_set_wait_test(long long wait_cycles, int withhold);
+
 /* Bytes of device workspace emusv_adjoint_step needs when each of its two Lanczos bases
  * may hold `basis_capacity` vectors (3 * (capacity + 1) + 1 vectors of 2^n amplitudes
  * plus small tables); 0 for registers above 20 qubits. */
