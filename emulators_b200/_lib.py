@@ -48,6 +48,7 @@ SIGNATURES: dict[str, tuple] = {
     "emusv_krylov_step": (_I, [_I, _I, _D, _P, _P, _P, _P, _P, _P, _D, _D, _I, _I, _P, _SZ,
                                ctypes.POINTER(KrylovInfo), _P]),
     "emusv_krylov_set_wait_test": (_I, [ctypes.c_longlong, _I]),
+    "emusv_krylov_set_streaming": (_I, [_I]),
     "emusv_adjoint_workspace_bytes": (_SZ, [_I, _I, _I]),
     "emusv_adjoint_step": (_I, [_I, _I, _D, _P, _P, _P, _P, _P, _P, _D, _I, _P, _P, _P, _P, _P, _SZ,
                                 _P]),

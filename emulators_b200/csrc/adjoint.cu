@@ -317,7 +317,7 @@ int emusv_adjoint_step(int nqubits, int dtype, double dt, const double *omegas,
     int st;
     KHead h[2];
     KState *const ks2[2] = {W.ks_s, W.ks_g};
-    if (persist_applies(dtype, n)) {  // both in one launch, side by side where they fit
+    if (persist_applies(P, dtype)) {  // both in one launch, side by side where they fit
         const PJob jobs[2] = {{state, nullptr, W.ks_s, W.x_s, W.basis_s, 0},
                               {grad_out, nullptr, W.ks_g, W.x_g, W.basis_g, 0}};
         st = persist_launch(P, dtype, dt, jobs, 2, W.capacity, tolerance, tolerance, max_krylov_dim, s);

@@ -627,7 +627,7 @@ int emusv_krylov_step(int nqubits, int dtype, double dt, const double *omegas,
     if (capacity < 1) return EMUSV_WORKSPACE_TOO_SMALL;
 
     KHead h;
-    if (persist_applies(dtype, nqubits)) {  // the whole step in one launch
+    if (persist_applies(P, dtype)) {  // the whole step in one launch
         const PJob job = {psi_in, psi_out, W.ks, W.x, W.basis, 1};
         int st = persist_launch(P, dtype, dt, &job, 1, capacity, exp_tolerance, norm_tolerance, max_krylov_dim, s);
         if (st || (st = read_heads(&W.ks, 1, s, &h))) return st;
@@ -654,6 +654,11 @@ int emusv_krylov_step(int nqubits, int dtype, double dt, const double *omegas,
 
 int emusv_krylov_set_wait_test(long long wait_cycles, int withhold) {
     persist_set_wait_test(wait_cycles, withhold);
+    return EMUSV_OK;
+}
+
+int emusv_krylov_set_streaming(int on) {
+    persist_set_streaming(on);
     return EMUSV_OK;
 }
 

@@ -403,37 +403,84 @@ static PShape persist_shape(int n, int njobs) {
     s.na_bits = s.tbits > lb ? s.tbits - lb : 0;
     return s;
 }
-// Clusters of a grid job that the current device holds at once (a CTA per SM).
-static int grid_clusters() {
-    static std::atomic<int> cached[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    int n = cached[dev].load();
-    if (n) return n;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1 << PGC_BITS);
-    cfg.blockDim = dim3(GCT);
-    cfg.dynamicSmemBytes = 0;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1 << PGC_BITS;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, k_lanczos_persist<double, true, 1, GCT, 0, false>, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        n = 0;
-    }
-    cached[dev].store(n);
-    return n;
+template <typename R, bool REALC, int NA>
+static void *pick_na(bool cluster) {
+    return cluster ? reinterpret_cast<void *>(k_lanczos_persist<R, REALC, NA, CCT, CND, true>)
+                   : reinterpret_cast<void *>(k_lanczos_persist<R, REALC, NA, GCT, 0, false>);
 }
-static bool shape_fits(const PShape &s, int dtype, int njobs) {
-    return s.na_bits <= 4 && persist_smem(s, dtype) <= 200 * 1024 &&
-           (s.cluster || (njobs << s.gbits >> PGC_BITS) + 1 <= grid_clusters());
+template <typename R, bool REALC>
+static void *pick(const PShape &s) {
+    switch (s.na_bits) {
+    case 0: return pick_na<R, REALC, 1>(s.cluster);
+    case 1: return pick_na<R, REALC, 2>(s.cluster);
+    case 2: return pick_na<R, REALC, 4>(s.cluster);
+    case 3: return pick_na<R, REALC, 8>(s.cluster);
+    default: return pick_na<R, REALC, 16>(s.cluster);
+    }
 }
 
-bool persist_applies(int dtype, int n) {
-    return n >= 1 && (dtype == EMUSV_C128 || dtype == EMUSV_C64) && shape_fits(persist_shape(n, 1), dtype, 1);
+static void *pick(const PShape &s, int dtype, bool realc) {
+    return dtype == EMUSV_C128 ? (realc ? pick<double, true>(s) : pick<double, false>(s))
+                               : (realc ? pick<float, true>(s) : pick<float, false>(s));
+}
+static cudaError_t set_attributes(void *kern, const PShape &s, size_t smem) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess || !s.cluster || s.gbits <= 3) return e;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+static void fill_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute (&attr)[2], const PShape &s, int njobs,
+                        size_t smem) {
+    *cfg = {};
+    cfg->gridDim = dim3((njobs << s.gbits) + (s.cluster ? 0 : 1 << PGC_BITS));
+    cfg->blockDim = dim3(s.cluster ? CCT + 32 * CND : GCT);
+    cfg->dynamicSmemBytes = smem;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1u << (s.cluster ? s.gbits : PGC_BITS);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeCooperative;  // grid jobs wait for one another's CTAs:
+    attr[1].val.cooperative = 1;                  // all resident at once
+    cfg->attrs = attr;
+    cfg->numAttrs = s.cluster ? 1 : 2;
+}
+// Does the current device hold a launch of this shape: the cluster of a cluster job (up to 16 CTAs
+// in one cluster's reach, which a partition of a GPU may not have), every cluster of a grid job at
+// once?  The launched kernel with its own shared memory is what is asked about, once per device.
+static bool shape_fits(const PShape &s, int n, int dtype, bool realc, int njobs) {
+    const size_t smem = persist_smem(s, dtype);
+    if (n > PMAXN || s.na_bits > 4 || smem > 200 * 1024) return false;
+    if (s.cluster && s.gbits == 0) return true;
+    static std::atomic<signed char> known[64][2][2][2][PMAXN + 1];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    std::atomic<signed char> &k = known[dev][dtype == EMUSV_C128][realc][njobs - 1][n];
+    if (!k.load()) {
+        void *kern = pick(s, dtype, realc);
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr[2];
+        fill_config(&cfg, attr, s, njobs, smem);
+        cfg.numAttrs = 1;  // the cluster's size
+        int clusters = 0;
+        if (set_attributes(kern, s, smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            clusters = 0;
+        }
+        k.store(clusters >= (s.cluster ? 1 : (njobs << s.gbits >> PGC_BITS) + 1) ? 1 : 2);
+    }
+    return k.load() == 1;
+}
+
+// Test switch of the calling thread (emusv_krylov_set_streaming).
+static thread_local int tl_streaming = 0;
+void persist_set_streaming(int on) { tl_streaming = on ? 1 : 0; }
+
+bool lz_applies(int dtype, int n);
+// A register that no launch of this kind holds takes the streaming passes (lanczos_run), which run
+// from 12 qubits on; up to 11 a run is one CTA.
+bool persist_applies(const HamParams &P, int dtype) {
+    if (P.n < 1 || (dtype != EMUSV_C128 && dtype != EMUSV_C64)) return false;
+    if (tl_streaming && lz_applies(dtype, P.n)) return false;
+    return shape_fits(persist_shape(P.n, 1), P.n, dtype, P.real_coef != 0, 1);
 }
 size_t persist_exchange_bytes() { return (sizeof(PExchange) + 255) / 256 * 256; }
 
@@ -452,27 +499,12 @@ static unsigned long long next_epoch() {
     return next.fetch_add(4 * KMAX) & ~(1ull << 63);
 }
 
-template <typename R, bool REALC, int NA>
-static void *pick_na(bool cluster) {
-    return cluster ? reinterpret_cast<void *>(k_lanczos_persist<R, REALC, NA, CCT, CND, true>)
-                   : reinterpret_cast<void *>(k_lanczos_persist<R, REALC, NA, GCT, 0, false>);
-}
-template <typename R, bool REALC>
-static void *pick(const PShape &s) {
-    switch (s.na_bits) {
-    case 0: return pick_na<R, REALC, 1>(s.cluster);
-    case 1: return pick_na<R, REALC, 2>(s.cluster);
-    case 2: return pick_na<R, REALC, 4>(s.cluster);
-    case 3: return pick_na<R, REALC, 8>(s.cluster);
-    default: return pick_na<R, REALC, 16>(s.cluster);
-    }
-}
-
 int persist_launch(const HamParams &P, int dtype, double dt, const PJob *jobs, int njobs, int capacity,
                    double exp_tol, double norm_tol, int maxdim, cudaStream_t s) {
     PShape sh = persist_shape(P.n, njobs);
     int together = njobs;
-    if (!shape_fits(sh, dtype, njobs)) {  // in turn
+    const bool realc = P.real_coef != 0;
+    if (njobs > 1 && !shape_fits(sh, P.n, dtype, realc, njobs)) {  // in turn
         sh = persist_shape(P.n, 1);
         together = 1;
     }
@@ -489,26 +521,15 @@ int persist_launch(const HamParams &P, int dtype, double dt, const PJob *jobs, i
     A.wait = tl_wait;
     A.withhold = tl_withhold;
     const size_t smem = persist_smem(sh, dtype);
-    void *kern = dtype == EMUSV_C128 ? (P.real_coef ? pick<double, true>(sh) : pick<double, false>(sh))
-                                     : (P.real_coef ? pick<float, true>(sh) : pick<float, false>(sh));
-    EMUSV_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    if (sh.cluster && sh.gbits > 3) EMUSV_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    void *kern = pick(sh, dtype, realc);
+    EMUSV_CHECK(set_attributes(kern, sh, smem));
     for (int j0 = 0; j0 < njobs; j0 += together) {
         for (int j = 0; j < together; ++j) A.job[j] = jobs[j0 + j];
         A.epoch = next_epoch();
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((together << sh.gbits) + (sh.cluster ? 0 : 1 << PGC_BITS));
-        cfg.blockDim = dim3(sh.cluster ? CCT + 32 * CND : GCT);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = s;
+        cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 1u << (sh.cluster ? sh.gbits : PGC_BITS);
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        attr[1].id = cudaLaunchAttributeCooperative;  // grid jobs wait for one another's CTAs:
-        attr[1].val.cooperative = 1;                  // all resident at once
-        cfg.attrs = attr;
-        cfg.numAttrs = sh.cluster ? 1 : 2;
+        fill_config(&cfg, attr, sh, together, smem);
+        cfg.stream = s;
         void *args[] = {(void *)&A};
         ProfScope ps_(PROF_HPSI, s);
         EMUSV_CHECK(cudaLaunchKernelExC(&cfg, kern, args));

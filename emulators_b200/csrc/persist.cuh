@@ -39,6 +39,7 @@
 
 namespace emusv {
 
+constexpr int PMAXN = 20;          // qubits of a run at most
 constexpr int PMAXG_BITS = 7;      // CTAs per job: at most 128
 constexpr int PMAXG = 1 << PMAXG_BITS;
 constexpr int PCL_BITS = 4;        // CTAs of a cluster job: at most 16
@@ -80,9 +81,10 @@ struct PArgs {
 };
 
 // Host side (persist.cu).
-bool persist_applies(int dtype, int n);
+bool persist_applies(const HamParams &P, int dtype);  // on the current device
 size_t persist_exchange_bytes();
 void persist_set_wait_test(long long wait_cycles, int withhold);
+void persist_set_streaming(int on);
 // Runs 1 or 2 jobs of the same operator; the caller reads their states afterwards.
 int persist_launch(const HamParams &P, int dtype, double dt, const PJob *jobs, int njobs, int capacity,
                    double exp_tol, double norm_tol, int maxdim, cudaStream_t s);

@@ -128,8 +128,8 @@ size_t emusv_krylov_workspace_bytes(int nqubits, int dtype, int basis_capacity);
  * Convergence is tested on the device at every iteration, as the reference does; the
  * host reads the device's decision from iteration `krylov_dim_hint` on (0: every
  * iteration), so the hint only saves host synchronisations and never moves the stopping
- * iteration.  Registers of up to 20 qubits run the whole step in one launch and do not use
- * the hint.
+ * iteration.  Registers of up to 20 qubits run the whole step in one launch (where the GPU
+ * holds it) and do not use the hint.
  * The workspace carries one value from call to call: the previous step's energy, which
  * the next step subtracts from H inside H*psi (same basis and coefficients; less
  * complex64 rounding of the diagonal).  Zero the workspace once before its first call.
@@ -151,6 +151,11 @@ int emusv_krylov_step(int nqubits, int dtype, double dt, const double *omegas,
  * runs out, all CTAs return and the call gives EMUSV_TIMEOUT; the device stays usable.  Off by
  * default; for tests.  Host-side only (takes effect at the next call). */
 int emusv_krylov_set_wait_test(long long wait_cycles, int withhold);
+/* Test switch of the calling thread: with on != 0 its emusv_krylov_step and emusv_adjoint_step run
+ * registers of 12 to 20 qubits by the streaming passes, as they do by themselves on a GPU (or a
+ * partition of one) that does not hold the one-launch run's clusters of CTAs.  Same stopping
+ * iteration, results within rounding.  Host-side only. */
+int emusv_krylov_set_streaming(int on);
 
 /* Bytes of device workspace emusv_adjoint_step needs when each of its two Lanczos bases
  * may hold `basis_capacity` vectors (3 * (capacity + 1) + 1 vectors of 2^n amplitudes
