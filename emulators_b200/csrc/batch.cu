@@ -1642,6 +1642,14 @@ __device__ __forceinline__ bool job_ok(const KState *ks) {
     return st == KS_CONVERGED || st == KS_HAPPY;
 }
 
+// Both bases of instance i are there: the launch that built them met no error (a wait that ran out
+// leaves states of an earlier launch, or none, behind) and both runs ended with one.
+__device__ __forceinline__ bool bases_ok(const BArgs &A, int i) {
+    const int err = ld_vol(&A.ctl->err);
+    const bool s = job_ok(A.ks + 2 * i), g = job_ok(A.ks + 2 * i + 1);
+    return !err && s && g;
+}
+
 // dS column `col` of instance i: y = exp(B) e_{ms+col} for the block matrix
 // B = [[A_s, e0 e0^T], [0, A_g]] (A = -i dt T of each basis, the coupling taken as 1:
 // double_krylov.py:54-57 scales it by |state||grad| afterwards), rows 0..ms-1 of y.
@@ -1661,7 +1669,7 @@ __global__ void __launch_bounds__(BWARPS * 32) k_batch_dS(const BArgs A, const B
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i = blockIdx.y, col = blockIdx.x * BWARPS + warp;
     const KState *kss = A.ks + 2 * i, *ksg = A.ks + 2 * i + 1;
-    if (!job_ok(kss) || !job_ok(ksg)) return;
+    if (!bases_ok(A, i)) return;
     const int ms = basis_size(kss), mg = basis_size(ksg), M = ms + mg;
     if (col >= mg || M > 32 * DS_NE || ms > D.mmax || mg > D.mmax) return;
     const double dt = A.inst[2 * i].dt;
@@ -1706,7 +1714,7 @@ __global__ void __launch_bounds__(PE_T, 2) k_post_E(const BArgs A, const BAdj D)
     __shared__ double2 cf[KMAX][PE_K];
     const int i = blockIdx.z, k0 = blockIdx.y * PE_K;
     const KState *kss = A.ks + 2 * i, *ksg = kss + 1;
-    if (!job_ok(kss) || !job_ok(ksg)) return;
+    if (!bases_ok(A, i)) return;
     const int ms = basis_size(kss), mg = basis_size(ksg);
     const BInst I = A.inst[2 * i];
     const long long x0 = (long long)blockIdx.x * PE_T * PE_X + threadIdx.x, len = 1LL << I.n;
@@ -1767,8 +1775,8 @@ __global__ void __launch_bounds__(PE_T) k_post_gout(const BArgs A, const BAdj D)
     const long long x = (long long)blockIdx.x * PE_T + threadIdx.x;
     if (x >= 1LL << I.n) return;  // whole blocks: registers have 2^8 amplitudes or more
     C *out = reinterpret_cast<C *>(D.gout) + I.off0;
-    if (!job_ok(kss) || !job_ok(ksg)) {
-        if (__ldcg(&ksg->s0) == 0.0) out[x] = cmake<C>(0.0, 0.0);  // exp(+i dt H) 0 = 0
+    if (!bases_ok(A, i)) {
+        if (!ld_vol(&A.ctl->err) && __ldcg(&ksg->s0) == 0.0) out[x] = cmake<C>(0.0, 0.0);  // exp(+i dt H) 0 = 0
         return;
     }
     const int nvec = __ldcg(&ksg->nvec);
@@ -1810,8 +1818,8 @@ __device__ __forceinline__ double *post_row(const BAdj &D, const BInst &I, int i
     return D.partC + ((size_t)((I.off0 >> PC_TB) + i) * PC_KS + block) * NCP;
 }
 __device__ __forceinline__ bool post_block(const BArgs &A, int i, BInst *I, BInst *IG, int *mg) {
-    const KState *kss = A.ks + 2 * i, *ksg = kss + 1;
-    if (!job_ok(kss) || !job_ok(ksg)) return false;
+    if (!bases_ok(A, i)) return false;
+    const KState *ksg = A.ks + 2 * i + 1;
     *I = A.inst[2 * i];
     *IG = A.inst[2 * i + 1];
     *mg = basis_size(ksg);
@@ -2020,12 +2028,13 @@ __global__ void __launch_bounds__(128 * PF_G) k_post_finish(const BArgs A, const
     const BInst I = A.inst[2 * i];
     const int n = I.n, p = threadIdx.x;
     double *g = D.grads + (size_t)i * 3 * BMAXQ;
-    if (!job_ok(kss) || !job_ok(ksg)) {  // a zero gradient (or a failed basis): no parameter gradient
+    if (!bases_ok(A, i)) {  // a zero gradient (or a failed basis): no parameter gradient
+        const int err = ld_vol(&A.ctl->err);
         const bool zero = __ldcg(&ksg->s0) == 0.0;
         if (p < n) g[p] = g[BMAXQ + p] = g[2 * BMAXQ + p] = 0.0;
         if (p == 0) {
-            int e = EMUSV_OK;
-            if (!zero) {
+            int e = err;
+            if (!err && !zero) {
                 e = EMUSV_NONFINITE;
                 for (const KState *k2 : {kss, ksg}) {
                     const int st = ld_status(k2);

@@ -333,7 +333,8 @@ int emusv_batch_results(int ninst, int max_steps, void *workspace, int *status_o
  * takes step `step` of every instance: states (psi_step, packed) and grad_in (dL/dpsi
  * after the step, packed) in, grad_out (dL/dpsi before the step = exp(+i dt H) grad_in)
  * and grads_dev [ninst][3][20] (dL/dOmega_q, dL/ddelta_q, dL/dphi_q by qubit q; FP64,
- * device) out, plus an emusv status per instance in status_dev [ninst] (device).  The
+ * device) out, plus an emusv status per instance in status_dev [ninst] (device;
+ * EMUSV_TIMEOUT for all of them, with zero gradients and no grad_out, if a wait gave up).  The
  * interaction-matrix gradient is not formed here (emusv_adjoint_step has it).
  * Capturable: a launch issues two memsets and one cooperative kernel. */
 size_t emusv_batch_adjoint_workspace_bytes(int ninst, const int *nqubits, const int *nsteps,
