@@ -405,7 +405,7 @@ __device__ __forceinline__ void load_rows(const KState *ks, int m, double dt, do
 // NE entries per lane: the smallest layout that holds the jj + 3 rows (the work of every
 // Chebyshev term scales with NE; each entry's arithmetic is the same in every layout).
 template <int NE>
-static __device__ __noinline__ double krylov_eval_ne(const KState *ks, int jj, double dt, double *c_re, double *c_im) {
+__device__ __forceinline__ double krylov_eval_to(const KState *ks, int jj, double dt, double *c_re, double *c_im) {
     const int lane = threadIdx.x & 31;
     const int m = jj + 1, M = m + 2;
     double2 d[NE], l[NE], u[NE], y[NE];
@@ -440,16 +440,25 @@ static __device__ __noinline__ double krylov_eval_ne(const KState *ks, int jj, d
     __syncwarp();
     return err1 < err2 ? err1 : (err1 * err2 / (err1 - err2));  // krylov_exp.py:84
 }
-static __device__ double krylov_eval(const KState *ks, int jj, double dt, double *c_re, double *c_im) {
+// Into the run's state, or into a caller's arrays: two functions, because with the arrays as
+// arguments of one function for both the batch's decision (job_decide) reloads 660 bytes of spilled
+// registers instead of 484.
+template <int NE>
+static __device__ __noinline__ double krylov_eval_ne(KState *ks, int jj, double dt) {
+    return krylov_eval_to<NE>(ks, jj, dt, ks->c_re, ks->c_im);
+}
+template <int NE>
+static __device__ __noinline__ double krylov_eval_ne(const KState *ks, int jj, double dt, double *c_re, double *c_im) {
+    return krylov_eval_to<NE>(ks, jj, dt, c_re, c_im);
+}
+template <typename State, typename... Out>
+static __device__ double krylov_eval(State *ks, int jj, double dt, Out... out) {
     constexpr int NEMAX = (KMAX + 2 + 31) / 32;
     const int M = jj + 3;
-    if (M <= 32) return krylov_eval_ne<1>(ks, jj, dt, c_re, c_im);
-    if (M <= 64) return krylov_eval_ne<2>(ks, jj, dt, c_re, c_im);
-    if (M <= 96) return krylov_eval_ne<3>(ks, jj, dt, c_re, c_im);
-    return krylov_eval_ne<NEMAX>(ks, jj, dt, c_re, c_im);
-}
-static __device__ double krylov_eval(KState *ks, int jj, double dt) {
-    return krylov_eval(ks, jj, dt, ks->c_re, ks->c_im);
+    if (M <= 32) return krylov_eval_ne<1>(ks, jj, dt, out...);
+    if (M <= 64) return krylov_eval_ne<2>(ks, jj, dt, out...);
+    if (M <= 96) return krylov_eval_ne<3>(ks, jj, dt, out...);
+    return krylov_eval_ne<NEMAX>(ks, jj, dt, out...);
 }
 
 // Decide iteration j of a Lanczos run from the FP64 sums v = ||w_j||^2 and
