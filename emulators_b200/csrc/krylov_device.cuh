@@ -235,14 +235,17 @@ static __device__ void reg_expm(int M, const double2 (&d)[NE], const double2 (&l
 // Bessel values J_k(|z|) in the same order (normalised at the end by
 // J_0 + 2 sum J_2k = 1).  About |z| + 40 tridiagonal products instead of the Taylor
 // form's ~12 |z|.  `Tdiag[e]` is T's (real) diagonal centre of row e and `Trad[e]` its
-// Gershgorin radius (|row| off-diagonal sum of T).  `abandon`: when given and set, the
-// result is no longer wanted and y is left undefined (looked at every eighth term).
+// Gershgorin radius (|row| off-diagonal sum of T).  dt = 0: e_col.
 template <int NE>
 static __device__ void cheb_expm(const double2 (&d)[NE], const double2 (&l)[NE], const double2 (&u)[NE],
                                  int cpl, double2 cplv, int col, double dt, const double (&Tdiag)[NE],
-                                 const double (&Trad)[NE], int M, double2 (&y)[NE],
-                                 const volatile int *abandon = nullptr) {
+                                 const double (&Trad)[NE], int M, double2 (&y)[NE]) {
     const int lane = threadIdx.x & 31;
+    if (dt == 0.0) {
+#pragma unroll
+        for (int e = 0; e < NE; ++e) y[e] = make_double2(lane * NE + e == col ? 1.0 : 0.0, 0.0);
+        return;
+    }
     double lo = 1e300, hi = -1e300;
 #pragma unroll
     for (int e = 0; e < NE; ++e) {
@@ -301,7 +304,7 @@ static __device__ void cheb_expm(const double2 (&d)[NE], const double2 (&l)[NE],
     };
     const int N = (int)ceil(1.1 * z) + 40;  // terms kept
     const int K = N + 30;                   // Miller's start
-    const double twoz = z > 0.0 ? 2.0 / z : 0.0;  // no division inside the recurrence
+    const double twoz = 2.0 / z;            // no division inside the recurrence
     double2 b1[NE], b2[NE];  // b_{k+1}, b_{k+2}
 #pragma unroll
     for (int e = 0; e < NE; ++e) b1[e] = b2[e] = make_double2(0.0, 0.0);
@@ -316,7 +319,6 @@ static __device__ void cheb_expm(const double2 (&d)[NE], const double2 (&l)[NE],
     }
     const double2 up_step = make_double2(0.0, sgn);
     for (int k = K; k >= 1; --k) {
-        if (abandon && (k & 7) == 0 && *abandon) return;
         if ((k & 1) == 0) S += 2.0 * jk;
         if (k <= N) {  // b_k = coef_k e_col + 2 X b_{k+1} - b_{k+2}
             double2 xb[NE];
@@ -357,12 +359,11 @@ static __device__ void cheb_expm(const double2 (&d)[NE], const double2 (&l)[NE],
     double2 xb[NE];
     xmul(b1, xb);
     const double2 ea = make_double2(cos(alpha.y), sin(alpha.y));  // e^{alpha}, alpha imaginary
-    const double inv = z > 0.0 ? 1.0 / S : 1.0;
+    const double inv = 1.0 / S;
 #pragma unroll
     for (int e = 0; e < NE; ++e) {
         double2 v = make_double2(xb[e].x - b2[e].x, xb[e].y - b2[e].y);
         if (lane * NE + e == col) v.x += jk;
-        if (z == 0.0) v = make_double2(lane * NE + e == col ? 1.0 : 0.0, 0.0);
         v.x *= inv;
         v.y *= inv;
         y[e] = cm(ea, v);

@@ -29,7 +29,7 @@ __device__ __forceinline__ double reg_pick(const double (&v)[NE], int k) {  // e
 // terms above.  Kept real for the chain's length, which is what a single step waits for at its
 // end: a step of 10 qubits takes 196 us with it and 235 with the complex rows of cheb_expm (the
 // rounding-level imaginary part of the diagonal in them, 1.1 z + 40 terms), which stay where a
-// decision is hidden behind other registers or a long iteration.
+// decision is hidden behind other registers or a long iteration.  dt = 0: e_col.
 // `abandon`: when given and set, the result is no longer wanted and y is left undefined
 // (looked at every eighth term).
 template <int NE>
@@ -37,6 +37,11 @@ static __device__ void cheb_expm_real(const double (&d)[NE], const double (&l)[N
                                  double cplv, int col, double dt, int M, double2 (&y)[NE],
                                  const volatile int *abandon = nullptr) {
     const int lane = threadIdx.x & 31;
+    if (dt == 0.0) {  // (a coupling entry of 1/dt is left out: what it leads to is multiplied by dt)
+#pragma unroll
+        for (int e = 0; e < NE; ++e) y[e] = make_double2(lane * NE + e == col ? 1.0 : 0.0, 0.0);
+        return;
+    }
     double lo = 1e300, hi = -1e300;
 #pragma unroll
     for (int e = 0; e < NE; ++e) {
