@@ -2087,8 +2087,8 @@ static size_t al256(size_t v) { return (v + 255) / 256 * 256; }
 // (gradient) per instance, plus the adjoint's own arrays.
 struct BLayout {
     size_t args, ctl, ints, rec, cta0, inst, coef, ubits, elow, ks, sums, iters, partA, partB, partN, slots;
-    size_t dS, escr, E, partC, total;
-    int njobs, total_tiles, coef_count, max_steps, mmax, escr_warps;
+    size_t dS, E, partC, total;
+    int njobs, total_tiles, coef_count, max_steps, mmax;
     long long inst_amps, slot_amps;
 };
 
@@ -2136,8 +2136,7 @@ static bool layout(int ninst, const int *nq, const int *nsteps, int es, int T, i
     L->partB = take(sizeof(double) * 4 * L->total_tiles);
     L->partN = take(sizeof(double) * 4 * L->total_tiles);
     L->slots = take((size_t)capacity * (size_t)L->slot_amps * es);
-    L->dS = L->escr = L->E = L->partC = off;
-    L->escr_warps = 0;
+    L->dS = L->E = L->partC = off;
     if (adjoint) {
         L->dS = take(sizeof(double2) * ninst * (size_t)L->mmax * L->mmax);
         L->E = take((size_t)L->mmax * (size_t)amps * es);
@@ -2174,9 +2173,9 @@ static void *pick_kernel(int dtype, int T, int kind) {
     return nullptr;
 }
 
-// Dynamic shared memory of a kernel kind: the H v phase's partner-tile stages.  Set as the
+// Dynamic shared memory of every kind: the H v phase's partner-tile stages.  Set as the
 // kernel's limit before its occupancy is queried or it is launched.
-static size_t kernel_smem(int dtype, int T, int kind) {
+static size_t kernel_smem(int dtype, int T) {
     const size_t es = dtype == EMUSV_C128 ? 16 : 8;
     return (size_t)BWARPS * PSTAGES * (es << T);
 }
@@ -2216,7 +2215,7 @@ static int prepare_common(int ninst, const int *nqubits, const int *nsteps, cons
     // the shared-memory limits of the kernels the launches may use (host calls, so that a
     // launch recorded into a CUDA graph issues none)
     for (int kind : {0, 1, 3, 4}) {
-        const int st = configure_smem(pick_kernel(dtype, T, kind), kernel_smem(dtype, T, kind));
+        const int st = configure_smem(pick_kernel(dtype, T, kind), kernel_smem(dtype, T));
         if (st) return st;
     }
     const int es = dtype == EMUSV_C128 ? 16 : 8;
@@ -2358,7 +2357,7 @@ static int prepare_common(int ninst, const int *nqubits, const int *nsteps, cons
     for (int J = 0; J < nj; ++J) cta0[J + 1] = cta0[J] + (inst[J].ntiles + BWARPS - 1) / BWARPS;
     int per_sm = 0;
     EMUSV_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick_kernel(dtype, T, 4), BWARPS * 32,
-                                                              kernel_smem(dtype, T, 4)));
+                                                              kernel_smem(dtype, T)));
     // as many deciding warps a job as fit beside the gangs
     P.width = BWARPS;
     auto deciding = [&] { return (nj * P.width + BWARPS - 1) / BWARPS; };
@@ -2427,7 +2426,7 @@ static int gang_launch(int dtype, const Prepared &P, const BArgs &A, unsigned ch
     EMUSV_CHECK(cudaMemsetAsync(G.rec, 0, sizeof(PRec) * (7 * (size_t)A.total_tiles + (size_t)GANG_JREC * A.ninst), s));
     void *args[] = {(void *)&G};
     return cooperative_launch(pick_kernel(dtype, A.T, 4), 1, args, s, P.gang + (A.ninst * P.width + BWARPS - 1) / BWARPS,
-                              PROF_BATCH, kernel_smem(dtype, A.T, 4));
+                              PROF_BATCH, kernel_smem(dtype, A.T));
 }
 
 }  // namespace emusv
@@ -2488,7 +2487,7 @@ int emusv_batch_launch_steps(int dtype, int tile_bits, int blocks_per_sm, int fi
     if (P.engine && P.gang) return gang_launch(dtype, P, A, ws, s);
     void *args[] = {(void *)&A};
     return cooperative_launch(kern, blocks_per_sm, args, s, 0, PROF_BATCH,
-                              kernel_smem(dtype, tile_bits, kind));
+                              kernel_smem(dtype, tile_bits));
 }
 
 // Scheduling of a prepared forward workspace's launches: 0 (default) lock-step rounds,
@@ -2503,8 +2502,9 @@ int emusv_batch_set_engine(void *workspace, int engine) {
 }
 
 // Clears the control block and launches the persistent kernel over every step on the
-// states given to emusv_batch_prepare.  Issues only stream-ordered device work (one memset
-// and one cooperative launch), so the call can be recorded into a CUDA graph and replayed.
+// states given to emusv_batch_prepare.  Issues only stream-ordered device work (a memset, or two
+// where gangs run, and one cooperative launch), so the call can be recorded into a CUDA graph and
+// replayed.
 int emusv_batch_launch(int dtype, int tile_bits, int blocks_per_sm, void *workspace, void *stream) {
     Prepared P;
     if (!workspace || lookup(workspace, false, &P)) return EMUSV_BAD_ARGUMENT;
@@ -2515,7 +2515,7 @@ int emusv_batch_launch(int dtype, int tile_bits, int blocks_per_sm, void *worksp
 int emusv_batch_max_blocks_per_sm(int dtype, int tile_bits) {
     void *kern = pick_kernel(dtype, tile_bits, 0);
     if (!kern) return 0;
-    const size_t smem = kernel_smem(dtype, tile_bits, 0);
+    const size_t smem = kernel_smem(dtype, tile_bits);
     if (configure_smem(kern, smem)) return 0;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BWARPS * 32, smem) != cudaSuccess)
@@ -2608,7 +2608,7 @@ int emusv_batch_adjoint_launch(int dtype, int tile_bits, int blocks_per_sm, int 
     void *args[] = {(void *)&A, (void *)&D};
     const int st = P.gang ? gang_launch(dtype, P, A, ws, s)
                           : cooperative_launch(k1, blocks_per_sm, args, s, 0, PROF_BATCH,
-                                               kernel_smem(dtype, tile_bits, 1));
+                                               kernel_smem(dtype, tile_bits));
     if (st) return st;
     {
         ProfScope ps_(PROF_ADJOINT, s);

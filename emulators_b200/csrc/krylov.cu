@@ -483,11 +483,12 @@ int lanczos_run(const HamParams &P, int dtype, double dt, const void *v0, KState
     EMUSV_CHECK_LAUNCH();
 
     int status = KS_RUNNING;
-    // The H-first iteration: the pass H kernels write part = X_high v_j (the flips of the bits above the pass-L tile) and their share
-    // of <v_j, H v_j>; k_lz_coef forms a_j; the pass L kernel forms H v_j tile by tile and
-    // writes w = H v_j - a_j v_j - b_j v_{j-1} and the pass-L share of <w, H w> for the
-    // next a; k_lz_norms and k_lz_decide conclude the iteration.  Streamed vector units per iteration: pass L 4 (read v_j,
-    // part, v_{j-1}; write w), one H pass 2 (read v_j, write part) or two H passes 2 + 3.
+    // The H-first iteration: the pass H kernels write part = X_high v_j (the flips of the bits
+    // above the pass-L tile) and their share of <v_j, H v_j>; k_lz_coef forms a_j; the pass L
+    // kernel forms H v_j tile by tile and writes w = H v_j - a_j v_j - b_j v_{j-1} and the pass-L
+    // share of <w, H w> for the next a; k_lz_norms and k_lz_decide conclude the iteration.
+    // Streamed vector units per iteration: pass L 4 (read v_j, part, v_{j-1}; write w), one H pass
+    // 2 (read v_j, write part) or two H passes 2 + 3.
     {
         // with `overlap`, the decision of iteration j (k_lz_decide) runs on a second stream
         // while the main stream goes on with iteration j+1, which needs only k_lz_norms'

@@ -392,7 +392,7 @@ static size_t persist_smem(const PShape &s, int dtype) {
 // three SMs left to others); clusters to 15 (16 qubits on a cluster of 16: 14.6 us an
 // iteration, on the grid 10: the partners' amplitudes come through distributed shared memory
 // at about 18 bytes a clock); the grid to 20, where v_j and the diagonal still fit (20 qubits
-// complex128: 1370 us against 1909 for the streaming passes).
+// complex128: 1340 us against 1909 for the streaming passes).
 static PShape persist_shape(int n, int njobs) {
     PShape s;
     s.cluster = n <= 15;
@@ -403,10 +403,13 @@ static PShape persist_shape(int n, int njobs) {
     s.na_bits = s.tbits > lb ? s.tbits - lb : 0;
     return s;
 }
+
 template <typename R, bool REALC, int NA>
 static void *pick_na(bool cluster) {
-    return cluster ? reinterpret_cast<void *>(k_lanczos_persist<R, REALC, NA, CCT, CND, true>)
-                   : reinterpret_cast<void *>(k_lanczos_persist<R, REALC, NA, GCT, 0, false>);
+    if constexpr (NA < 16) {  // a cluster job's CTA has at most 2^11 amplitudes
+        if (cluster) return reinterpret_cast<void *>(k_lanczos_persist<R, REALC, NA, CCT, CND, true>);
+    }
+    return reinterpret_cast<void *>(k_lanczos_persist<R, REALC, NA, GCT, 0, false>);
 }
 template <typename R, bool REALC>
 static void *pick(const PShape &s) {
@@ -418,7 +421,6 @@ static void *pick(const PShape &s) {
     default: return pick_na<R, REALC, 16>(s.cluster);
     }
 }
-
 static void *pick(const PShape &s, int dtype, bool realc) {
     return dtype == EMUSV_C128 ? (realc ? pick<double, true>(s) : pick<double, false>(s))
                                : (realc ? pick<float, true>(s) : pick<float, false>(s));

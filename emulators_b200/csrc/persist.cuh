@@ -20,15 +20,18 @@
 // The decisions (krylov_exp.py:60-96: happy breakdown, exponential of the extended tridiagonal
 // matrix, Expokit estimate) are taken by extra warps (of every CTA of a cluster job, of one
 // more CTA of a grid job), one iteration each, while the compute warps go on: an iteration of
-// a small register takes a few us, a decision about ten.  An iteration that ends the run does so once every earlier one is known not to, so the run stops
-// at the first iteration that converges, where the reference stops; the iterations computed
-// meanwhile are left unused.
+// a small register takes a few us, a decision about ten.  An iteration that ends the run does so
+// once every earlier one is known not to, so the run stops at the first iteration that converges,
+// where the reference stops; the iterations computed meanwhile are left unused.
 //
-// Bound by latencies: per iteration two exchanges and the flips.  Measured on B200 (us per
-// iteration, complex128 unless said; launches per iteration before): 10 qubits 2.7 (40), 12
-// 4.2 (47), 15 complex64 6.9 (50), 16 10, 18 14.5, 20 36 (60).  An exchange takes 0.4 us in one
-// CTA, 1.5-1.8 in a cluster, 3.1-3.8 through the L2 with 32 clusters of four (4.9-6.4 when 128
-// CTAs read each other's records).
+// Bound by latencies: per iteration two exchanges and the flips.  Measured on B200 (us per further
+// iteration of the kernel, complex128 unless said; in brackets the us an iteration took as several
+// kernels): 12 qubits 4.3 (47), 14 6.2, 15 complex64 7.0 (50), 16 9.9, 18 14.7, 20 38 (60).  In one
+// CTA the decisions bound it, whose work grows with the basis and which four warps share: 10 qubits
+// 79 us for 14 iterations, 142 for 28, 400 for 54 (40 us each as kernels).  An exchange takes 0.4 us in one CTA, 1.5-1.8 in
+// a cluster, 3.1-3.8 through the L2 with 32 clusters of four (4.9-6.4 when 128 CTAs read each
+// other's records); one warp a sum waits and hands it on (with all eight warps waiting 12 qubits
+// took 4.5 us an iteration, 14 6.5, 18 15.4).
 //
 // Every wait is bounded (PArgs::wait): on a timeout the CTA records EMUSV_TIMEOUT in the run's state
 // and the job's CTAs return.  Whether a wait ran out is decided by the warps that wait and handed

@@ -1,6 +1,6 @@
 // Device code of the runs that stay on chip: the exchange of sums between a job's CTAs and the
-// convergence decisions (see persist.cuh), shared by the single steps (persist.cu) and the
-// batches (batch_cluster.cu).
+// convergence decisions (see persist.cuh) of the single steps (persist.cu), and the records of
+// value and epoch, which the batches' gangs (batch.cu) use too.
 #pragma once
 
 #include "persist.cuh"
@@ -21,8 +21,8 @@ __device__ __forceinline__ PRec rec_get(const PRec *r) {
         asm volatile("{\n .reg .b128 t;\n ld.acquire.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
                      : "=l"(v), "=l"(e) : "l"(r) : "memory");
     else
-    asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
-                 : "=l"(v), "=l"(e) : "l"(r) : "memory");
+        asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+                     : "=l"(v), "=l"(e) : "l"(r) : "memory");
     PRec o;
     o.v = __longlong_as_double(v);
     o.e = e;

@@ -307,8 +307,10 @@ int emusv_batch_prepare(int ninst, const int *nqubits, const int *nsteps, const 
                         double norm_tolerance, int max_krylov_dim, int tile_bits,
                         int basis_capacity, void *workspace, size_t workspace_bytes,
                         void *stream);
-/* One memset and one cooperative launch (stream-ordered only, so it can be captured in a
- * CUDA graph and replayed): evolves every instance through all its steps. */
+/* A memset (two where gangs run, emusv_batch_set_engine) and one cooperative launch
+ * (stream-ordered only, so it can be captured in a CUDA graph and replayed): evolves every
+ * instance through all its steps.  Gangs take as many CTAs as they need: blocks_per_sm has no
+ * effect on them. */
 int emusv_batch_launch(int dtype, int tile_bits, int blocks_per_sm, void *workspace, void *stream);
 /* Steps [first_step, first_step + steps) of the prepared batch on `states` (NULL: the
  * prepared states), in place; when `history` is given, the packed states after every
@@ -336,7 +338,8 @@ int emusv_batch_results(int ninst, int max_steps, void *workspace, int *status_o
  * device) out, plus an emusv status per instance in status_dev [ninst] (device;
  * EMUSV_TIMEOUT for all of them, with zero gradients and no grad_out, if a wait gave up).  The
  * interaction-matrix gradient is not formed here (emusv_adjoint_step has it).
- * Capturable: a launch issues two memsets and one cooperative kernel. */
+ * Capturable: a launch issues two memsets (three where gangs build the bases; blocks_per_sm
+ * then has no effect), the cooperative kernel of the bases and the kernels that contract them. */
 size_t emusv_batch_adjoint_workspace_bytes(int ninst, const int *nqubits, const int *nsteps,
                                            int dtype, int tile_bits, int basis_capacity);
 int emusv_batch_adjoint_prepare(int ninst, const int *nqubits, const int *nsteps, const double *dt,
