@@ -92,8 +92,14 @@ __device__ __forceinline__ double warp_transpose_sum(double (&v)[32]) {
 }
 
 constexpr int LAG_E = 4;  // amplitudes per thread and chunk
+// Blocks of pass A per SM.  Its 16 to 32 loads and 32 sums a thread take 202 registers: complex128
+// (half the amplitudes in flight) streams at one block an SM.  Complex64 does the same arithmetic
+// on half the bytes, conversions besides, and one block's eight warps do not cover it: 2^22
+// amplitudes, 18 iterations 420 us a pass with one block and 176 with two on 128 registers (2^20
+// 107 and 52; 208 and 67 with one value at a time).
+template <typename R> constexpr int LAG_BLOCKS = sizeof(R) == 8 ? 1 : 2;
 template <typename R>
-__global__ void __launch_bounds__(ORTHO_THREADS, 1)
+__global__ void __launch_bounds__(ORTHO_THREADS, LAG_BLOCKS<R>)
 k_arn_lagdots(const KState *ks, int j, const void *v0_, const unsigned char *basis, i64 D,
               const void *w_, double *part) {
     typedef typename cvec<R>::T C;
@@ -198,9 +204,9 @@ k_arn_lagdots(const KState *ks, int j, const void *v0_, const unsigned char *bas
 
 // Pass B: w' = cw w - ct vt - sum cw1_l v_l (in place over w) and, for j >= 1, the
 // corrected v_j = cv vt - sum cvj_l v_l (in place over vt, stored with scale 1); ||w'||^2.
-// The chunks run from the last to the first, pass A's from the first to the last: each pass
-// begins on the part of the basis that the other left in the L2.
-template <typename R, int E = 4, int KB = 4>
+// REVERSE: the chunks run from the last to the first, pass A's from the first to the last, so each
+// pass begins on the part of the basis that the other left in the L2 (for a basis larger than that).
+template <typename R, bool REVERSE, int E = 4, int KB = 4>
 __global__ void __launch_bounds__(ORTHO_THREADS)
 k_arn_lagupdate(const KState *ks, const ArnState *as, int j, const void *v0_, unsigned char *basis,
                 i64 D, void *w_, double *part) {
@@ -228,8 +234,8 @@ k_arn_lagupdate(const KState *ks, const ArnState *as, int j, const void *v0_, un
     auto vk = [&](int k) -> const C * { return k == 0 ? v0 : bs + (i64)k * D; };
     double nacc = 0.0;
     const i64 CH = (i64)ORTHO_THREADS * E, nch = (D + CH - 1) / CH;
-    for (i64 ch = nch - 1 - blockIdx.x; ch >= 0; ch -= gridDim.x) {
-        const i64 c0 = ch * CH;
+    for (i64 ch = blockIdx.x; ch < nch; ch += gridDim.x) {
+        const i64 c0 = (REVERSE ? nch - 1 - ch : ch) * CH;
         double ur[E], ui[E], qr[E], qi[E];
 #pragma unroll
         for (int e = 0; e < E; ++e) {
@@ -666,26 +672,32 @@ static size_t decide_smem(int maxdim) {
 }
 
 // Grid of the Gram-Schmidt passes: never more blocks than chunks; *grid_out receives the
-// number of blocks in x (the partial sums per value).  Pass A holds one block per SM (its 32
-// sums and 16 loads a thread fill the registers), a persistent grid; where that leaves SMs
-// idle, the groups of basis vectors are spread over blocks in y.
+// number of blocks in x (the partial sums per value).  Pass A is a persistent grid (LAG_BLOCKS an
+// SM); where that leaves SMs idle, the groups of basis vectors are spread over blocks in y.  Pass B
+// runs backwards once the vectors of an iteration are more than the L2 holds (126 MB): 2^20
+// complex128 amplitudes, 21 iterations 32.1 us a pass against 35.8 forwards; on a basis inside the
+// L2 forwards is the faster one (2^18: 8.4 against 9.1, complex64 10.0 against 11.2).
+constexpr i64 LAG_L2_BYTES = i64(100) << 20;
 template <typename R>
 static int launch_lagged(int pass, const KState *ks, const ArnState *as, int j, const void *v0,
                          unsigned char *basis, i64 D, void *w, double *part, cudaStream_t s,
                          int *grid_out) {
     constexpr int E = LAG_E;
     const i64 chunks = (D + (i64)ORTHO_THREADS * E - 1) / ((i64)ORTHO_THREADS * E);
-    i64 grid = pass == 0 ? (i64)sm_count() : (i64)krylov_stream_grid(D);
+    const i64 resident = (i64)sm_count() * LAG_BLOCKS<R>;
+    i64 grid = pass == 0 ? resident : (i64)krylov_stream_grid(D);
     if (grid > chunks) grid = chunks;
     *grid_out = (int)grid;
     ProfScope ps_(PROF_ORTH, s);
     if (pass == 0) {
         const int groups = ((j >= 1 ? j : 1) + ARN_KB - 1) / ARN_KB;
-        int gy = (int)(sm_count() / grid);
+        int gy = (int)(resident / grid);
         if (gy > groups) gy = groups;
         k_arn_lagdots<R><<<dim3((unsigned)grid, gy), ORTHO_THREADS, 0, s>>>(ks, j, v0, basis, D, w, part);
     } else {
-        k_arn_lagupdate<R, E><<<(int)grid, ORTHO_THREADS, 0, s>>>(ks, as, j, v0, basis, D, w, part);
+        const bool reverse = (i64)(j + 2) * D * (i64)sizeof(typename cvec<R>::T) > LAG_L2_BYTES;
+        auto *kern = reverse ? k_arn_lagupdate<R, true, E> : k_arn_lagupdate<R, false, E>;
+        kern<<<(int)grid, ORTHO_THREADS, 0, s>>>(ks, as, j, v0, basis, D, w, part);
     }
     EMUSV_CHECK_LAUNCH();
     return EMUSV_OK;
