@@ -67,7 +67,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_block_prefix(const double *bsu
     }
 }
 
-template <typename R>
+// GU groups of 32 amplitudes at a time: their loads and scans overlap, the running sum goes through
+// the groups in order, so every GU gives the same draw (n = 22, 1000 draws: 62 us with one group at
+// a time, every group waiting for its own load; see single_groups).
+template <typename R, int GU>
 __global__ void __launch_bounds__(BLOCK)
 k_draw(const void *psi_, i64 D, const double *prefix, i64 nb, const double *u, int shots,
        long long *out, int *bad) {
@@ -91,10 +94,6 @@ k_draw(const void *psi_, i64 D, const double *prefix, i64 nb, const double *u, i
     const i64 SB = i64(1) << SB_BITS;
     double run = prefix[lo];
     long long found = -1;
-    // GU groups of 32 amplitudes at a time: their loads and scans overlap, the running sum
-    // goes through the groups in order (n = 22, 1000 draws: 62 us with one group at a time,
-    // every group waiting for its own load)
-    constexpr int GU = 8;
     for (i64 x0 = lo * SB; x0 < D && found < 0; x0 += 32 * GU) {
         double sc[GU];  // inclusive warp scan of |psi|^2 per group
 #pragma unroll
@@ -124,6 +123,12 @@ k_draw(const void *psi_, i64 D, const double *prefix, i64 nb, const double *u, i
     }
     if (lane == 0) out[w] = found < 0 ? (long long)(D - 1) : found;  // searchsorted clamp
 }
+
+// Groups a draw takes at a time: eight, except where a draw has few groups to go through and other
+// draws hide its loads.  us at 1 and 8 groups a time, complex64: 2^6 amplitudes 2.6 and 3.3 for 1000
+// draws, 22 and 62 for 100000; 2^8 4.7 and 3.3, 46 and 64; 2^10 14 and 8, 156 and 168 (30000 draws
+// 54 and 56); 2^12 50 and 26, 563 and 531.
+static bool single_groups(i64 D, int draws) { return D <= 64 || (D <= 2048 && (i64)draws >= 32 * D); }
 
 }  // namespace emusv
 
@@ -158,10 +163,10 @@ int emusv_sample(int nqubits, int dtype, const void *psi, int num_shots, const d
         else k_block_sums<float><<<g, BLOCK, 0, s>>>(psi, D, bsum);
         k_block_prefix<<<1, SCAN_THREADS, 0, s>>>(bsum, nb, prefix);
         const int gd = (int)(((i64)num_shots * 32 + BLOCK - 1) / BLOCK);
-        if (dtype == EMUSV_C128)
-            k_draw<double><<<gd, BLOCK, 0, s>>>(psi, D, prefix, nb, uniforms, num_shots, indices, bad);
-        else
-            k_draw<float><<<gd, BLOCK, 0, s>>>(psi, D, prefix, nb, uniforms, num_shots, indices, bad);
+        const bool one = single_groups(D, num_shots);
+        auto *draw = dtype == EMUSV_C128 ? (one ? k_draw<double, 1> : k_draw<double, 8>)
+                                         : (one ? k_draw<float, 1> : k_draw<float, 8>);
+        draw<<<gd, BLOCK, 0, s>>>(psi, D, prefix, nb, uniforms, num_shots, indices, bad);
     }
     EMUSV_CHECK_LAUNCH();
     int hbad = 0;
