@@ -47,9 +47,9 @@ def peaks() -> tuple[float, str]:
 # DRAM bytes (read + write) of one Lanczos iteration at N=26, complex64: ncu's
 # dram__bytes_read.sum + dram__bytes_write.sum of the iteration's three kernels at N=25
 # (python -m emulators_b200.profile_case --n 25 --steps 1 --hpsi 0 --max-krylov-dim 20,
-# launches 4-6 of k_pass_(lz|high): 1610.8 MB read, 669.5 MB written), doubled.  A constant
+# launches 4-6 of k_pass_(lz|high): 1610.8 MB read, 667.6 MB written), doubled.  A constant
 # of the kernels it was measured on; the CUDA-event split reports the streamed units live.
-ITERATION_TRAFFIC_N26_C64 = 2 * (1610.8 + 669.5) * 1e6
+ITERATION_TRAFFIC_N26_C64 = 2 * (1610.8 + 667.6) * 1e6
 
 
 def log(msg: str) -> None:
