@@ -559,6 +559,16 @@ __device__ __forceinline__ int ld_status(const KState *ks) {
 }
 __device__ __forceinline__ int ld_vol(const int *p) { return *(volatile const int *)p; }
 
+// Job i's status for the launch: what made it fail, else a step that reached max_krylov_dim (its
+// decision left that in status_out, zero at the launch's start; later steps may have converged),
+// else its last step's status.
+__device__ __forceinline__ int final_status(const BArgs &A, int i, int last) {
+    const int f = ld_vol(&A.fail[i]);
+    if (f) return f;
+    if (ld_vol(&A.status_out[i]) == KS_MAXDIM) return KS_MAXDIM;
+    return last == BS_IDLE ? KS_CONVERGED : last;
+}
+
 // ---------------------------------------------------------------- phases
 // Decision for iteration j of job i (krylov_exp.py:60-96) by warp 0 of the job's CTA
 // (not inlined: its registers would otherwise crowd the tile loops, which then spill):
@@ -585,6 +595,7 @@ __device__ __noinline__ bool job_decide(const BArgs &A, int i, int j, int rstep)
         }
         if (st == KS_NONFINITE || st == BS_CAPACITY) A.fail[i] = st;
         if (st != KS_RUNNING) {
+            if (st == KS_MAXDIM) A.status_out[i] = st;
             A.iters_out[(size_t)i * A.max_steps + rstep] = ks->iters;
             A.hint[i] = ks->iters > 3 ? ks->iters - 3 : 0;  // poll a little early
         }
@@ -838,8 +849,7 @@ __global__ void __launch_bounds__(BWARPS * 32, MINB) k_batch(const BArgs A) {
     if (threadIdx.x < 32) {  // final statuses
         for (int i = blockIdx.x * 32 + lane; i < A.ninst; i += gridDim.x * 32) {
             const int st = ld_status(A.ks + i);
-            const int f = A.fail[i];
-            A.status_out[i] = f ? f : (st == BS_IDLE ? KS_CONVERGED : st);
+            A.status_out[i] = final_status(A, i, st);
         }
     }
 }
@@ -915,9 +925,7 @@ __device__ void publish(const BArgs &A, int i, unsigned phi, unsigned c) {
 // The job has no phase left in this launch: its final status, then the idle count.
 __device__ void job_idle(const BArgs &A, int i, unsigned phi) {
     if ((threadIdx.x & 31) == 0) {
-        const int st = ld_status(A.ks + i);
-        const int f = ld_vol(&A.fail[i]);
-        A.status_out[i] = f ? f : (st == BS_IDLE ? KS_CONVERGED : st);
+        A.status_out[i] = final_status(A, i, ld_status(A.ks + i));
     }
     publish(A, i, phi, pcode(PK_IDLE, 0, 0));
     if ((threadIdx.x & 31) == 0) {
@@ -1479,6 +1487,7 @@ __device__ __noinline__ void gang_decider(const GArgs &B, int i, int sub, GDec *
                 ks->iters = iters;
                 ks->status = st;
                 if (st == KS_NONFINITE || st == BS_CAPACITY) A.fail[i] = st;
+                if (st == KS_MAXDIM) A.status_out[i] = st;
                 A.iters_out[(size_t)i * A.max_steps + rstep] = iters;
                 const int h = iters > 3 ? iters - 3 : 0;  // poll a little early
                 A.hint[i] = h;
@@ -1623,10 +1632,7 @@ __global__ void __launch_bounds__(BWARPS * 32, MINB) k_batch_gang(const __grid_c
         nv[0] = tile_combine_sum<R, T, MINB == 1 ? 4 : 2>(A, I, i, t, rstep);
         if (!gang_exchange<1>(A, S, turn, nw, rn, I, tl, ++en, nv, false, &stop, mute)) return;
     }
-    if (lead) {
-        const int f = ld_vol(&A.fail[i]);
-        A.status_out[i] = f ? f : (last == BS_IDLE ? KS_CONVERGED : last);
-    }
+    if (lead) A.status_out[i] = final_status(A, i, last);
 }
 
 // ---------------------------------------------------------------- adjoint kernel

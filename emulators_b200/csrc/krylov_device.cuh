@@ -443,7 +443,7 @@ __device__ __forceinline__ double krylov_eval_to(const KState *ks, int jj, doubl
 }
 // Into the run's state, or into a caller's arrays: two functions, because with the arrays as
 // arguments of one function for both the batch's decision (job_decide) reloads 660 bytes of spilled
-// registers instead of 484.
+// registers instead of 496.
 template <int NE>
 static __device__ __noinline__ double krylov_eval_ne(KState *ks, int jj, double dt) {
     return krylov_eval_to<NE>(ks, jj, dt, ks->c_re, ks->c_im);
