@@ -126,16 +126,21 @@ class PulseGradientBatch:
             self.grads[step].data_ptr(), self.status[step].data_ptr(), self.ws_a.data_ptr(),
             torch.cuda.current_stream(self.device).cuda_stream), "batch adjoint")
 
+    def _check_f(self, iterations: np.ndarray | None = None) -> None:
+        """Raises for the last forward launch (waits for it)."""
+        st = np.zeros(self.nsets, dtype=np.int32)
+        _lib.check(_lib.load().emusv_batch_results(
+            self.nsets, self.nsteps, self.ws_f.data_ptr(), st.ctypes.data,
+            iterations.ctypes.data if iterations is not None else None,
+            torch.cuda.current_stream(self.device).cuda_stream), "batch forward")
+
     def forward(self, check: bool = True) -> None:
         """All steps of every set; checkpoints after every ``checkpoint_every`` steps."""
         self.states.copy_(self.initial)
         self._launch_f(0, self.nsteps, self.states, self.hist, self.ck)
         if check:
-            st = np.zeros(self.nsets, dtype=np.int32)
             it = np.zeros((self.nsets, self.nsteps), dtype=np.int32)
-            _lib.check(_lib.load().emusv_batch_results(
-                self.nsets, self.nsteps, self.ws_f.data_ptr(), st.ctypes.data, it.ctypes.data,
-                torch.cuda.current_stream(self.device).cuda_stream), "batch forward")
+            self._check_f(it)
             self.forward_iterations = it
 
     def occupations(self) -> torch.Tensor:
@@ -170,6 +175,8 @@ class PulseGradientBatch:
                 psi = start if k == 0 else self.rec.view(-1, S * D)[k - 1]
                 self._launch_a(first + k, psi, self.g, self.g2)
                 self.g, self.g2 = self.g2, self.g
+            if L > 1:  # the recomputed states of the segment were what its gradients took them for
+                self._check_f()
 
     def loss_and_grad(self):
         """(loss [nsets], dL/dOmega_seg [nsets, nseg], dL/ddelta_seg [nsets, nseg],
