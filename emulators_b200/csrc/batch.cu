@@ -2268,12 +2268,14 @@ static int prepare_common(int ninst, const int *nqubits, const int *nsteps, cons
                 U[q * BMAXQ + p] = u;
             }
         double *E = elow.data() + ((size_t)i << T);
-        for (int l = 0; l < (1 << T); ++l) {
+        // (over the set bits, 40 registers, T = 9: the whole call 355 us; testing every pair of bits, 890
+        // or 1190 as the linker happened to align the loop)
+        for (unsigned l = 0; l < (1u << T); ++l) {
             double e = 0.0;
-            for (int p = 0; p < T; ++p)
-                if ((l >> p) & 1)
-                    for (int q = p + 1; q < T; ++q)
-                        if ((l >> q) & 1) e += U[p * BMAXQ + q];
+            for (unsigned m = l; m; m &= m - 1) {
+                const double *Up = U + __builtin_ctz(m) * BMAXQ;
+                for (unsigned k = m & (m - 1); k; k &= k - 1) e += Up[__builtin_ctz(k)];
+            }
             E[l] = e;
         }
         const int per = adjoint ? 2 : 1;
